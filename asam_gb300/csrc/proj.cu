@@ -50,6 +50,7 @@
 // divisions by the Thomas pivots use the correctly rounded div_rn with
 // precomputed reciprocals, so every value equals the oracle's zebra run bit
 // for bit.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -65,7 +66,9 @@ constexpr int kMaxLev = 8;
 constexpr int kPlaneBlock = 256;
 constexpr int kRedGrid = 1024;
 constexpr int kRedBlock = 256;
-constexpr size_t kRingBytes = (size_t)4 * 8 * kPlaneBlock * sizeof(double);  // ring rows * fields * block, 64 KB
+// Dynamic shared memory of k_plane_half: one CTA per SM, or two (227 KB of the
+// SM less the kernel's static part)
+constexpr size_t kPlaneSmem1 = 229376, kPlaneSmem2 = 112640;
 constexpr double kTiny = 1.0e-40;  // initial diagonal of Allocate_1D (TriDiagT_Mod.f90:99)
 
 // One plane level of a 3D level (all its planes); T = double for the
@@ -75,7 +78,7 @@ template <typename T>
 struct Lev2T {
   int c1, c2, h, w, m3;
   size_t ps;
-  T *d, *uz, *lz, *fw, *ft, *frt, *ux, *lx, *res;
+  T *d, *uz, *lz, *fw, *ft, *frt, *ux, *lx;
   T *x, *b;  // own vectors of the coarse plane levels (nullptr on the 3D level's own planes)
   // periodic-Laplacian hierarchy only (nullptr otherwise): the couplings
   // across the periodic x side, between line 0 and line c2-1 of row i of
@@ -656,7 +659,7 @@ __device__ void line_half_lanes(const Lev2T<T>& P, size_t mo, const T* __restric
 
 template <typename T, bool kWrap = false>
 __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __restrict__ b, T* __restrict__ x, int c,
-                                       int fwd, T* __restrict__ ring) {
+                                       int fwd, T* __restrict__ ring, int rs) {
   if constexpr (sizeof(T) == 4) {  // few lines: K lanes per line (the whole block takes part in the shuffles)
     const int nl = (P.c2 - c + 1) / 2;
     int K = 1;
@@ -675,7 +678,11 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __
   const T* __restrict__ fw = P.fw + mo;
   constexpr int kRing = RingCfg<T>::ring, kAhead = RingCfg<T>::ahead;
   const int nl = (c2 - c + 1) / 2;
-  const int bd = blockDim.x, tid = threadIdx.x;
+  // slots of the ring: rs threads take part (rs = min(block, the lines of one
+  // parity rounded up to a warp)), so a narrow plane leaves the shared memory
+  // to its resident levels
+  const int bd = rs, tid = threadIdx.x;
+  if (tid >= rs) return;
   for (int q = tid; q < nl; q += bd) {
     const int j = 2 * q + c;
     const size_t col = (size_t)c * h + q;
@@ -761,102 +768,334 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __
   }
 }
 
+// ---------------------------------------------------------------------------
+// Plane levels resident in shared memory.
+//
+// What bounds a plane's multigrid is the serial row recurrence of its line
+// solves plus a fixed cost per half-sweep: filling the row ring from L2, the
+// first loads of the back substitution, the restriction's round trips.  A
+// 64x32 block runs 2240 half-sweeps per V-cycle and the coarse plane levels
+// have rows and lines in the tens, so the fixed cost was half of the time.
+// The plane levels that fit (from the coarsest up, all of them for a plane of
+// up to about 2800 FP64 entries) are therefore copied to shared memory once
+// per plane solve, and their smoothing, residuals and transfers touch nothing
+// else; a level that does not fit streams through the ring as before.
+//
+// One resident level, in units of T from its offset: the arrays d, uz, lz,
+// fw, ft, frt, ux, lx, x, b of n = padded(ps) values each, then (kWrap) wxl, wxh.
+template <typename T>
+__host__ __device__ inline int res_pad(size_t n) {
+  constexpr size_t v = 16 / sizeof(T);
+  return (int)((n + v - 1) / v * v);
+}
+template <typename T>
+__host__ __device__ inline int res_elems(int c1, size_t ps, bool wrap) {
+  return 10 * res_pad<T>(ps) + (wrap ? 2 * res_pad<T>((size_t)c1) : 0);
+}
+
+extern __shared__ __align__(16) unsigned char plane_smem[];
+
+// the level's descriptor with the pointers of its resident copy (plane offset 0)
+template <typename T>
+__device__ __forceinline__ Lev2T<T> res_level(const Lev2T<T>& G, int off) {
+  Lev2T<T> S;
+  T* p = reinterpret_cast<T*>(plane_smem) + off;
+  const int n = res_pad<T>(G.ps);
+  S.c1 = G.c1;
+  S.c2 = G.c2;
+  S.h = G.h;
+  S.w = G.w;
+  S.m3 = 1;
+  S.ps = G.ps;
+  S.d = p;
+  S.uz = p + n;
+  S.lz = p + 2 * n;
+  S.fw = p + 3 * n;
+  S.ft = p + 4 * n;
+  S.frt = p + 5 * n;
+  S.ux = p + 6 * n;
+  S.lx = p + 7 * n;
+  S.x = p + 8 * n;
+  S.b = p + 9 * n;
+  S.wxl = G.wxl ? p + 10 * n : nullptr;
+  S.wxh = G.wxl ? p + 10 * n + res_pad<T>((size_t)G.c1) : nullptr;
+  return S;
+}
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+
+// starts the copy of plane k's matrix of one level (rows of an even number of
+// values, so a plane starts on 8 bytes; on 16 when its size is a multiple)
+template <typename T>
+__device__ __forceinline__ void res_copy(const Lev2T<T>& G, int off, int k) {
+  const Lev2T<T> S = res_level(G, off);
+  const T* src[8] = {G.d, G.uz, G.lz, G.fw, G.ft, G.frt, G.ux, G.lx};
+  const size_t bytes = G.ps * sizeof(T);
+  const int n = res_pad<T>(G.ps);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    unsigned char* dst = reinterpret_cast<unsigned char*>(S.d + q * n);
+    const unsigned char* s = reinterpret_cast<const unsigned char*>(src[q] + (size_t)k * G.ps);
+    if (bytes % 16 == 0) {
+      for (size_t e = (size_t)threadIdx.x * 16; e < bytes; e += (size_t)blockDim.x * 16) cp_async16(dst + e, s + e);
+    } else {
+      for (size_t e = (size_t)threadIdx.x * 8; e < bytes; e += (size_t)blockDim.x * 8) cp_async8(dst + e, s + e);
+    }
+  }
+  if (S.wxl)
+    for (int i = threadIdx.x; i < G.c1; i += blockDim.x) {
+      S.wxl[i] = G.wxl[(size_t)k * G.c1 + i];
+      S.wxh[i] = G.wxh[(size_t)k * G.c1 + i];
+    }
+}
+
+// line_half on a resident level: the same relaxation with its operands in
+// shared memory.  The next row's operands are loaded and its right-hand side
+// formed while this row's recurrence runs, so a row costs the recurrence
+// alone: five dependent FP64 operations forward and two backward, 64 cycles
+// each (the ring version waits for its row first, then forms the right-hand
+// side).  A missing neighbour contributes t - 0*0, which leaves every bit of t.
+template <typename T, bool kWrap>
+__device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd) {
+  if constexpr (sizeof(T) == 4) {
+    const int nl = (S.c2 - c + 1) / 2;
+    int K = 1;
+    while (K < 32 && nl * K * 2 <= (int)blockDim.x && K * 4 <= S.c1) K *= 2;
+    if (K >= 8) {
+      line_half_lanes<T, kWrap>(S, 0, S.b, S.x, c, fwd, K);
+      return;
+    }
+  }
+  const int c1 = S.c1, c2 = S.c2, h = S.h, w = S.w;
+  const int nl = (c2 - c + 1) / 2;
+  struct Row {
+    T b, xl, xr, cl, cr, lz, ft, frt;
+  };
+  for (int q = threadIdx.x; q < nl; q += blockDim.x) {
+    const int j = 2 * q + c;
+    const int col = c * h + q;
+    const bool hasL = j > 0, hasR = j < c2 - 1;
+    const int colL = hasL ? (1 - c) * h + ((j - 1) >> 1) : col;
+    const int colR = hasR ? (1 - c) * h + ((j + 1) >> 1) : col;
+    const bool wrap = kWrap && S.wxl && c2 >= 2 && ((c2 - 1) & 1);
+    const bool wL = wrap && j == 0, wR = wrap && j == c2 - 1;
+    const bool useL = hasL || wL, useR = hasR || wR;
+    const T* xL = S.x + (wL ? (int)slot(0, h, 0, c2 - 1) : colL);
+    const T* xR = S.x + (wR ? 0 : colR);
+    const T* cL = wL ? S.wxl : S.lx + colL;
+    const T* cR = wR ? S.wxh : S.ux + col;
+    const int sL = wL ? 1 : w, sR = wR ? 1 : w;
+    const T* bp = S.b + col;
+    const T* lzp = S.lz + col;
+    const T* ftp = S.ft + col;
+    const T* frtp = S.frt + col;
+    T* xp = S.x + col;
+    auto load = [&](int i, Row& r) {
+      const int o = i * w;
+      r.b = bp[o];
+      r.xl = useL ? xL[o] : (T)0;
+      r.cl = useL ? cL[i * sL] : (T)0;
+      r.xr = useR ? xR[o] : (T)0;
+      r.cr = useR ? cR[i * sR] : (T)0;
+      r.lz = i > 0 ? lzp[o - w] : (T)0;
+      r.ft = ftp[o];
+      r.frt = frtp[o];
+    };
+    auto rhs = [&](const Row& r) {
+      const T ml = r.cl * r.xl, mr = r.cr * r.xr;
+      return fwd ? (r.b - ml) - mr : (r.b - mr) - ml;
+    };
+    Row cur, nxt;
+    load(0, cur);
+    load(c1 > 1 ? 1 : 0, nxt);
+    T t = rhs(cur), prev = (T)0;
+    T lz = (T)0, ft = cur.ft, frt = cur.frt;
+    for (int i = 0; i < c1; ++i) {
+      const T m = lz * prev;
+      Row nn;
+      load(i + 2 < c1 ? i + 2 : c1 - 1, nn);
+      const T tt = t - m;
+      const T y = div_rn(tt, ft, frt);
+      t = rhs(nxt);
+      lz = nxt.lz;
+      ft = nxt.ft;
+      frt = nxt.frt;
+      nxt = nn;
+      xp[i * w] = y;
+      prev = y;
+    }
+    const T* fwp = S.fw + col;
+    T ya = (T)0, wa = (T)0;
+    if (c1 > 1) {
+      ya = xp[(c1 - 2) * w];
+      wa = fwp[(c1 - 2) * w];
+    }
+    for (int i = c1 - 2; i >= 0; --i) {
+      const T m = wa * prev;
+      const int in = i > 0 ? i - 1 : 0;
+      const T yn = xp[in * w], wn = fwp[in * w];
+      prev = ya - m;
+      xp[i * w] = prev;
+      ya = yn;
+      wa = wn;
+    }
+  }
+}
+
+// GaussSeidel_2D in zebra order on a global (kRes false) or resident level
 template <typename T, bool kWrap = false>
-__device__ void gs2d(const Lev2T<T>& P, size_t mo, const T* b, T* x, int gi, T* ring) {
+__device__ void gs2d(const Lev2T<T>& P, size_t mo, const T* b, T* x, int gi, T* ring, int rs) {
   if (P.c2 > 1) {
-    for (int it = 0; it < gi; ++it) {
-      line_half<T, kWrap>(P, mo, b, x, 0, 1, ring);
-      __syncthreads();
-      line_half<T, kWrap>(P, mo, b, x, 1, 1, ring);
-      __syncthreads();
-      line_half<T, kWrap>(P, mo, b, x, 1, 0, ring);
-      __syncthreads();
-      line_half<T, kWrap>(P, mo, b, x, 0, 0, ring);
+    for (int hs = 0; hs < 4 * gi; ++hs) {
+      const int s = hs & 3;
+      line_half<T, kWrap>(P, mo, b, x, s == 1 || s == 2, s < 2, ring, rs);
       __syncthreads();
     }
   } else {
-    line_half<T, kWrap>(P, mo, b, x, 0, 1, ring);
+    line_half<T, kWrap>(P, mo, b, x, 0, 1, ring, rs);
+    __syncthreads();
+  }
+}
+template <typename T, bool kWrap>
+__device__ __noinline__ void gs2d_res(const Lev2T<T>& G, int off, int gi) {
+  const Lev2T<T> S = res_level(G, off);
+  const int nh = S.c2 > 1 ? 4 * gi : 1;
+  for (int hs = 0; hs < nh; ++hs) {
+    const int s = hs & 3;
+    line_half_res<T, kWrap>(S, s == 1 || s == 2, s < 2);
     __syncthreads();
   }
 }
 
-// Multigrid_2D (TriDiagT_Mod.f90:490-551) on plane k of a 3D level, inside one CTA
+// Restriction of the residual: the coarse right-hand side is the sum of the
+// four fine residuals b - A x in the reference's order (one pass: the residual
+// itself is not stored), the coarse iterate starts from 0
+template <typename T, bool kWrap>
+__device__ __forceinline__ void restrict2d(const Lev2T<T>& P, size_t mo, const T* b, const T* x, int k, int cw, int ch,
+                                           int cc2, size_t cps, T* bq, T* xq) {
+  for_plane(cw, cps, [&](size_t s, int a, int r) {
+    const int bb = line_of(r, ch, cc2);
+    if (bb < 0) return;
+    T v = (T)0;
+    for (int i1 = 2 * a; i1 <= 2 * a + 1 && i1 < P.c1; ++i1)
+      for (int i2 = 2 * bb; i2 <= 2 * bb + 1 && i2 < P.c2; ++i2) {
+        const size_t e = slot(P.w, P.h, i1, i2);
+        v = v + (b[e] - matvec2_at<T, kWrap>(P, mo, x, e, i1, i2, k));
+      }
+    bq[s] = v;
+    xq[s] = (T)0;
+  });
+}
+template <typename T, bool kWrap>
+__device__ __noinline__ void restrict2d_res(const Lev2T<T>& G, int off, const Lev2T<T>& Gc, int offc) {
+  const Lev2T<T> S = res_level(G, off), C = res_level(Gc, offc);
+  restrict2d<T, kWrap>(S, 0, S.b, S.x, 0, C.w, C.h, C.c2, C.ps, C.b, C.x);
+}
+
+// x of level F corrected by x of the next coarser level P
+template <typename T>
+__device__ __forceinline__ void prolong2d(int fw, int fh, int fc2, size_t fps, T* xf, int pw, int ph, const T* x) {
+  for_plane(fw, fps, [&](size_t s, int i, int r) {
+    const int j = line_of(r, fh, fc2);
+    if (j >= 0) xf[s] = xf[s] + x[slot(pw, ph, i >> 1, j >> 1)];
+  });
+}
+
+// Multigrid_2D (TriDiagT_Mod.f90:490-551) on plane k of a 3D level, inside one
+// CTA; the plane levels from mr on are resident at roff[level]
 template <typename T, bool kWrap = false>
-__device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, T* ring) {
+__device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, T* ring, int rs, int mr, const int* roff) {
   const int nl = A.nl;
   int gi = 1;
-  int lv = 0;
-  for (;;) {
-    const Lev2T<T>& P = A.pl[lv];
-    T* x = lv == 0 ? x0 : P.x + (size_t)k * P.ps;
-    const T* b = lv == 0 ? b0 : P.b + (size_t)k * P.ps;
-    const size_t mo = (size_t)k * P.ps;
-    gs2d<T, kWrap>(P, mo, b, x, gi, ring);
+  auto xg = [&](int lv) { return lv == 0 ? x0 : A.pl[lv].x + (size_t)k * A.pl[lv].ps; };
+  auto bg = [&](int lv) { return lv == 0 ? b0 : A.pl[lv].b + (size_t)k * A.pl[lv].ps; };
+  auto smooth = [&](int lv) {
+    if (lv >= mr)
+      gs2d_res<T, kWrap>(A.pl[lv], roff[lv], gi);
+    else
+      gs2d<T, kWrap>(A.pl[lv], (size_t)k * A.pl[lv].ps, bg(lv), xg(lv), gi, ring, rs);
+  };
+  for (int lv = 0; lv < nl; ++lv) {
+    smooth(lv);
+    if (lv + 1 == nl) break;
     gi += gi2;
-    if (lv + 1 < nl) {
-      T* res = P.res + (size_t)k * P.ps;
-      const size_t np = P.ps;
-      for_plane(P.w, np, [&](size_t s, int i, int r) {
-        const int j = line_of(r, P.h, P.c2);
-        if (j >= 0) res[s] = b[s] - matvec2_at<T, kWrap>(P, mo, x, s, i, j, k);
-      });
-      __syncthreads();
-      const Lev2T<T>& Q = A.pl[lv + 1];
-      T* bq = Q.b + (size_t)k * Q.ps;
-      T* xq = Q.x + (size_t)k * Q.ps;
-      for_plane(Q.w, Q.ps, [&](size_t s, int a, int r) {
-        const int bb = line_of(r, Q.h, Q.c2);
-        if (bb < 0) return;
-        T v = (T)0;
-        for (int i1 = 2 * a; i1 <= 2 * a + 1 && i1 < P.c1; ++i1)
-          for (int i2 = 2 * bb; i2 <= 2 * bb + 1 && i2 < P.c2; ++i2) v = v + res[slot(P.w, P.h, i1, i2)];
-        bq[s] = v;
-        xq[s] = (T)0;
-      });
-      __syncthreads();
-      ++lv;
-    } else {
-      gi -= gi2;
-      break;
-    }
-  }
-  for (;;) {
     const Lev2T<T>& P = A.pl[lv];
-    T* x = lv == 0 ? x0 : P.x + (size_t)k * P.ps;
-    const T* b = lv == 0 ? b0 : P.b + (size_t)k * P.ps;
-    gs2d<T, kWrap>(P, (size_t)k * P.ps, b, x, gi, ring);
-    gi -= gi2;
-    if (lv > 0) {
-      const Lev2T<T>& F = A.pl[lv - 1];
-      T* xf = lv - 1 == 0 ? x0 : F.x + (size_t)k * F.ps;
-      for_plane(F.w, F.ps, [&](size_t s, int i, int r) {
-        const int j = line_of(r, F.h, F.c2);
-        if (j >= 0) xf[s] = xf[s] + x[slot(P.w, P.h, i >> 1, j >> 1)];
-      });
-      __syncthreads();
-      --lv;
+    const Lev2T<T>& Q = A.pl[lv + 1];
+    if (lv >= mr) {
+      restrict2d_res<T, kWrap>(P, roff[lv], Q, roff[lv + 1]);
     } else {
-      break;
+      T *bq, *xq;
+      if (lv + 1 >= mr) {
+        const Lev2T<T> S = res_level(Q, roff[lv + 1]);
+        bq = S.b;
+        xq = S.x;
+      } else {
+        bq = Q.b + (size_t)k * Q.ps;
+        xq = Q.x + (size_t)k * Q.ps;
+      }
+      restrict2d<T, kWrap>(P, (size_t)k * P.ps, bg(lv), xg(lv), k, Q.w, Q.h, Q.c2, Q.ps, bq, xq);
     }
+    __syncthreads();
+  }
+  for (int lv = nl - 1;; --lv) {
+    smooth(lv);
+    gi -= gi2;
+    if (lv == 0) break;
+    const Lev2T<T>& P = A.pl[lv];
+    const Lev2T<T>& F = A.pl[lv - 1];
+    if (lv - 1 >= mr) {
+      const Lev2T<T> S = res_level(P, roff[lv]), SF = res_level(F, roff[lv - 1]);
+      prolong2d(F.w, F.h, F.c2, F.ps, SF.x, P.w, P.h, S.x);
+    } else if (lv >= mr) {
+      const Lev2T<T> S = res_level(P, roff[lv]);
+      prolong2d(F.w, F.h, F.c2, F.ps, xg(lv - 1), P.w, P.h, S.x);
+    } else {
+      prolong2d(F.w, F.h, F.c2, F.ps, xg(lv - 1), P.w, P.h, (const T*)xg(lv));
+    }
+    __syncthreads();
   }
 }
 
 // One zebra half-sweep of GaussSeidel_3D over the planes of parity `color` of
 // 3D level L: each CTA forms its plane's right-hand side (forward or backward
-// operation order of the reference) and runs Solve_2D on it.
+// operation order of the reference) and runs Solve_2D on it.  mr: the first
+// resident plane level (0: the whole plane solve runs in shared memory, only
+// x goes back; A.nl: none); rs: threads of the ring.
 template <typename T, bool kWrap = false>
 __global__ void __launch_bounds__(kPlaneBlock, 2) k_plane_half(const Lev3T<T>* __restrict__ lvs, int L, int color, int fwd,
-                                                             int mult_iter2, int gi2) {
+                                                             int mult_iter2, int gi2, int mr, int rs) {
   __shared__ Lev3T<T> A;
-  extern __shared__ __align__(16) unsigned char ring_raw[];  // kRing * kFields * blockDim values of T
-  T* ring = reinterpret_cast<T*>(ring_raw);
-  if (threadIdx.x == 0) A = lvs[L];
+  __shared__ int roff[kMaxLev + 1];
+  T* ring = reinterpret_cast<T*>(plane_smem);  // kRing * kFields * rs values of T (mr > 0), then the resident levels
+  if (threadIdx.x == 0) {
+    A = lvs[L];
+    int o = mr > 0 ? RingCfg<T>::ring * kFields * rs : 0;
+    for (int lv = mr; lv < A.nl; ++lv) {
+      roff[lv] = o;
+      o += res_elems<T>(A.pl[lv].c1, A.pl[lv].ps, A.pl[lv].wxl != nullptr);
+    }
+  }
   __syncthreads();
   const Lev2T<T>& P0 = A.pl[0];
   for (int q = blockIdx.x;; q += gridDim.x) {
     const int k = 2 * q + color;
     if (k >= A.m3) break;
+    for (int lv = mr; lv < A.nl; ++lv) res_copy(A.pl[lv], roff[lv], k);
+    cp_commit();
     const size_t off = (size_t)k * P0.ps, ps = P0.ps;
+    T *x0 = A.x + off, *t0 = A.t + off;
+    if (mr == 0) {
+      const Lev2T<T> S = res_level(P0, roff[0]);
+      x0 = S.x;
+      t0 = S.b;
+    }
     for_plane(P0.w, ps, [&](size_t s, int, int r) {
       if (line_of(r, P0.h, P0.c2) < 0) return;
       const size_t e = off + s;
@@ -874,10 +1113,17 @@ __global__ void __launch_bounds__(kPlaneBlock, 2) k_plane_half(const Lev3T<T>* _
         if (k == 0) v = v - A.wyl[s] * A.x[(size_t)(A.m3 - 1) * ps + s];
         if (k == A.m3 - 1) v = v - A.wyh[s] * A.x[s];
       }
-      A.t[e] = v;
+      t0[s] = v;
+      if (mr == 0) x0[s] = A.x[e];
     });
+    cp_wait<0>();
     __syncthreads();
-    for (int it = 0; it < mult_iter2; ++it) mg2d<T, kWrap>(A, k, A.x + off, A.t + off, gi2, ring);
+    for (int it = 0; it < mult_iter2; ++it) mg2d<T, kWrap>(A, k, x0, t0, gi2, ring, rs, mr, roff);
+    if (mr == 0) {  // x0 is final: the last smoother ended with a block barrier
+      for_plane(P0.w, ps, [&](size_t s, int, int r) {
+        if (line_of(r, P0.h, P0.c2) >= 0) A.x[off + s] = x0[s];
+      });
+    }
     __syncthreads();
   }
 }
@@ -1637,7 +1883,7 @@ int alloc_lev2(ProjState* s, Lev2& P, int c1, int c2, int m3, bool own_vectors) 
   P.m3 = m3;
   P.ps = (size_t)c1 * P.w;
   const size_t n = P.ps * m3;
-  double** arr[] = {&P.d, &P.uz, &P.lz, &P.fw, &P.ft, &P.frt, &P.ux, &P.lx, &P.res};
+  double** arr[] = {&P.d, &P.uz, &P.lz, &P.fw, &P.ft, &P.frt, &P.ux, &P.lx};
   for (double** q : arr)
     if (int rc = palloc(s, q, n)) return rc;
   P.x = P.b = nullptr;
@@ -1733,10 +1979,10 @@ int proj_build(asam_ctx* h) {
     if (int rc = palloc(s, &s->d_lvD, (size_t)R)) return rc;
     CK(cudaMemcpyAsync(s->d_lvD, s->lvD.data(), sizeof(Lev3) * R, cudaMemcpyHostToDevice, s->st));
   }
-  CK(cudaFuncSetAttribute(k_plane_half<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingBytes));
-  CK(cudaFuncSetAttribute(k_plane_half<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingBytes));
-  CK(cudaFuncSetAttribute(k_plane_half<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingBytes));
-  CK(cudaFuncSetAttribute(k_plane_half<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingBytes));
+  CK(cudaFuncSetAttribute(k_plane_half<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem1));
+  CK(cudaFuncSetAttribute(k_plane_half<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem1));
+  CK(cudaFuncSetAttribute(k_plane_half<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem1));
+  CK(cudaFuncSetAttribute(k_plane_half<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem1));
   if (int rc = palloc(s, &s->d_lv, (size_t)R)) return rc;
   CK(cudaMemcpyAsync(s->d_lv, s->lv.data(), sizeof(Lev3) * R, cudaMemcpyHostToDevice, s->st));
   CK(cudaStreamSynchronize(s->st));
@@ -1764,6 +2010,31 @@ int proj_build(asam_ctx* h) {
   return kOk;
 }
 
+// Which plane levels of a 3D level a half-sweep over np planes keeps in shared
+// memory: as many as fit, from the coarsest up, in one CTA's share of an SM
+// (two CTAs per SM when there are more planes than SMs)
+struct PlanePlan {
+  int mr, rs;
+  size_t smem;
+};
+template <typename T>
+PlanePlan plane_plan(const Lev3T<T>& A, int np) {
+  const size_t cap = np > 152 ? kPlaneSmem2 : kPlaneSmem1;
+  const int rs = std::min(kPlaneBlock, (A.pl[0].h + 31) / 32 * 32);
+  const size_t ring = (size_t)RingCfg<T>::ring * kFields * rs * sizeof(T);
+  size_t used = 0;
+  int mr = A.nl;
+  while (mr > 0) {
+    const Lev2T<T>& P = A.pl[mr - 1];
+    if (P.ps > cap / (10 * sizeof(T))) break;
+    const size_t add = (size_t)res_elems<T>(P.c1, P.ps, P.wxl != nullptr) * sizeof(T);
+    if (used + add + (mr > 1 ? ring : 0) > cap) break;
+    used += add;
+    --mr;
+  }
+  return PlanePlan{mr, rs, used + (mr > 0 ? ring : 0)};
+}
+
 // Solve_3D from a zero start on level 0 (VCycleCG's MatrixT branch): lv[0].b
 // holds the right-hand side, the result is left in lv[0].x
 template <typename T, bool kWrap = false>
@@ -1772,7 +2043,6 @@ void vcycle_run(asam_ctx* h, std::vector<Lev3T<T>>& lv, Lev3T<T>* d_lv, int gi2,
   const cudaStream_t st = h->L.stream;
   const int R = s->R;
   const int mi2 = s->cfg.mult_iter2;
-  const size_t ring = (size_t)RingCfg<T>::ring * kFields * kPlaneBlock * sizeof(T);
   long long nl = 0;
   cudaMemsetAsync(lv[0].x, 0, sizeof(T) * len0(s), st);
   auto gs3 = [&](int L, int gi) {
@@ -1780,7 +2050,8 @@ void vcycle_run(asam_ctx* h, std::vector<Lev3T<T>>& lv, Lev3T<T>* d_lv, int gi2,
     auto half = [&](int c, int fwd) {
       const int np = (A.m3 - c + 1) / 2;
       if (np <= 0) return;
-      k_plane_half<T, kWrap><<<np, kPlaneBlock, ring, st>>>(d_lv, L, c, fwd, mi2, gi2);
+      const PlanePlan pp = plane_plan(A, np);
+      k_plane_half<T, kWrap><<<np, kPlaneBlock, pp.smem, st>>>(d_lv, L, c, fwd, mi2, gi2, pp.mr, pp.rs);
       ++nl;
     };
     if (A.m3 > 1) {
@@ -1919,7 +2190,7 @@ int alloc_lev32(ProjState* s) {
       Q.m3 = P.m3;
       Q.ps = P.ps;
       const size_t n = P.ps * P.m3;
-      float** arr[] = {&Q.d, &Q.uz, &Q.lz, &Q.fw, &Q.ft, &Q.frt, &Q.ux, &Q.lx, &Q.res};
+      float** arr[] = {&Q.d, &Q.uz, &Q.lz, &Q.fw, &Q.ft, &Q.frt, &Q.ux, &Q.lx};
       for (float** r : arr)
         if (int rc = palloc(s, r, n)) return rc;
       Q.x = Q.b = nullptr;
