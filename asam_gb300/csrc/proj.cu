@@ -657,6 +657,49 @@ __device__ void line_half_lanes(const Lev2T<T>& P, size_t mo, const T* __restric
   }
 }
 
+// FP64: the line right-hand sides of one half-sweep formed by the whole block
+// and left in x of the lines to be solved, before their recurrences.  A GB300
+// sub-partition takes 64 cycles per FP64 warp instruction, dependent or not, so
+// a warp that forms its own right-hand sides (four operations a row) and then
+// runs the recurrence (seven) pays all eleven one after the other while the
+// block's other warps wait: 704 cycles a row against 448.  With more lines
+// than four warps the solving warps fill all four sub-partitions by
+// themselves and the split would only move the same work (kSplitLines).
+constexpr int kSplitLines = 128;
+template <typename T>
+__device__ __forceinline__ bool split_rhs(int nl) {
+  return sizeof(T) == 8 && nl <= kSplitLines;
+}
+template <typename T, bool kWrap>
+__device__ __forceinline__ void rhs_half(const Lev2T<T>& P, size_t mo, const T* __restrict__ b, T* x, int c, int fwd) {
+  const int c1 = P.c1, c2 = P.c2, h = P.h, w = P.w;
+  const T* lx = P.lx + mo;
+  const T* ux = P.ux + mo;
+  const int nl = (c2 - c + 1) / 2;
+  const bool wrap = kWrap && P.wxl && c2 >= 2 && ((c2 - 1) & 1);
+  const size_t wk = kWrap ? (mo / P.ps) * (size_t)c1 : 0;
+  for_plane(nl, (size_t)nl * c1, [&](size_t, int i, int q) {
+    const int j = 2 * q + c;
+    const int o = i * w, oth = o + (1 - c) * h;
+    const int e = o + c * h + q;
+    const T bv = b[e];
+    T ml = (T)0, mr = (T)0;  // a missing neighbour: t - 0 leaves every bit of t
+    if (j > 0) {
+      const int a = oth + ((j - 1) >> 1);
+      ml = lx[a] * x[a];
+    } else if (wrap) {
+      ml = P.wxl[wk + i] * x[o + slot(0, h, 0, c2 - 1)];
+    }
+    if (j < c2 - 1) {
+      mr = ux[e] * x[oth + ((j + 1) >> 1)];
+    } else if (wrap) {
+      mr = P.wxh[wk + i] * x[o];
+    }
+    x[e] = fwd ? (bv - ml) - mr : (bv - mr) - ml;
+  });
+  __syncthreads();
+}
+
 template <typename T, bool kWrap = false>
 __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __restrict__ b, T* __restrict__ x, int c,
                                        int fwd, T* __restrict__ ring, int rs) {
@@ -669,6 +712,8 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __
       return;
     }
   }
+  const bool split = split_rhs<T>((P.c2 - c + 1) / 2);
+  if (split) rhs_half<T, kWrap>(P, mo, b, x, c, fwd);
   const int c1 = P.c1, c2 = P.c2, h = P.h, w = P.w;
   const T* __restrict__ lx = P.lx + mo;
   const T* __restrict__ ux = P.ux + mo;
@@ -696,19 +741,22 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __
     // slots of the missing neighbour, so they stream ahead like the others.
     const bool wrap = kWrap && P.wxl && c2 >= 2 && ((c2 - 1) & 1);
     const bool wL = wrap && j == 0, wR = wrap && j == c2 - 1;
-    const bool useL = hasL || wL, useR = hasR || wR;
+    const bool useL = !split && (hasL || wL), useR = !split && (hasR || wR);
     const size_t wk = (mo / P.ps) * (size_t)c1;
     const size_t xL0 = wL ? slot(0, h, 0, c2 - 1) : colL, xR0 = wR ? slot(0, h, 0, 0) : colR;
+    const T* rb = split ? x : b;
     auto issue = [&](int i) {
       T* sl = ring + (size_t)(i % kRing) * kFields * bd + tid;
       const bool ok = i < c1;
       const size_t io = ok ? (size_t)i : 0, o = io * w;
       const size_t om = i > 0 && ok ? o - w : o;
-      cp_async_elem(sl + 0 * bd, b + col + o, ok);
-      cp_async_elem(sl + 1 * bd, x + xL0 + o, ok && useL);
-      cp_async_elem(sl + 2 * bd, x + xR0 + o, ok && useR);
-      cp_async_elem(sl + 3 * bd, wL ? P.wxl + wk + io : lx + colL + o, ok && useL);
-      cp_async_elem(sl + 4 * bd, wR ? P.wxh + wk + io : ux + col + o, ok && useR);
+      cp_async_elem(sl + 0 * bd, rb + col + o, ok);
+      if (!split) {
+        cp_async_elem(sl + 1 * bd, x + xL0 + o, ok && useL);
+        cp_async_elem(sl + 2 * bd, x + xR0 + o, ok && useR);
+        cp_async_elem(sl + 3 * bd, wL ? P.wxl + wk + io : lx + colL + o, ok && useL);
+        cp_async_elem(sl + 4 * bd, wR ? P.wxh + wk + io : ux + col + o, ok && useR);
+      }
       cp_async_elem(sl + 5 * bd, lz + col + om, ok && i > 0);
       cp_async_elem(sl + 6 * bd, ft + col + o, ok);
       cp_async_elem(sl + 7 * bd, frt + col + o, ok);
@@ -857,11 +905,10 @@ __device__ __forceinline__ void res_copy(const Lev2T<T>& G, int off, int k) {
 }
 
 // line_half on a resident level: the same relaxation with its operands in
-// shared memory.  The next row's operands are loaded and its right-hand side
-// formed while this row's recurrence runs, so a row costs the recurrence
-// alone: five dependent FP64 operations forward and two backward, 64 cycles
-// each (the ring version waits for its row first, then forms the right-hand
-// side).  A missing neighbour contributes t - 0*0, which leaves every bit of t.
+// shared memory.  The next row's operands are loaded while this row's
+// recurrence runs, so an FP64 row costs the recurrence alone (five dependent
+// operations forward and two backward).  A missing neighbour contributes
+// t - 0*0, which leaves every bit of t.
 template <typename T, bool kWrap>
 __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd) {
   if constexpr (sizeof(T) == 4) {
@@ -875,6 +922,8 @@ __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd)
   }
   const int c1 = S.c1, c2 = S.c2, h = S.h, w = S.w;
   const int nl = (c2 - c + 1) / 2;
+  const bool split = split_rhs<T>(nl);
+  if (split) rhs_half<T, kWrap>(S, 0, S.b, S.x, c, fwd);
   struct Row {
     T b, xl, xr, cl, cr, lz, ft, frt;
   };
@@ -897,39 +946,55 @@ __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd)
     const T* ftp = S.ft + col;
     const T* frtp = S.frt + col;
     T* xp = S.x + col;
-    auto load = [&](int i, Row& r) {
-      const int o = i * w;
-      r.b = bp[o];
-      r.xl = useL ? xL[o] : (T)0;
-      r.cl = useL ? cL[i * sL] : (T)0;
-      r.xr = useR ? xR[o] : (T)0;
-      r.cr = useR ? cR[i * sR] : (T)0;
-      r.lz = i > 0 ? lzp[o - w] : (T)0;
-      r.ft = ftp[o];
-      r.frt = frtp[o];
-    };
-    auto rhs = [&](const Row& r) {
-      const T ml = r.cl * r.xl, mr = r.cr * r.xr;
-      return fwd ? (r.b - ml) - mr : (r.b - mr) - ml;
-    };
-    Row cur, nxt;
-    load(0, cur);
-    load(c1 > 1 ? 1 : 0, nxt);
-    T t = rhs(cur), prev = (T)0;
-    T lz = (T)0, ft = cur.ft, frt = cur.frt;
-    for (int i = 0; i < c1; ++i) {
-      const T m = lz * prev;
-      Row nn;
-      load(i + 2 < c1 ? i + 2 : c1 - 1, nn);
-      const T tt = t - m;
-      const T y = div_rn(tt, ft, frt);
-      t = rhs(nxt);
-      lz = nxt.lz;
-      ft = nxt.ft;
-      frt = nxt.frt;
-      nxt = nn;
-      xp[i * w] = y;
-      prev = y;
+    T prev = (T)0;
+    if (split) {
+      T t = xp[0], lz = (T)0, ft = ftp[0], frt = frtp[0];
+      for (int i = 0; i < c1; ++i) {
+        const T m = lz * prev;
+        const int in = (i + 1 < c1 ? i + 1 : i) * w;
+        const T tn = xp[in], lzn = lzp[in - (i + 1 < c1 ? w : 0)], ftn = ftp[in], frtn = frtp[in];
+        prev = div_rn(t - m, ft, frt);
+        xp[i * w] = prev;
+        t = tn;
+        lz = lzn;
+        ft = ftn;
+        frt = frtn;
+      }
+    } else {
+      auto load = [&](int i, Row& r) {
+        const int o = i * w;
+        r.b = bp[o];
+        r.xl = useL ? xL[o] : (T)0;
+        r.cl = useL ? cL[i * sL] : (T)0;
+        r.xr = useR ? xR[o] : (T)0;
+        r.cr = useR ? cR[i * sR] : (T)0;
+        r.lz = i > 0 ? lzp[o - w] : (T)0;
+        r.ft = ftp[o];
+        r.frt = frtp[o];
+      };
+      auto rhs = [&](const Row& r) {
+        const T ml = r.cl * r.xl, mr = r.cr * r.xr;
+        return fwd ? (r.b - ml) - mr : (r.b - mr) - ml;
+      };
+      Row cur, nxt;
+      load(0, cur);
+      load(c1 > 1 ? 1 : 0, nxt);
+      T t = rhs(cur);
+      T lz = (T)0, ft = cur.ft, frt = cur.frt;
+      for (int i = 0; i < c1; ++i) {
+        const T m = lz * prev;
+        Row nn;
+        load(i + 2 < c1 ? i + 2 : c1 - 1, nn);
+        const T tt = t - m;
+        const T y = div_rn(tt, ft, frt);
+        t = rhs(nxt);
+        lz = nxt.lz;
+        ft = nxt.ft;
+        frt = nxt.frt;
+        nxt = nn;
+        xp[i * w] = y;
+        prev = y;
+      }
     }
     const T* fwp = S.fw + col;
     T ya = (T)0, wa = (T)0;
