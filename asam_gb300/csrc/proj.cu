@@ -1014,27 +1014,28 @@ __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd)
   }
 }
 
-// GaussSeidel_2D in zebra order on a global (kRes false) or resident level
+// GaussSeidel_2D in zebra order: gi times the half-sweeps (even lines forward,
+// odd forward, odd backward, even backward).  A line solve reads b and the
+// lines of the other parity only, so a half-sweep that directly follows one
+// of the same parity overwrites its result unread; what is left of an
+// iteration is even forward, odd backward, and after the last one even
+// backward: 2*gi + 1 half-sweeps instead of 4*gi, with the same x.
+__device__ __forceinline__ int gs_half_sweeps(int gi) { return gi > 0 ? 2 * gi + 1 : 0; }
+
 template <typename T, bool kWrap = false>
 __device__ void gs2d(const Lev2T<T>& P, size_t mo, const T* b, T* x, int gi, T* ring, int rs) {
-  if (P.c2 > 1) {
-    for (int hs = 0; hs < 4 * gi; ++hs) {
-      const int s = hs & 3;
-      line_half<T, kWrap>(P, mo, b, x, s == 1 || s == 2, s < 2, ring, rs);
-      __syncthreads();
-    }
-  } else {
-    line_half<T, kWrap>(P, mo, b, x, 0, 1, ring, rs);
+  const int nh = P.c2 > 1 ? gs_half_sweeps(gi) : 1;
+  for (int hs = 0; hs < nh; ++hs) {  // a single line is solved once
+    line_half<T, kWrap>(P, mo, b, x, hs & 1, P.c2 == 1 || (!(hs & 1) && hs + 1 < nh), ring, rs);
     __syncthreads();
   }
 }
 template <typename T, bool kWrap>
 __device__ __noinline__ void gs2d_res(const Lev2T<T>& G, int off, int gi) {
   const Lev2T<T> S = res_level(G, off);
-  const int nh = S.c2 > 1 ? 4 * gi : 1;
+  const int nh = S.c2 > 1 ? gs_half_sweeps(gi) : 1;
   for (int hs = 0; hs < nh; ++hs) {
-    const int s = hs & 3;
-    line_half_res<T, kWrap>(S, s == 1 || s == 2, s < 2);
+    line_half_res<T, kWrap>(S, hs & 1, S.c2 == 1 || (!(hs & 1) && hs + 1 < nh));
     __syncthreads();
   }
 }
