@@ -11,6 +11,7 @@
 #include <string>
 
 #include "context.h"
+#include "fp64_int.cuh"
 
 #include <atomic>
 #include <mutex>
@@ -755,6 +756,30 @@ __global__ void k_probe_div(unsigned long long n, unsigned long long seed, int s
     const double e = __fma_rn(-q0, dd, x);
     const double qq = __fma_rn(e, r, q0);
     if (qq != x / dd) ++cnt;
+    // the integer-unit product and quotient on the same pair, and on operands
+    // where they round, carry or leave their range: long runs of zeros and ones
+    // in the significands, powers of two, dividends next to the midpoint of two
+    // quotients, zeros, infinities, NaN, numbers of either end of the range
+    const unsigned long long s = splitmix(seed ^ ~q);
+    double a = x, b = dd;
+    unsigned long long ab = (unsigned long long)__double_as_longlong(a), bb = (unsigned long long)__double_as_longlong(b);
+    if ((s & 3) == 1) ab |= (1ull << (s >> 8) % 53) - 1;
+    if ((s & 3) == 2) ab &= ~((1ull << (s >> 8) % 53) - 1);
+    if ((s >> 2 & 3) == 1) bb |= (1ull << (s >> 16) % 53) - 1;
+    if ((s >> 2 & 3) == 2) bb &= ~((1ull << (s >> 16) % 53) - 1);
+    a = __longlong_as_double((long long)ab);
+    b = __longlong_as_double((long long)bb);
+    if ((s >> 4 & 3) == 1) {
+      const double m = __longlong_as_double((long long)((ab & 0xfffffffffffffull) | 1023ull << 52));
+      a = __fma_rn(ldexp(1.0, -53), b, __dmul_rn(m, b));
+      a = __longlong_as_double(__double_as_longlong(a) + (long long)((s >> 24) % 5) - 2);
+    }
+    const double ends[8] = {0.0, -0.0, INFINITY, NAN, 4.9e-324, 1.7e308, 2.3e-308, 1.0};
+    if ((s >> 6 & 63) == 1) a = ends[s >> 32 & 7];
+    if ((s >> 6 & 63) == 2) b = ends[s >> 32 & 7];
+    auto same = [](double u, double v) { return __double_as_longlong(u) == __double_as_longlong(v) || (isnan(u) && isnan(v)); };
+    if (!same(fpi::mul_rn(a, b), __dmul_rn(a, b))) ++cnt;
+    if (!same(fpi::div_rn(a, b), __ddiv_rn(a, b))) ++cnt;
   }
   if (cnt) atomicAdd(bad, cnt);
 }

@@ -35,8 +35,8 @@ __device__ __forceinline__ u64 left_sig(unsigned hi, unsigned lo) {
   return ((u64)h << 32) | (lo << 11);
 }
 
-__device__ __noinline__ double mul_special(double a, double b) { return __dmul_rn(a, b); }
-__device__ __noinline__ double div_special(double a, double b) { return __ddiv_rn(a, b); }
+static __device__ __noinline__ double mul_special(double a, double b) { return __dmul_rn(a, b); }
+static __device__ __noinline__ double div_special(double a, double b) { return __ddiv_rn(a, b); }
 
 // RN(a*b)
 __device__ __forceinline__ double mul_rn(double a, double b) {

@@ -14,6 +14,7 @@
 #include <memory>
 
 #include "context.h"
+#include "fp64_int.cuh"
 
 namespace {
 
@@ -189,14 +190,12 @@ __global__ void k_tri_tb_gs_2d(int tr, int nplane, int n2, int n1, const double*
 
 // RestrictTB_2D (TriDiagTB_Mod.f90:495-525) per coarse entry: the value the
 // reference's overwriting loops leave there
-__device__ __forceinline__ void restrict_2d_entry(int n2, int n1, const double* __restrict__ res,
-                                                  double* __restrict__ resc, size_t e) {
-  const int n1c = (n1 + 1) / 2, n2c = (n2 + 1) / 2;
+// of one plane; rf(i, j) the fine residual
+template <typename F>
+__device__ __forceinline__ void restrict_2d_entry_of(int n2, int n1, F&& rf, double* resc, size_t e) {
+  const int n1c = (n1 + 1) / 2;
   const int ic = (int)(e % n1c);
-  const int jc = (int)((e / n1c) % n2c);
-  const size_t p = e / ((size_t)n1c * n2c);
-  const double* R = res + p * n2 * n1 * 2;
-  auto rf = [&](int i, int j) { return ld_v(R + ((size_t)j * n1 + i) * 2); };
+  const int jc = (int)(e / n1c);
   V2 v;
   if (jc < n2 / 2) {
     const int jf = 2 * jc;
@@ -210,6 +209,13 @@ __device__ __forceinline__ void restrict_2d_entry(int n2, int n1, const double* 
     v = ic < n1 / 2 ? add_v(rf(2 * ic, n2 - 1), rf(2 * ic + 1, n2 - 1)) : rf(n1 - 1, n2 - 1);
   }
   st_v(resc + e * 2, v);
+}
+__device__ __forceinline__ void restrict_2d_entry(int n2, int n1, const double* __restrict__ res,
+                                                  double* __restrict__ resc, size_t e) {
+  const size_t npc = (size_t)((n1 + 1) / 2) * ((n2 + 1) / 2), p = e / npc;
+  const double* R = res + p * n2 * n1 * 2;
+  restrict_2d_entry_of(n2, n1, [&](int i, int j) { return ld_v(R + ((size_t)j * n1 + i) * 2); }, resc + p * npc * 2,
+                       e - p * npc);
 }
 
 __global__ void k_tri_tb_restrict_2d(int nplane, int n2, int n1, const double* __restrict__ res,
@@ -776,140 +782,220 @@ __global__ void k_tb_coarse_cells(int n3, int n2, int n1, TbFields g, int c3, in
   c.dur[e] = __ddiv_rn(rv, __dadd_rn(v, asam::kEps));
 }
 
-// Zebra half-sweep of GaussSeidel_2D (the GPU's parallel order): one thread per
-// line j = j0 + m*jstep (m < jcount) of every plane, its right-hand side with
-// the forward ((b - l x(j-1)) - u x(j+1)) or backward ((b - u x(j+1)) -
-// l x(j-1)) operation order written over x(j), then Solve_1D in place; the
-// lines of one parity read only lines of the other
-__device__ __forceinline__ void relax_line(int tr, int n2, int n1, const double* __restrict__ d,
-                                           const double* __restrict__ u1, const double* __restrict__ l1,
-                                           const double* __restrict__ u2, const double* __restrict__ l2,
-                                           const double* __restrict__ b, double* __restrict__ x, size_t p, int j,
-                                           int bwd, double* __restrict__ w, size_t ws) {
-  const size_t line = p * n2 + j;
-  double* xl = x + line * n1 * 2;
-  const double* bl = b + line * n1 * 2;
-  for (int i = 0; i < n1; ++i) {
-    V2 v = ld_v(bl + 2 * i);
-    const double* cl = j > 0 ? l2 + ((p * (n2 - 1) + j - 1) * n1 + i) * 4 : nullptr;
-    const double* cu = j < n2 - 1 ? u2 + ((p * (n2 - 1) + j) * n1 + i) * 4 : nullptr;
-    if (!bwd) {
-      if (cl) v = couple_sub(tr, v, cl, ld_v(xl - (size_t)n1 * 2 + 2 * i));
-      if (cu) v = couple_sub(tr, v, cu, ld_v(xl + (size_t)n1 * 2 + 2 * i));
-    } else {
-      if (cu) v = couple_sub(tr, v, cu, ld_v(xl + (size_t)n1 * 2 + 2 * i));
-      if (cl) v = couple_sub(tr, v, cl, ld_v(xl - (size_t)n1 * 2 + 2 * i));
+// ---------------------------------------------------------------------------
+// Zebra order of the smoothers (the GPU's parallel order) on a resident
+// hierarchy: the lines of one parity of a plane, and the planes of one parity
+// of a level, at once.
+//
+// The elimination factors of Solve_1D depend on the matrix only, so they are
+// computed once per hierarchy (k_tb_factor): the pivot blocks t(i), w(i) =
+// t(i)^-1 u(i), Det(t(i)) and its 64-bit reciprocal.  A record of kTbFac
+// doubles per entry, its 2x2 blocks by rows so that the lane of component r
+// reads its row as one double2:
+//   [0..3]   adjugate of t(i): (t22, -t12), (-t21, t11)  (Div_2's numerators)
+//   [4..7]   l(i-1), the coupling to the previous row (0 in row 0)
+//   [8..11]  w(i) (0 in the last row)
+//   [12]     Det(t(i)); [13] its reciprocal for fpi::quot_rn
+constexpr int kTbFac = 14;
+
+__global__ void k_tb_factor(size_t nline, int n1, const double* __restrict__ d, const double* __restrict__ u,
+                            const double* __restrict__ l, double* __restrict__ fac) {
+  const size_t line = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (line >= nline) return;
+  const double *dc = d + line * n1 * 4, *uc = u + line * (n1 - 1) * 4, *lc = l + line * (n1 - 1) * 4;
+  double* f = fac + line * n1 * kTbFac;
+  M2 t = ld_m(dc), li{0.0, 0.0, 0.0, 0.0};
+  for (int i = 0; i < n1; ++i, f += kTbFac) {
+    const double dt = det(t);
+    const unsigned long long R = fpi::recip(dt);
+    st_v(f, V2{t.a22, -t.a12});
+    st_v(f + 2, V2{-t.a21, t.a11});
+    st_v(f + 4, V2{li.a11, li.a12});
+    st_v(f + 6, V2{li.a21, li.a22});
+    M2 w{0.0, 0.0, 0.0, 0.0};
+    if (i + 1 < n1) {  // Div_22(u, t), then t = d - l*w
+      const M2 ui = ld_m(uc + (size_t)i * 4);
+      w = M2{fpi::quot_rn(__dsub_rn(__dmul_rn(t.a22, ui.a11), __dmul_rn(t.a12, ui.a21)), dt, R),
+             fpi::quot_rn(__dadd_rn(__dmul_rn(-t.a21, ui.a11), __dmul_rn(t.a11, ui.a21)), dt, R),
+             fpi::quot_rn(__dsub_rn(__dmul_rn(t.a22, ui.a12), __dmul_rn(t.a12, ui.a22)), dt, R),
+             fpi::quot_rn(__dadd_rn(__dmul_rn(-t.a21, ui.a12), __dmul_rn(t.a11, ui.a22)), dt, R)};
+      li = ld_m(lc + (size_t)i * 4);
+      t = sub_m(ld_m(dc + (size_t)(i + 1) * 4), mult_22(li, w));
     }
-    st_v(xl + 2 * i, v);
+    st_v(f + 8, V2{w.a11, w.a12});
+    st_v(f + 10, V2{w.a21, w.a22});
+    st_v(f + 12, V2{dt, __longlong_as_double((long long)R)});
   }
-  solve_col(n1, d + line * n1 * 4, u1 + line * (n1 - 1) * 4, l1 + line * (n1 - 1) * 4, xl, w, ws);
 }
 
-__global__ void k_tri_tb_gs_2d_lines(int tr, int nplane, int n2, int n1, const double* __restrict__ d,
-                                     const double* __restrict__ u1, const double* __restrict__ l1,
-                                     const double* __restrict__ u2, const double* __restrict__ l2,
-                                     const double* __restrict__ b, double* __restrict__ x, int j0, int jstep,
-                                     int jcount, int bwd, double* __restrict__ w) {
-  const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nth = (size_t)nplane * jcount;
-  if (tid >= nth) return;
-  relax_line(tr, n2, n1, d, u1, l1, u2, l2, b, x, tid / jcount, j0 + (int)(tid % jcount) * jstep, bwd, w + tid, nth);
-}
-
-// Solve_2D on nplane planes in zebra order as one launch: one CTA per plane
-// runs all mult_iter V-cycles of its plane hierarchy, its threads taking the
-// lines of one parity (or the entries of a residual, restriction or
-// correction) between block barriers; every relaxation, residual and
-// transfer is the multi-launch path's arithmetic, so the bits are the same.
-constexpr int kPlaneHierMax = 12;
+constexpr int kTbLevMax = 24;
 struct PlaneHierDev {
   int nlev;
-  int n2[kPlaneHierMax], n1[kPlaneHierMax];
-  const double* a[kPlaneHierMax][5];
-  double *b[kPlaneHierMax], *x[kPlaneHierMax], *res[kPlaneHierMax];
+  int n2[kTbLevMax], n1[kTbLevMax];
+  const double* a[kTbLevMax][5];
+  const double* fac[kTbLevMax];
+  double *b[kTbLevMax], *x[kTbLevMax];
 };
 
-__global__ void __launch_bounds__(128) k_tb_plane_vcycles(int tr, int nplane, PlaneHierDev H, int gauss_iter2,
-                                                          int mult_iter, double* __restrict__ w) {
-  const size_t p = blockIdx.x;
-  if (p >= (size_t)nplane) return;
+// One zebra half-sweep over the lines of parity c of plane p (n2 lines of n1
+// rows): every line's right-hand side (forward (b - l x(j-1)) - u x(j+1),
+// backward (b - u x(j+1)) - l x(j-1)) is formed by the whole block and left in
+// x, then Solve_1D runs on it.  The lines of one parity read only lines of
+// the other.
+// What bounds the solve is its serial chain: an FP64 warp instruction takes
+// 64 cycles of a sub-partition, dependent or not.  Two lanes share a line, one
+// per component, so a row is seven FP64 instructions, a quotient on the
+// integer units and two exchanges with the partner lane forward, and four
+// instructions backward (one lane per line with its own factors: about 70
+// and 8).  The next row's operands are loaded while this row runs.
+__device__ __forceinline__ void tb_half(int tr, int n2, int n1, const double* __restrict__ l2,
+                                        const double* __restrict__ u2, const double* __restrict__ fac,
+                                        const double* b, double* x, int c, int bwd) {
+  const int nl = (n2 - c + 1) / 2, w1 = 2 * n1;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const size_t ws = (size_t)nplane * H.n2[0];  // one factor slot per line of the finest level
-  auto gs = [&](int l, int gi) {
-    const int n2 = H.n2[l], n1 = H.n1[l];
-    const double *d = H.a[l][0], *u1 = H.a[l][1], *l1 = H.a[l][2], *u2 = H.a[l][3], *l2 = H.a[l][4];
-    if (n2 > 1)
-      for (int it = 0; it < gi; ++it)
-        for (int half = 0; half < 4; ++half) {
-          const int par = half == 1 || half == 2;
-          for (int j = par + 2 * tid; j < n2; j += 2 * nt)
-            relax_line(tr, n2, n1, d, u1, l1, u2, l2, H.b[l], H.x[l], p, j, half >= 2, w + p * H.n2[0] + j, ws);
-          __syncthreads();
-        }
-    if (tid == 0) relax_line(tr, n2, n1, d, u1, l1, u2, l2, H.b[l], H.x[l], p, 0, 1, w + p * H.n2[0], ws);
-    __syncthreads();
-  };
-  for (int it = 0; it < mult_iter; ++it) {
-    int gi = 1, l = 0;
-    for (;;) {  // the way down (MULTI/TriDiagTB_Mod.f90:449-470)
-      gs(l, gi);
-      gi += gauss_iter2;
-      if (l + 1 == H.nlev) {
-        gi -= gauss_iter2;
-        break;
-      }
-      const int n2 = H.n2[l], n1 = H.n1[l];
-      const size_t np = (size_t)n2 * n1, base = p * np;
-      for (size_t e = tid; e < np; e += nt)
-        st_v(H.res[l] + (base + e) * 2,
-             sub_v(ld_v(H.b[l] + (base + e) * 2), level_entry(tr, nplane, n2, n1, H.a[l][0], H.a[l][1], H.a[l][2],
-                                                              H.a[l][3], H.a[l][4], nullptr, nullptr, H.x[l], base + e)));
-      __syncthreads();
-      const size_t npc = (size_t)H.n2[l + 1] * H.n1[l + 1], basec = p * npc;
-      for (size_t e = tid; e < npc; e += nt) {
-        restrict_2d_entry(n2, n1, H.res[l], H.b[l + 1], basec + e);
-        st_v(H.x[l + 1] + (basec + e) * 2, V2{0.0, 0.0});
-      }
-      __syncthreads();
-      ++l;
+  for (int e = tid; e < nl * w1; e += nt) {
+    const int q = e / w1, o = e - q * w1, r = o & 1;
+    const int j = 2 * q + c;
+    const size_t pos = (size_t)j * w1 + o;
+    const double bv = b[pos];
+    double ml = 0.0, mu = 0.0;  // a missing neighbour: t - 0 leaves every bit of t
+    auto mult = [&](const double* cp, const double* xn) {
+      return tr ? __dadd_rn(__dmul_rn(cp[r], xn[0]), __dmul_rn(cp[r + 2], xn[1])) : __dmul_rn(cp[r], xn[0]);
+    };
+    if (j > 0) ml = mult(l2 + ((size_t)(j - 1) * w1 + (o - r)) * 2, x + pos - r - w1);
+    if (j < n2 - 1) mu = mult(u2 + ((size_t)j * w1 + (o - r)) * 2, x + pos - r + w1);
+    x[pos] = bwd ? __dsub_rn(__dsub_rn(bv, mu), ml) : __dsub_rn(__dsub_rn(bv, ml), mu);
+  }
+  __syncthreads();
+  const int r = tid & 1;
+  for (int q0 = tid >> 1; (q0 & ~15) < nl; q0 += nt >> 1) {  // whole warps (16 lines) take part in the exchanges
+    const int q = min(q0, nl - 1);
+    const bool live = q0 < nl;
+    const int j = 2 * q + c;
+    double* xp = x + (size_t)j * w1 + r;
+    const double* fp = fac + (size_t)j * n1 * kTbFac;
+    auto pair = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
+    auto other = [](double v) { return __shfl_xor_sync(0xffffffffu, v, 1); };
+    double t = xp[0], c1 = 0.0, c2 = 0.0, y = 0.0;
+    double2 ad = pair(fp + 2 * r), l = pair(fp + 4 + 2 * r), dr = pair(fp + 12);
+    for (int i = 0; i < n1; ++i) {
+      const int in = i + 1 < n1 ? i + 1 : i;
+      const double* fn = fp + (size_t)in * kTbFac;
+      const double2 adn = pair(fn + 2 * r), ln = pair(fn + 4 + 2 * r), drn = pair(fn + 12);
+      const double tn = in > i ? xp[2 * in] : 0.0;
+      const double v = __dsub_rn(t, __dadd_rn(__dmul_rn(l.x, c1), __dmul_rn(l.y, c2)));
+      const double vo = other(v);
+      const double num = __dadd_rn(__dmul_rn(ad.x, r ? vo : v), __dmul_rn(ad.y, r ? v : vo));
+      y = fpi::quot_rn(num, dr.x, (unsigned long long)__double_as_longlong(dr.y));
+      if (live) xp[2 * i] = y;
+      const double yo = other(y);
+      c1 = r ? yo : y;
+      c2 = r ? y : yo;
+      t = tn;
+      ad = adn;
+      l = ln;
+      dr = drn;
     }
-    for (;;) {  // and up (:471-493)
-      gs(l, gi);
-      gi -= gauss_iter2;
-      if (l == 0) break;
-      --l;
-      const int n2 = H.n2[l], n1 = H.n1[l], n1c = (n1 + 1) / 2, n2c = (n2 + 1) / 2;
-      const size_t np = (size_t)n2 * n1;
-      for (size_t e = tid; e < np; e += nt) {
-        const int i = (int)(e % n1), j = (int)(e / n1);
-        const size_t q = (p * np + e) * 2;
-        st_v(H.x[l] + q, add_v(ld_v(H.x[l] + q), ld_v(H.x[l + 1] + ((p * n2c + j / 2) * n1c + i / 2) * 2)));
-      }
-      __syncthreads();
+    __syncwarp();
+    double2 w = make_double2(0.0, 0.0);
+    if (n1 > 1) {
+      t = xp[2 * (n1 - 2)];
+      w = pair(fp + (size_t)(n1 - 2) * kTbFac + 8 + 2 * r);
+    }
+    for (int i = n1 - 2; i >= 0; --i) {
+      const int in = i > 0 ? i - 1 : 0;
+      const double tn = xp[2 * in];
+      const double2 wn = pair(fp + (size_t)in * kTbFac + 8 + 2 * r);
+      y = __dsub_rn(t, __dadd_rn(__dmul_rn(w.x, c1), __dmul_rn(w.y, c2)));
+      if (live) xp[2 * i] = y;
+      const double yo = other(y);
+      c1 = r ? yo : y;
+      c2 = r ? y : yo;
+      t = tn;
+      w = wn;
     }
   }
+  __syncthreads();
 }
 
-// the right-hand sides of every plane of a level at once (zebra order of
-// GaussSeidel_3D): b(k) minus its couplings to planes k-1 and k+1 in the
-// forward or backward operation order
-__global__ void k_tri_tb_rhs3(int tr, int n3, size_t npl, const double* __restrict__ b,
-                              const double* __restrict__ u3, const double* __restrict__ l3,
-                              const double* __restrict__ x, int bwd, double* __restrict__ t) {
-  const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (e >= (size_t)n3 * npl) return;
-  const int k = (int)(e / npl);
-  const size_t r = e % npl;
-  V2 v = ld_v(b + e * 2);
-  const double* cl = k > 0 ? l3 + ((size_t)(k - 1) * npl + r) * 4 : nullptr;
-  const double* cu = k < n3 - 1 ? u3 + ((size_t)k * npl + r) * 4 : nullptr;
-  if (!bwd) {
-    if (cl) v = couple_sub(tr, v, cl, ld_v(x + (e - npl) * 2));
-    if (cu) v = couple_sub(tr, v, cu, ld_v(x + (e + npl) * 2));
-  } else {
-    if (cu) v = couple_sub(tr, v, cu, ld_v(x + (e + npl) * 2));
-    if (cl) v = couple_sub(tr, v, cl, ld_v(x + (e - npl) * 2));
+// GaussSeidel_2D of one plane in zebra order: gi iterations of the half-sweeps
+// even forward, odd forward, odd backward, even backward, then line 1 once
+// more.  A half-sweep that directly follows one of the same parity overwrites
+// its result unread, and line 1 once more repeats the last even half-sweep's
+// solve of it, so 2*gi + 1 half-sweeps give the same x.
+__device__ __noinline__ void tb_smooth(int tr, int n2, int n1, const double* l2, const double* u2, const double* fac,
+                                       const double* b, double* x, int gi) {
+  const int nh = n2 > 1 ? 2 * gi + 1 : 1;
+  for (int hs = 0; hs < nh; ++hs) tb_half(tr, n2, n1, l2, u2, fac, b, x, hs & 1, (hs & 1) || hs + 1 == nh);
+}
+
+// Solve_2D (mult_iter V-cycles of Multigrid_2D) on the planes k0, k0+kstep, ...
+// of a level, a CTA per plane: the plane's right-hand side b(k) minus its
+// couplings to planes k-1 and k+1 in the forward or backward operation order
+// (left in t), then the V-cycles in place on x; residual, restriction and
+// correction as in the multi-launch path, so the bits are the same.
+__global__ void __launch_bounds__(256) k_tb_planes(int tr, int n3, int k0, int kstep, int bwd, PlaneHierDev H,
+                                                   const double* __restrict__ u3, const double* __restrict__ l3,
+                                                   const double* __restrict__ b3, double* x3, double* t3,
+                                                   int gauss_iter2, int mult_iter) {
+  const int k = k0 + (int)blockIdx.x * kstep;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const size_t npl = (size_t)H.n2[0] * H.n1[0];
+  double* x0 = x3 + (size_t)k * npl * 2;
+  double* t0 = t3 + (size_t)k * npl * 2;
+  for (size_t e = tid; e < npl; e += nt) {
+    V2 v = ld_v(b3 + ((size_t)k * npl + e) * 2);
+    const double* cl = k > 0 ? l3 + ((size_t)(k - 1) * npl + e) * 4 : nullptr;
+    const double* cu = k < n3 - 1 ? u3 + ((size_t)k * npl + e) * 4 : nullptr;
+    if (!bwd && cl) v = couple_sub(tr, v, cl, ld_v(x0 - npl * 2 + e * 2));
+    if (cu) v = couple_sub(tr, v, cu, ld_v(x0 + npl * 2 + e * 2));
+    if (bwd && cl) v = couple_sub(tr, v, cl, ld_v(x0 - npl * 2 + e * 2));
+    st_v(t0 + e * 2, v);
   }
-  st_v(t + e * 2, v);
+  __syncthreads();
+  auto X = [&](int l) { return l == 0 ? x0 : H.x[l] + (size_t)k * H.n2[l] * H.n1[l] * 2; };
+  auto B = [&](int l) { return l == 0 ? t0 : H.b[l] + (size_t)k * H.n2[l] * H.n1[l] * 2; };
+  auto blk = [&](int l, int q) {  // plane k's part of array q of level l
+    const size_t n2 = H.n2[l], n1 = H.n1[l];
+    return H.a[l][q] + (size_t)k * (q == 0 ? n2 * n1 : (q < 3 ? n2 * (n1 - 1) : (n2 - 1) * n1)) * 4;
+  };
+  auto smooth = [&](int l, int gi) {
+    tb_smooth(tr, H.n2[l], H.n1[l], blk(l, 4), blk(l, 3), H.fac[l] + (size_t)k * H.n2[l] * H.n1[l] * kTbFac, B(l), X(l),
+              gi);
+  };
+  for (int it = 0; it < mult_iter; ++it) {
+    int gi = 1;
+    for (int l = 0; l < H.nlev; ++l) {  // the way down (MULTI/TriDiagTB_Mod.f90:449-470)
+      smooth(l, gi);
+      if (l + 1 == H.nlev) break;
+      gi += gauss_iter2;
+      const int n2 = H.n2[l], n1 = H.n1[l];
+      const double *b = B(l), *x = X(l), *d = blk(l, 0), *u1 = blk(l, 1), *l1 = blk(l, 2), *u2 = blk(l, 3), *l2 = blk(l, 4);
+      double *bc = B(l + 1), *xc = X(l + 1);
+      const size_t npc = (size_t)H.n2[l + 1] * H.n1[l + 1];
+      for (size_t e = tid; e < npc; e += nt) {
+        restrict_2d_entry_of(n2, n1, [&](int i, int j) {
+          const size_t q = (size_t)j * n1 + i;
+          return sub_v(ld_v(b + q * 2), level_entry(tr, 1, n2, n1, d, u1, l1, u2, l2, nullptr, nullptr, x, q));
+        }, bc, e);
+        st_v(xc + e * 2, V2{0.0, 0.0});
+      }
+      __syncthreads();
+    }
+    for (int l = H.nlev - 1;; --l) {  // and up (:471-493)
+      smooth(l, gi);
+      gi -= gauss_iter2;
+      if (l == 0) break;
+      const int n2 = H.n2[l - 1], n1 = H.n1[l - 1], n1c = (n1 + 1) / 2;
+      double* x = X(l - 1);
+      const double* xc = X(l);
+      for (int e = tid; e < n2 * n1; e += nt) {
+        const int j = e / n1, i = e - j * n1;
+        st_v(x + (size_t)e * 2, add_v(ld_v(x + (size_t)e * 2), ld_v(xc + ((size_t)(j / 2) * n1c + i / 2) * 2)));
+      }
+      __syncthreads();
+    }
+  }
 }
 
 struct DevBufs {
@@ -938,16 +1024,12 @@ struct PlaneLevel {
   int n2 = 0, n1 = 0;
   const double* a[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   double *b = nullptr, *x = nullptr, *res = nullptr;
+  double* fac = nullptr;  // zebra order: the elimination factors (k_tb_factor)
 };
 // the smoother's per-plane scratch, sized for the finest plane
 struct Scratch {
   double *t, *w;
-  // zebra order: the line solves' factors (nplane x ceil(n2/2) lines of the
-  // finest plane level), every plane's right-hand side and a copy of x
-  double *wz = nullptr, *tall = nullptr, *xtmp = nullptr;
-  // the one-launch plane V-cycle's factors: a slot per line of the finest
-  // plane level of every plane
-  double* wl = nullptr;
+  double* tall = nullptr;  // zebra order: every plane's right-hand side
 };
 
 size_t plane_block_len(int nplane, int n2, int n1) {
@@ -999,51 +1081,14 @@ cudaError_t stage_plane_level(PlaneLevel& L, int nplane, int n2, int n1, const d
 // coarse levels' b, x and every residual are work space.  Kernels on the
 // legacy stream, the level loop here.
 cudaError_t plane_cycles(int variant, int nplane, int nlev, PlaneLevel* lv, const Scratch& sc, int gauss_iter2,
-                         int mult_iter, long& launches, int zebra = 0) {
-  if (zebra && sc.wl && nlev <= kPlaneHierMax) {  // the whole Solve_2D as one launch, a CTA per plane
-    PlaneHierDev H;
-    H.nlev = nlev;
-    for (int l = 0; l < nlev; ++l) {
-      H.n2[l] = lv[l].n2;
-      H.n1[l] = lv[l].n1;
-      for (int q = 0; q < 5; ++q) H.a[l][q] = lv[l].a[q];
-      H.b[l] = lv[l].b;
-      H.x[l] = lv[l].x;
-      H.res[l] = lv[l].res;
-    }
-    k_tb_plane_vcycles<<<nplane, 128>>>(variant, nplane, H, gauss_iter2, mult_iter, sc.wl);
-    ++launches;
-    return cudaGetLastError();
-  }
+                         int mult_iter, long& launches) {
   auto grid = [&](const PlaneLevel& L) { return (unsigned)(((size_t)nplane * L.n2 * L.n1 + 255) / 256); };
-  // GaussSeidel_2D of one level in zebra order: four half-sweeps per
-  // iteration, then line 1 with the backward right-hand side
-  auto gs_zebra = [&](const PlaneLevel& L, int gi) {
-    auto lines = [&](int j0, int jstep, int jcount, int bwd) {
-      const size_t nth = (size_t)nplane * jcount;
-      k_tri_tb_gs_2d_lines<<<(unsigned)((nth + 127) / 128), 128>>>(variant, nplane, L.n2, L.n1, L.a[0], L.a[1], L.a[2],
-                                                                   L.a[3], L.a[4], L.b, L.x, j0, jstep, jcount, bwd,
-                                                                   sc.wz);
-      ++launches;
-    };
-    if (L.n2 > 1)
-      for (int it = 0; it < gi; ++it)
-        for (int half = 0; half < 4; ++half) {
-          const int par = half == 1 || half == 2;
-          lines(par, 2, (L.n2 - par + 1) / 2, half >= 2);
-        }
-    lines(0, 1, 1, 1);
-  };
 #define TB_LEVEL(L) variant, nplane, (L).n2, (L).n1, (L).a[0], (L).a[1], (L).a[2], (L).a[3], (L).a[4]
   for (int it = 0; it < mult_iter; ++it) {
     int gi = 1, l = 0;
     for (;;) {  // the way down (:449-470)
-      if (zebra) {
-        gs_zebra(lv[l], gi);
-      } else {
-        k_tri_tb_gs_2d<<<(nplane + 63) / 64, 64>>>(TB_LEVEL(lv[l]), lv[l].b, lv[l].x, gi, sc.t, sc.w);
-        ++launches;
-      }
+      k_tri_tb_gs_2d<<<(nplane + 63) / 64, 64>>>(TB_LEVEL(lv[l]), lv[l].b, lv[l].x, gi, sc.t, sc.w);
+      ++launches;
       gi += gauss_iter2;
       if (l + 1 == nlev) {
         gi -= gauss_iter2;
@@ -1057,12 +1102,8 @@ cudaError_t plane_cycles(int variant, int nplane, int nlev, PlaneLevel* lv, cons
       ++l;
     }
     for (;;) {  // and up (:471-493)
-      if (zebra) {
-        gs_zebra(lv[l], gi);
-      } else {
-        k_tri_tb_gs_2d<<<(nplane + 63) / 64, 64>>>(TB_LEVEL(lv[l]), lv[l].b, lv[l].x, gi, sc.t, sc.w);
-        ++launches;
-      }
+      k_tri_tb_gs_2d<<<(nplane + 63) / 64, 64>>>(TB_LEVEL(lv[l]), lv[l].b, lv[l].x, gi, sc.t, sc.w);
+      ++launches;
       gi -= gauss_iter2;
       if (l == 0) break;
       --l;
@@ -1096,7 +1137,7 @@ cudaError_t level_gs(int variant, int n3, const PlaneLevel* pl, int nlev2, const
     }
     one[0].b = const_cast<double*>(rhs);
     one[0].x = x + (size_t)k * npl * 2;
-    return plane_cycles(variant, 1, nlev2, one, sc, gauss_iter2, mult_iter2, launches, zebra);
+    return plane_cycles(variant, 1, nlev2, one, sc, gauss_iter2, mult_iter2, launches);
   };
   const unsigned g = (unsigned)((npl + 255) / 256);
   auto couple = [&](const double* tin, const double* c, const double* xn) {
@@ -1112,30 +1153,30 @@ cudaError_t level_gs(int variant, int n3, const PlaneLevel* pl, int nlev2, const
   auto B = [&](int k) { return b + (size_t)k * npl * 2; };
   auto U = [&](int k) { return u3 + (size_t)k * npl * 4; };
   auto Lo = [&](int k) { return l3 + (size_t)k * npl * 4; };
-  if (n3 > 1 && zebra) {
-    // the planes of one parity at once: every plane's right-hand side, the 2D
-    // V-cycles of all planes on a copy of x, the parity's planes copied back
-    const size_t nv = (size_t)n3 * npl * 2;
-    const unsigned g3 = (unsigned)((n3 * npl + 255) / 256);
-    PlaneLevel all[32];
-    for (int m = 0; m < nlev2; ++m) all[m] = pl[m];
-    all[0].b = sc.tall;
-    all[0].x = sc.xtmp;
-    for (int it = 0; it < gauss_iter; ++it)
+  if (zebra) {
+    // the planes of one parity at once, each CTA one plane; then plane 1 and
+    // plane n3 once more (they share no neighbour update when n3 > 2)
+    PlaneHierDev H;
+    H.nlev = nlev2;
+    for (int m = 0; m < nlev2; ++m) {
+      H.n2[m] = pl[m].n2;
+      H.n1[m] = pl[m].n1;
+      for (int q = 0; q < 5; ++q) H.a[m][q] = pl[m].a[q];
+      H.fac[m] = pl[m].fac;
+      H.b[m] = pl[m].b;
+      H.x[m] = pl[m].x;
+    }
+    auto planes = [&](int k0, int kstep, int count, int bwd) {
+      k_tb_planes<<<count, 256>>>(variant, n3, k0, kstep, bwd, H, u3, l3, b, x, sc.tall, gauss_iter2, mult_iter2);
+      ++launches;
+    };
+    for (int it = 0; it < gauss_iter && n3 > 1; ++it)
       for (int half = 0; half < 4; ++half) {
         const int par = half == 1 || half == 2;
-        k_tri_tb_rhs3<<<g3, 256>>>(variant, n3, npl, b, u3, l3, x, half >= 2, sc.tall);
-        ++launches;
-        TB_CHECK(cudaMemcpyAsync(sc.xtmp, x, nv * sizeof(double), cudaMemcpyDeviceToDevice));
-        TB_CHECK(plane_cycles(variant, n3, nlev2, all, sc, gauss_iter2, mult_iter2, launches, 1));
-        TB_CHECK(cudaMemcpy2DAsync(x + par * npl * 2, 2 * npl * 2 * sizeof(double), sc.xtmp + par * npl * 2,
-                                   2 * npl * 2 * sizeof(double), npl * 2 * sizeof(double), (n3 - par + 1) / 2,
-                                   cudaMemcpyDeviceToDevice));
+        planes(par, 2, (n3 - par + 1) / 2, half >= 2);
       }
-    couple(B(0), U(0), X(1));
-    TB_CHECK(solve(0, t));
-    couple(B(n3 - 1), Lo(n3 - 2), X(n3 - 2));
-    TB_CHECK(solve(n3 - 1, t));
+    planes(0, n3 - 1, n3 > 2 ? 2 : 1, 1);
+    if (n3 == 2) planes(1, 1, 1, 1);
   } else if (n3 > 1) {
     for (int it = 0; it < gauss_iter; ++it) {
       TB_CHECK(cudaMemcpyAsync(t, b, npl * 2 * sizeof(double), cudaMemcpyDeviceToDevice));
@@ -1551,22 +1592,24 @@ int asam_tri_tb_hier_create(int variant, int ref_level, int n3, int n2, int n1, 
     h->nlev2s[L] = ref_level - L;
     for (int m = 0; m < h->nlev2s[L]; ++m)
       tot += plane_block_len(h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m)) +
-             3 * plane_vec_len(h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m));
+             3 * plane_vec_len(h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m)) +
+             (size_t)h->n3s[L] * cdiv(n2, L + m) * cdiv(n1, L + m) * kTbFac;
     tot += 2 * (size_t)(h->n3s[L] - 1) * h->n2s[L] * h->n1s[L] * 4;
   }
   const size_t npl = (size_t)n2 * n1, nc = (size_t)n3 * npl;
   const size_t nz = (size_t)n3 * n2 * (n1 + 1), nx = (size_t)n3 * (n2 + 1) * n1, ny = (size_t)(n3 + 1) * npl;
   const size_t nt = (size_t)n1 * 2, nw = (size_t)(n1 > 1 ? n1 - 1 : 1) * 4;
   const size_t fields = 4 * (nz + nx + ny) + 3 * nc;  // the finest fields, and room for one coarsening of them
-  const size_t nwz = (size_t)n3 * ((n2 + 1) / 2) * (n1 > 1 ? n1 - 1 : 1) * 4;
-  const size_t nwl = (size_t)n3 * n2 * (n1 > 1 ? n1 - 1 : 1) * 4;
-  TCU(cudaMalloc((void**)&h->mem, (tot + npl * 2 + nt + nw + nwz + 2 * nc * 2 + nwl) * sizeof(double)));
+  TCU(cudaMalloc((void**)&h->mem, (tot + npl * 2 + nt + nw + nc * 2) * sizeof(double)));
   DevBufs work;
   TCU(cudaMalloc((void**)&work.p[0], 2 * fields * sizeof(double)));
   double* cur = h->mem;
   for (int L = 0; L < ref_level; ++L) {
-    for (int m = 0; m < h->nlev2s[L]; ++m)
+    for (int m = 0; m < h->nlev2s[L]; ++m) {
       TCU(stage_plane_level(h->pl[L][m], h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m), nullptr, cur));
+      h->pl[L][m].fac = cur;
+      cur += (size_t)h->n3s[L] * cdiv(n2, L + m) * cdiv(n1, L + m) * kTbFac;
+    }
     const size_t ncp = (size_t)(h->n3s[L] - 1) * h->n2s[L] * h->n1s[L] * 4;
     h->du3[L] = ncp ? cur : nullptr;
     h->dl3[L] = ncp ? cur + ncp : nullptr;
@@ -1574,10 +1617,7 @@ int asam_tri_tb_hier_create(int variant, int ref_level, int n3, int n2, int n1, 
   }
   h->t = cur;
   h->sc = Scratch{cur + npl * 2, cur + npl * 2 + nt};
-  h->sc.wz = cur + npl * 2 + nt + nw;
-  h->sc.tall = h->sc.wz + nwz;
-  h->sc.xtmp = h->sc.tall + nc * 2;
-  h->sc.wl = h->sc.xtmp + nc * 2;
+  h->sc.tall = cur + npl * 2 + nt + nw;
   // the finest fields on the device
   TbFields g;
   double* fp = work.p[0];
@@ -1626,7 +1666,9 @@ int asam_tri_tb_hier_create(int variant, int ref_level, int n3, int n2, int n1, 
                                                                    const_cast<double*>(P.a[0]),
                                                                    couple ? h->du3[L3] : nullptr,
                                                                    couple ? h->dl3[L3] : nullptr);
-      launches += 3;
+      const size_t nline = (size_t)c3 * c2;
+      k_tb_factor<<<(unsigned)((nline + 63) / 64), 64>>>(nline, c1, P.a[0], P.a[1], P.a[2], P.fac);
+      launches += 4;
       TCU(cudaGetLastError());
     }
   TCU(cudaDeviceSynchronize());

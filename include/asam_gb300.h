@@ -549,8 +549,9 @@ int asam_probe_fp64_fma(int iters, double *gflops);
 
 /* Diagnostic: count operand pairs (n pseudo-random pairs, exponents within
  * +-span binades) where the library's FMA-corrected quotient from a
- * precomputed reciprocal differs from the IEEE quotient (no reference
- * counterpart; guards the bit-exact FP64 path). */
+ * precomputed reciprocal differs from the IEEE quotient, or its integer-unit
+ * product or quotient (special operands mixed in) from the IEEE one (no
+ * reference counterpart; guards the bit-exact FP64 path). */
 int asam_probe_div(long long n, long long seed, int span, long long *mismatches);
 
 /* Batched block-tridiagonal column solve of the density/buoyancy-coupled
