@@ -5,6 +5,7 @@
 // its own copy, and the launch wrappers of launch.h are the only exports.
 #pragma once
 #include "asam_common.cuh"
+#include "fp64_int.cuh"
 #include "launch.h"
 
 namespace {
@@ -1967,8 +1968,15 @@ __global__ void k_scale_host(size_t len, T a, T* __restrict__ y) {
 // chunk from the tile, with the reference's operations in its order, and the
 // elimination factors w and the forward values are written back through the
 // tile the same way; the back substitution walks the chunks downwards.
+//
+// What bounds it: per row two quotients by the same pivot, which FP64
+// instructions would compute in some 25 of the 64-cycle slots a sub-partition
+// has for a warp.  Here the pivot's reciprocal and the quotients run on the integer
+// units (fp64_int.cuh), as does the product off the pivot's chain, so a row
+// costs the chain reciprocal - quotient - product - difference; the next
+// chunk is copied by cp.async while this one is solved, and a block is one
+// warp, so that few columns still spread over the SMs.
 constexpr int kTriRows = 8;
-constexpr int kTriWarps = 4;  // warps per block, each independent
 constexpr int kTriPitch = 34;
 
 template <typename T>
@@ -1979,7 +1987,7 @@ __device__ __forceinline__ void tri_tile_load(T (*tile)[kTriPitch], const T* __r
   for (int e = lane; e < 32 * kTriRows; e += 32) {
     const int c = e / kTriRows, r = e % kTriRows;
     const int row = r0 + r;
-    if (c0 + c < ncol && row >= 0 && row < nrow) tile[r][c] = src[(size_t)(c0 + c) * stride + row];
+    if (c0 + c < ncol && row >= 0 && row < nrow) cp_async_elem(&tile[r][c], src + (size_t)(c0 + c) * stride + row, true);
   }
 }
 template <typename T>
@@ -1992,41 +2000,58 @@ __device__ __forceinline__ void tri_tile_store(const T (*tile)[kTriPitch], T* __
     if (c0 + c < ncol && row >= 0 && row < nrow) dst[(size_t)(c0 + c) * stride + row] = tile[r][c];
   }
 }
+// the pivot with its reciprocal, quotients by it and the product off its chain
+__device__ __forceinline__ unsigned long long tri_recip(double t) { return fpi::recip(t); }
+__device__ __forceinline__ double tri_quot(double x, double t, unsigned long long R) { return fpi::quot_rn(x, t, R); }
+__device__ __forceinline__ double tri_mul(double a, double b) { return fpi::mul_rn(a, b); }
+__device__ __forceinline__ unsigned long long tri_recip(float) { return 0; }
+__device__ __forceinline__ float tri_quot(float x, float t, unsigned long long) { return x / t; }
+__device__ __forceinline__ float tri_mul(float a, float b) { return a * b; }
 
 template <typename T>
-__global__ void __launch_bounds__(32 * kTriWarps) k_tri_solve_w(int ncol, int n1, const T* __restrict__ dd,
-                                                                 const T* __restrict__ uu, const T* __restrict__ ll,
-                                                                 T* __restrict__ bb, T* __restrict__ ww) {
-  __shared__ T sh[kTriWarps][4][kTriRows][kTriPitch];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c0 = (blockIdx.x * kTriWarps + warp) * 32;
-  if (c0 >= ncol) return;  // uniform over the warp
-  T(*td)[kTriPitch] = sh[warp][0];
-  T(*tu)[kTriPitch] = sh[warp][1];  // u(i-1) in, w(i-1) out
-  T(*tl)[kTriPitch] = sh[warp][2];  // l(i-1)
-  T(*tb)[kTriPitch] = sh[warp][3];  // b(i) in, forward value out
+__global__ void __launch_bounds__(32) k_tri_solve_w(int ncol, int n1, const T* __restrict__ dd,
+                                                    const T* __restrict__ uu, const T* __restrict__ ll, T* bb, T* ww) {
+  __shared__ T sh[2][4][kTriRows][kTriPitch];
+  const int lane = threadIdx.x;
+  const int c0 = blockIdx.x * 32;
   const int m = n1 - 1;      // length of u, l and w's used part
   const bool live = c0 + lane < ncol;
   T t = (T)0, g = (T)0;
+  unsigned long long R = 0;
   // forward elimination, rows [r0, r0 + kTriRows); u, l and w at rows r0-1 ...
-  for (int r0 = 0; r0 < n1; r0 += kTriRows) {
-    tri_tile_load(td, dd, n1, c0, ncol, r0, n1, lane);
-    tri_tile_load(tb, bb, n1, c0, ncol, r0, n1, lane);
-    tri_tile_load(tu, uu, m, c0, ncol, r0 - 1, m, lane);
-    tri_tile_load(tl, ll, m, c0, ncol, r0 - 1, m, lane);
+  auto load = [&](int buf, int r0) {
+    if (r0 < n1) {
+      tri_tile_load(sh[buf][0], dd, n1, c0, ncol, r0, n1, lane);
+      tri_tile_load(sh[buf][1], uu, m, c0, ncol, r0 - 1, m, lane);
+      tri_tile_load(sh[buf][2], ll, m, c0, ncol, r0 - 1, m, lane);
+      tri_tile_load(sh[buf][3], (const T*)bb, n1, c0, ncol, r0, n1, lane);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  load(0, 0);
+  int buf = 0;
+  for (int r0 = 0; r0 < n1; r0 += kTriRows, buf ^= 1) {
+    load(buf ^ 1, r0 + kTriRows);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncwarp();
+    T(*td)[kTriPitch] = sh[buf][0];
+    T(*tu)[kTriPitch] = sh[buf][1];  // u(i-1) in, w(i-1) out
+    T(*tl)[kTriPitch] = sh[buf][2];  // l(i-1)
+    T(*tb)[kTriPitch] = sh[buf][3];  // b(i) in, forward value out
     if (live) {
       const int nr = min(kTriRows, n1 - r0);
       for (int r = 0; r < nr; ++r) {
-        const int i = r0 + r;
-        if (i == 0) {
+        if (r0 + r == 0) {
           t = td[r][lane];
-          g = tb[r][lane] / t;
+          R = tri_recip(t);
+          g = tri_quot(tb[r][lane], t, R);
         } else {
-          const T wi = tu[r][lane] / t;
+          const T li = tl[r][lane], wi = tri_quot(tu[r][lane], t, R);
+          const T bm = tb[r][lane] - tri_mul(li, g);
           tu[r][lane] = wi;
-          t = td[r][lane] - tl[r][lane] * wi;
-          g = (tb[r][lane] - tl[r][lane] * g) / t;
+          t = td[r][lane] - li * wi;
+          R = tri_recip(t);
+          g = tri_quot(bm, t, R);
         }
         tb[r][lane] = g;
       }
@@ -2037,15 +2062,27 @@ __global__ void __launch_bounds__(32 * kTriWarps) k_tri_solve_w(int ncol, int n1
     __syncwarp();
   }
   // back substitution x(i) = g(i) - w(i) x(i+1), i = n1-2 ... 0, chunks downwards
+  auto load_back = [&](int q, int r0) {
+    if (r0 >= 0) {
+      tri_tile_load(sh[q][0], (const T*)bb, n1, c0, ncol, r0, m, lane);
+      tri_tile_load(sh[q][1], (const T*)ww, n1, c0, ncol, r0, m, lane);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
   T x = g;  // x(n1-1) = g(n1-1), already stored
-  for (int r0 = ((m - 1) / kTriRows) * kTriRows; m > 0 && r0 >= 0; r0 -= kTriRows) {
-    tri_tile_load(tb, bb, n1, c0, ncol, r0, m, lane);
-    tri_tile_load(tu, ww, n1, c0, ncol, r0, m, lane);
+  const int last = m > 0 ? ((m - 1) / kTriRows) * kTriRows : -1;
+  load_back(0, last);
+  buf = 0;
+  for (int r0 = last; r0 >= 0; r0 -= kTriRows, buf ^= 1) {
+    load_back(buf ^ 1, r0 - kTriRows);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncwarp();
+    T(*tb)[kTriPitch] = sh[buf][0];
+    T(*tw)[kTriPitch] = sh[buf][1];
     if (live) {
       const int nr = min(kTriRows, m - r0);
       for (int r = nr - 1; r >= 0; --r) {
-        x = tb[r][lane] - tu[r][lane] * x;
+        x = tb[r][lane] - tw[r][lane] * x;
         tb[r][lane] = x;
       }
     }

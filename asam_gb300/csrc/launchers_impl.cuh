@@ -227,8 +227,7 @@ inline int gs_grid(const asam::Launch& L, size_t n) {
     k_scale_host<T><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, a, y); count_launches(1);                                          \
   }                                                                                                                \
   void launch_tri_solve(const Launch& L, int ncol, int n1, const T* dd, const T* uu, const T* ll, T* bb, T* ww) {  \
-    k_tri_solve_w<T><<<(ncol + 32 * kTriWarps - 1) / (32 * kTriWarps), 32 * kTriWarps, 0, L.stream>>>(             \
-        ncol, n1, dd, uu, ll, bb, ww);                                                                             \
+    k_tri_solve_w<T><<<(ncol + 31) / 32, 32, 0, L.stream>>>(ncol, n1, dd, uu, ll, bb, ww);                         \
     count_launches(1);                                                                                             \
   }                                                                                                                \
   void launch_tri_matvec(const Launch& L, int ncol, int n1, const T* dd, const T* uu, const T* ll, const T* xx,    \
