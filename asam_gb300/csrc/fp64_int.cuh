@@ -29,6 +29,8 @@ typedef unsigned long long u64;
 // are normal
 __device__ __forceinline__ bool in_range(unsigned hi) { return (hi & 0x7fffffffu) - (543u << 20) < (961u << 20); }
 
+__device__ __forceinline__ bool finite(unsigned hi) { return (hi & 0x7ff00000u) != 0x7ff00000u; }
+
 // significand with the leading one at bit 63
 __device__ __forceinline__ u64 left_sig(unsigned hi, unsigned lo) {
   const unsigned h = __funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, 11);
@@ -43,8 +45,7 @@ __device__ __forceinline__ double mul_rn(double a, double b) {
   const unsigned ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b), bl = __double2loint(b);
   const unsigned sign = (ah ^ bh) & 0x80000000u;
   if (!(in_range(ah) && in_range(bh))) {
-    if ((((ah << 1) | al) == 0 && in_range(bh)) || (((bh << 1) | bl) == 0 && in_range(ah)))
-      return __hiloint2double(sign, 0);
+    if ((((ah << 1) | al) == 0 || ((bh << 1) | bl) == 0) && finite(ah) && finite(bh)) return __hiloint2double(sign, 0);
     return mul_special(a, b);
   }
   const unsigned A1 = __funnelshift_l(al, (ah & 0xfffffu) | 0x100000u, 11), A0 = al << 11;

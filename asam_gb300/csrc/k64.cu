@@ -24,10 +24,16 @@ __global__ void k_cvt_d2f_scaled(size_t len, const double* __restrict__ x, doubl
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x)
     y[q] = (float)(s * x[q]);
 }
-// slot 7 of the DIA storage: 1/diagonal (IEEE division)
+// slots 7 and 8 of the DIA storage: 1/diagonal (correctly rounded) and its
+// 64-bit reciprocal
 __global__ void k_recip_diag(size_t n, double* __restrict__ val) {
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    val[7 * n + q] = 1.0 / val[3 * n + q];
+  {
+    const double dg = val[3 * n + q];
+    const unsigned long long R = fpi::recip(dg);
+    val[7 * n + q] = fpi::quot_rn(1.0, dg, R);
+    val[8 * n + q] = __longlong_as_double((long long)R);
+  }
 }
 }  // namespace
 

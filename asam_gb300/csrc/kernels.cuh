@@ -769,11 +769,17 @@ __global__ void k_jac(Dims d, GeomT<T> g, const T* __restrict__ rho, const T* __
     if (ii && kk && j == ny + 1) dg = dg - v[5];
     if (ii && jj && k == 0) dg = dg - v[0];
     if (ii && jj && k == nz + 1) dg = dg - v[6];
-    // scale to I - beta0*dt*J (:1857-1862); slot 7 holds 1/diagonal for the
-    // correctly rounded divisions of the Gauss-Seidel sweeps
+    // scale to I - beta0*dt*J (:1857-1862); slot 7 holds 1/diagonal, slot 8 (FP64)
+    // its 64-bit reciprocal for the quotients of the Gauss-Seidel sweeps
     const T diag = (T)1 - bdt * dg;
     val[3 * n + P] = diag;
-    val[7 * n + P] = (T)1 / diag;
+    if constexpr (sizeof(T) == 8) {
+      const unsigned long long R = fpi::recip(diag);
+      val[7 * n + P] = fpi::quot_rn(1.0, diag, R);
+      val[8 * n + P] = __longlong_as_double((long long)R);
+    } else {
+      val[7 * n + P] = (T)1 / diag;
+    }
     val[0 * n + P] = -(bdt * v[0]);
     val[1 * n + P] = -(bdt * v[1]);
     val[2 * n + P] = -(bdt * v[2]);
@@ -852,15 +858,48 @@ constexpr int GS_TZ = 4;
 // one launch the tile levels read and written in each buffer are disjoint.
 // Per cell the operation order is the reference's: b, U part (columns r+1,
 // r+NX, r+NXY), L part (columns r-NXY, r-NX, r-1), division.
-// Variant for the FP64 pipe (occupancy matters more than latency): each
-// thread prefetches its next two cells' operands into registers, two
-// hyperplanes ahead; no shared memory, so many tiles fit on an SM.
-template <typename TM, typename T>
-__global__ void __launch_bounds__(256) k_gs_pipe_reg(Dims d, int ncomp, const TM* __restrict__ val,
-                                                     const T* __restrict__ b, T* buf_last, T* buf_other, int tau,
-                                                     int nsweep, int ntx, int nty, int ntz, int nlev) {
-  static_assert(GS_TY * GS_TZ == 16, "one component's tile lines fill half a warp");
-  const int s = blockIdx.z;
+//
+// The FP64 kernel: one CTA per tile of kGsTx x 4 x 4 cells, sweep and group of
+// components.  What bounds a tile is the FP64 unit (a warp instruction takes 64
+// cycles of a sub-partition, dependent or not) along the tile's kGsTx + 6
+// hyperplanes, on which only the lower part has to wait:
+//   1. the block forms t = b - U x^{s-1} of all cells (coalesced loads, all
+//      lanes busy, the products on the integer units beside the FP64
+//      differences) and copies the lower part's coefficients, the diagonal,
+//      its reciprocal (slot 8) and the neighbour tiles' x^s faces to shared memory;
+//   2. a half-warp per component walks the hyperplanes from shared memory:
+//      three products and differences and the quotient, which runs on the
+//      integer units (fp64_int.cuh; the same bits);
+//   3. the block stores x^s.
+// A line's row pitch of kGsTx + 5 gives the 16 lines of a half-warp, each at its
+// own hyperplane offset, 16 different banks.
+constexpr int kGsTx = 16;
+constexpr int kGsBlock = 256;  // one thread per cell in phases 1 and 3
+constexpr int kGsPitch = kGsTx + 5;
+constexpr int kGsLines = GS_TY * GS_TZ;
+// values per component: t (then x^s), the faces below, south and west
+constexpr int kGsComp = kGsLines * kGsPitch + 2 * 4 * kGsTx + 16;
+constexpr int kGsCoef = 5 * kGsLines * kGsPitch;  // l0, l1, l2, diagonal, reciprocal
+inline size_t gs_tile_elems(int ncomp) { return (size_t)kGsCoef + (size_t)ncomp * kGsComp; }
+
+__device__ __forceinline__ double gs_mul(double a, double b) { return fpi::mul_rn(a, b); }
+__device__ __forceinline__ float gs_mul(float a, float b) { return a * b; }
+__device__ __forceinline__ double gs_quot(double t, double d, double r) {
+  return fpi::quot_rn(t, d, (unsigned long long)__double_as_longlong(r));
+}
+__device__ __forceinline__ float gs_quot(float t, float d, float r) { return div_rn(t, d, r); }
+
+template <typename TM, typename T, bool kIntL>
+__global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int group, const TM* __restrict__ val,
+                                                      const T* __restrict__ b, T* buf_last, T* buf_other, int tau,
+                                                      int nsweep, int ntx, int nty, int ntz, int nlev) {
+  static_assert(kGsLines == 16 && kGsTx * kGsLines == kGsBlock, "a half-warp holds a component's lines, a thread a cell");
+  extern __shared__ __align__(16) unsigned char gs_raw[];
+  T* coef = reinterpret_cast<T*>(gs_raw);
+  T* comp = coef + kGsCoef;
+  const int s = blockIdx.z % nsweep;
+  const int g0 = blockIdx.z / nsweep * group;  // this block's components: g0 .. g0+ncomp-1
+  const int ncomp = min(group, ncomp_all - g0);
   const int L = tau - 2 * s;
   if (L < 0 || L >= nlev) return;
   const int K = blockIdx.y;
@@ -872,76 +911,89 @@ __global__ void __launch_bounds__(256) k_gs_pipe_reg(Dims d, int ncomp, const TM
   const size_t n = d.npad();
   const size_t sy = (size_t)NX, sz = (size_t)NX * NY;
   const bool last_parity = ((nsweep - 1 - s) & 1) == 0;
-  T* xn_all = last_parity ? buf_last : buf_other;        // x^s
-  const T* xo_all = last_parity ? buf_other : buf_last;  // x^{s-1}
-  // lane = tb + GS_TY*tc + 16*(ic&1): the y-neighbour line is lane-1 and the
-  // z-neighbour line lane-GS_TY, both in this warp
-  const int lb = threadIdx.x % (GS_TY * GS_TZ);
-  const int ic = threadIdx.x / (GS_TY * GS_TZ);
-  const int tb = lb % GS_TY, tc = lb / GS_TY;
-  const int j = J * GS_TY + tb, k = K * GS_TZ + tc;
-  const bool line_ok = ic < ncomp && j < NY && k < NZ;
-  const size_t off = (size_t)(line_ok ? ic : 0) * n;
-  const T* bb = b + off;
-  T* xn = xn_all + off;
-  const T* xo = xo_all + off;
-  const int i0 = I * GS_TX;
-  const size_t rowP = sy * (size_t)j + sz * (size_t)k;
-  const bool up = s > 0;
-
-  // operands of one cell that do not depend on this sweep's current results
-  struct Cell {
-    T bb, u4, u5, u6, xo4, xo5, xo6, l0, l1, l2, dg, rd, xz, xy, xx;
-  };
-  auto load = [&](int a, Cell& c) {
-    const int i = i0 + a;
-    const size_t P = (size_t)i + rowP;
-    c.bb = bb[P];
-    c.u4 = c.u5 = c.u6 = c.xo4 = c.xo5 = c.xo6 = (T)0;
-    if (up) {
-      if (i < NX - 1) { c.u4 = (T)val[4 * n + P + 1]; c.xo4 = xo[P + 1]; }
-      if (j < NY - 1) { c.u5 = (T)val[5 * n + P + sy]; c.xo5 = xo[P + sy]; }
-      if (k < NZ - 1) { c.u6 = (T)val[6 * n + P + sz]; c.xo6 = xo[P + sz]; }
-    }
-    c.l0 = k > 0 ? (T)val[0 * n + P - sz] : (T)0;
-    c.l1 = j > 0 ? (T)val[1 * n + P - sy] : (T)0;
-    c.l2 = i > 0 ? (T)val[2 * n + P - 1] : (T)0;
-    c.dg = (T)val[3 * n + P];
-    c.rd = (T)val[7 * n + P];
-    // neighbours in the previous tiles (written by an earlier launch)
-    c.xz = (tc == 0 && k > 0) ? xn[P - sz] : (T)0;
-    c.xy = (tb == 0 && j > 0) ? xn[P - sy] : (T)0;
-    c.xx = (a == 0 && i > 0) ? xn[P - 1] : (T)0;
-  };
-
-  const int amax = min(GS_TX, NX - i0);  // cells of this line inside the box
-  Cell cur, nxt, nxt2;  // operands of cells a, a+1, a+2
-  if (line_ok && amax > 0) load(0, nxt);
-  if (line_ok && amax > 1) load(1, nxt2);
-  T last = (T)0;
-  const unsigned full = 0xffffffffu;
-  const int nlev_in = GS_TX + GS_TY + GS_TZ - 2;
-  for (int l = 0; l < nlev_in; ++l) {
-    const T from_y = __shfl_up_sync(full, last, 1);
-    const T from_z = __shfl_up_sync(full, last, GS_TY);
-    const int a = l - tb - tc;
-    if (line_ok && a >= 0 && a < amax) {
-      cur = nxt;
-      nxt = nxt2;
-      if (a + 2 < amax) load(a + 2, nxt2);
-      const int i = i0 + a;
-      T t = cur.bb;
-      if (up) {
-        if (i < NX - 1) t = t - cur.u4 * cur.xo4;
-        if (j < NY - 1) t = t - cur.u5 * cur.xo5;
-        if (k < NZ - 1) t = t - cur.u6 * cur.xo6;
+  T* xn = (last_parity ? buf_last : buf_other) + (size_t)g0 * n;        // x^s
+  const T* xo = (last_parity ? buf_other : buf_last) + (size_t)g0 * n;  // x^{s-1}
+  b += (size_t)g0 * n;
+  const int i0 = I * kGsTx, j0 = J * GS_TY, k0 = K * GS_TZ;
+  {
+    const int a = threadIdx.x % kGsTx, lb = threadIdx.x / kGsTx;
+    const int i = i0 + a, j = j0 + lb % GS_TY, k = k0 + lb / GS_TY;
+    const bool in = i < NX && j < NY && k < NZ;
+    const size_t P = (size_t)i + sy * (size_t)j + sz * (size_t)k;
+    const int e = lb * kGsPitch + a;
+    constexpr int kArr = kGsLines * kGsPitch;
+    if (in) {
+      // a missing neighbour: coefficient and value 0, t - 0 leaves every bit of t
+      coef[e] = k > 0 ? (T)val[0 * n + P - sz] : (T)0;
+      coef[e + kArr] = j > 0 ? (T)val[1 * n + P - sy] : (T)0;
+      coef[e + 2 * kArr] = i > 0 ? (T)val[2 * n + P - 1] : (T)0;
+      coef[e + 3 * kArr] = (T)val[3 * n + P];
+      coef[e + 4 * kArr] = reinterpret_cast<const T*>(val + (sizeof(TM) == 8 ? 8 : 7) * n)[P];
+      const bool u4 = s > 0 && i < NX - 1, u5 = s > 0 && j < NY - 1, u6 = s > 0 && k < NZ - 1;
+      const T c4 = u4 ? (T)val[4 * n + P + 1] : (T)0;
+      const T c5 = u5 ? (T)val[5 * n + P + sy] : (T)0;
+      const T c6 = u6 ? (T)val[6 * n + P + sz] : (T)0;
+      const int lz = lb / GS_TY, ly = lb % GS_TY;
+#pragma unroll 2
+      for (int ic = 0; ic < ncomp; ++ic) {
+        const size_t q = (size_t)ic * n + P;
+        T* cs = comp + (size_t)ic * kGsComp;
+        T t = b[q];
+        const T x4 = u4 ? xo[q + 1] : (T)0, x5 = u5 ? xo[q + sy] : (T)0, x6 = u6 ? xo[q + sz] : (T)0;
+        T* face = cs + kArr;  // faces: below [y][x], south [z][x], west [z][y]
+        if (lz == 0) face[ly * kGsTx + a] = k > 0 ? xn[q - sz] : (T)0;
+        if (ly == 0) face[4 * kGsTx + lz * kGsTx + a] = j > 0 ? xn[q - sy] : (T)0;
+        if (a == 0) face[8 * kGsTx + lb] = i > 0 ? xn[q - 1] : (T)0;
+        if (u4) t = t - gs_mul(c4, x4);
+        if (u5) t = t - gs_mul(c5, x5);
+        if (u6) t = t - gs_mul(c6, x6);
+        cs[e] = t;
       }
-      if (k > 0) t = t - cur.l0 * (tc > 0 ? from_z : cur.xz);
-      if (j > 0) t = t - cur.l1 * (tb > 0 ? from_y : cur.xy);
-      if (i > 0) t = t - cur.l2 * (a > 0 ? last : cur.xx);
-      t = div_rn(t, cur.dg, cur.rd);
-      xn[(size_t)i + rowP] = t;
-      last = t;
+    }
+  }
+  __syncthreads();
+  // whole warps (the shuffles); which of the block's warps walk changes from
+  // block to block, so that the blocks of an SM use all four sub-partitions
+  constexpr int kWarps = kGsBlock / 32;
+  const unsigned rot = ((blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) * 2654435761u) >> 29;
+  for (int c0 = 2 * ((threadIdx.x / 32 + rot) % kWarps); c0 < ncomp; c0 += 2 * kWarps) {
+    const int ic = c0 + (threadIdx.x / 16 & 1);
+    const int lb = threadIdx.x % 16, tb = lb % GS_TY, tc = lb / GS_TY;
+    const bool line_ok = ic < ncomp && j0 + tb < NY && k0 + tc < NZ;
+    T* cs = comp + (size_t)(ic < ncomp ? ic : 0) * kGsComp;
+    const T* face = cs + kGsLines * kGsPitch;
+    const T* zb = face + tb * kGsTx;
+    const T* yb = face + 4 * kGsTx + tc * kGsTx;
+    const int amax = min(kGsTx, NX - i0);
+    constexpr int kArr = kGsLines * kGsPitch;
+    T last = line_ok ? face[8 * kGsTx + lb] : (T)0;  // x^s west of the line, then of the previous cell
+    for (int l = 0; l < kGsTx + GS_TY + GS_TZ - 2; ++l) {
+      T from_y = __shfl_up_sync(0xffffffffu, last, 1);
+      T from_z = __shfl_up_sync(0xffffffffu, last, GS_TY);
+      const int a = l - tb - tc;
+      if (line_ok && a >= 0 && a < amax) {
+        const int e = lb * kGsPitch + a;
+        if (tc == 0) from_z = zb[a];
+        if (tb == 0) from_y = yb[a];
+        T t = cs[e];
+        const T mz = kIntL ? gs_mul(coef[e], from_z) : coef[e] * from_z;
+        const T my = kIntL ? gs_mul(coef[e + kArr], from_y) : coef[e + kArr] * from_y;
+        t = t - mz;
+        t = t - my;
+        t = t - coef[e + 2 * kArr] * last;
+        t = gs_quot(t, coef[e + 3 * kArr], coef[e + 4 * kArr]);
+        cs[e] = t;
+        last = t;
+      }
+    }
+  }
+  __syncthreads();
+  {
+    const int a = threadIdx.x % kGsTx, lb = threadIdx.x / kGsTx;
+    const int i = i0 + a, j = j0 + lb % GS_TY, k = k0 + lb / GS_TY;
+    if (i < NX && j < NY && k < NZ) {
+      const size_t P = (size_t)i + sy * (size_t)j + sz * (size_t)k;
+      for (int ic = 0; ic < ncomp; ++ic) xn[(size_t)ic * n + P] = comp[(size_t)ic * kGsComp + lb * kGsPitch + a];
     }
   }
 }

@@ -1,6 +1,8 @@
 // Definitions of the launch wrappers declared in launch.h for one scalar type.
 // Included once per precision translation unit after kernels.cuh.
 #pragma once
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace asam {
@@ -76,27 +78,42 @@ inline int gs_grid(const asam::Launch& L, size_t n) {
   }                                                                                                                \
   void launch_gs_sweeps(const Launch& L, const Dims& d, int ncomp, const TM* val, const T* b, T* out, T* work,     \
                         int nsweep, int group) {                                                                   \
-    const int ntx = (d.NX() + GS_TX - 1) / GS_TX;                                                                  \
+    const bool staged = sizeof(T) == sizeof(float);                                                                \
+    const int tx = staged ? GS_TX : kGsTx;                                                                         \
+    const int ntx = (d.NX() + tx - 1) / tx;                                                                        \
     const int nty = (d.NY() + GS_TY - 1) / GS_TY;                                                                  \
     const int ntz = (d.NZ() + GS_TZ - 1) / GS_TZ;                                                                  \
     const int nlev = ntx + nty + ntz - 2;                                                                          \
-    const bool staged = sizeof(T) == sizeof(float);                                                               \
-    /* whole warps (the sweep shuffles); the staged variant runs one component group per CTA */                 \
-    const int threads = (GS_TY * GS_TZ * (staged ? group : ncomp) + 31) / 32 * 32;                                \
-    const dim3 grid(ntx, ntz, nsweep * (staged ? gs_ngroups(ncomp, group) : 1));                                   \
-    const size_t smem = staged ? gs_smem_elems(group) * sizeof(T) : 0;                                             \
+    /* whole warps (the sweep shuffles); the FP32 variant runs one component group per CTA */                      \
+    const int threads = staged ? (GS_TY * GS_TZ * group + 31) / 32 * 32 : kGsBlock;                                \
+    /* FP64: all components in one CTA, unless a level has too few tiles for two CTAs on every SM: then groups     \
+       of an even number of components (a warp walks two), whose CTAs load the coefficients again */               \
+    if (!staged) {                                                                                                 \
+      const int tiles = std::max(1, ntx * nty * ntz / nlev * nsweep);                                              \
+      const int ng = std::min((ncomp + 1) / 2, std::max(1, 2 * L.sm_count / tiles));                               \
+      group = (ncomp + 2 * ng - 1) / (2 * ng) * 2;                                                                 \
+    }                                                                                                              \
+    const dim3 grid(ntx, ntz, nsweep * gs_ngroups(ncomp, group));                                                  \
+    const size_t smem = (staged ? gs_smem_elems(group) : gs_tile_elems(std::min(group, ncomp))) * sizeof(T);       \
     thread_local size_t smem_set = 0;                                                                              \
     if (staged && smem > smem_set) {                                                                               \
       cudaFuncSetAttribute(k_gs_pipe_smem<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
       smem_set = smem;                                                                                             \
     }                                                                                                              \
+    if (!staged) /* the same value whatever the call: threads with other component counts launch it too */         \
+      for (auto* f : {k_gs_tile<TM, T, false>, k_gs_tile<TM, T, true>})                                            \
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,                                       \
+                             (int)(gs_tile_elems(kMaxComp) * sizeof(T)));                                          \
+    /* the lower part's y and z products on the integer units once the block's walking warps outnumber the         \
+       sub-partitions (192x160x96, 10 components: 6.7 against 7.5 ms; 128x128x64, 3: 1.67 against 1.58) */         \
+    auto* gs_kernel = group > 8 ? k_gs_tile<TM, T, true> : k_gs_tile<TM, T, false>;                                \
     for (int tau = 0; tau < nlev + 2 * (nsweep - 1); ++tau) {                                                      \
       if (staged)                                                                                                  \
         k_gs_pipe_smem<TM, T><<<grid, threads, smem, L.stream>>>(d, ncomp, group, val, b, out, work, tau, nsweep,  \
                                                                  ntx, nty, ntz, nlev);                             \
       else                                                                                                         \
-        k_gs_pipe_reg<TM, T><<<grid, threads, 0, L.stream>>>(d, ncomp, val, b, out, work, tau, nsweep, ntx, nty,  \
-                                                             ntz, nlev);                                           \
+        gs_kernel<<<grid, threads, smem, L.stream>>>(d, ncomp, group, val, b, out, work, tau, nsweep, ntx, nty,    \
+                                                            ntz, nlev);                                            \
       count_launches(1);                                                                                           \
     }                                                                                                              \
   }                                                                                                                \

@@ -933,7 +933,7 @@ def transport_bench(a, torch, stream, hbm_peak, fp64_inst_peak):
                     f"{a.tol:g}",
         "value": ncell * a.steps / (r64["ms"] * 1e-3) / 1e6, "unit": METRIC, "ms_per_step": r64["ms"] / a.steps,
         "krylov_iterations": r64["iters"], "kernels_ms": r64["kernels"],
-        "roofline": {"kernel": "k_gs_pipe_reg (one PSolve: 1+IterG Gauss-Seidel sweeps)", "bound": "hbm",
+        "roofline": {"kernel": "k_gs_tile (one PSolve: 1+IterG Gauss-Seidel sweeps)", "bound": "hbm",
                      "achieved": gs_bytes / ps_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
                      "frac": gs_bytes / ps_s / 1e9 / hbm_peak, "traffic": None,
                      "algorithmic_bytes_per_call": gs_bytes,
