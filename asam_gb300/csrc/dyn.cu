@@ -21,7 +21,7 @@
 #include <vector>
 
 #include "context.h"
-#include "kernels.cuh"
+#include "launchers_impl.cuh"
 
 namespace asam {
 
@@ -288,15 +288,12 @@ void fcn_dyn_dev(asam_ctx* h, const double* c, const double* p, double* f) {
   launch_phi(L, d, h->cfg.ncomp, h->cfg.rho_pos, c, h->phi);
   launch_face_flux(L, d, h->geom(), h->cfg.ncomp, h->coef_x, h->coef_y, h->coef_z, h->mask_x, h->mask_y, h->mask_z,
                    h->phi, h->gx, h->gy, h->gz);
-  const int grid = grid_of(L, h->npad);
   const WallIn<double> wl{c, c + (size_t)h->cfg.rho_pos * h->npad};
   if (df)
-    k_flux_gather<double, true, true><<<grid, kB, 0, L.stream>>>(d, h->geom(), h->cfg.ncomp, h->gx, h->gy, h->gz,
-                                                                 h->rvol, f, ms, *df, wl);
+    run_flux_gather<double, true, true>(L, d, h->geom(), h->cfg.ncomp, h->gx, h->gy, h->gz, h->rvol, f, ms, *df, wl);
   else
-    k_flux_gather<double, true><<<grid, kB, 0, L.stream>>>(d, h->geom(), h->cfg.ncomp, h->gx, h->gy, h->gz, h->rvol,
-                                                             f, ms, DiffSrc<double>{}, wl);
-  count_launches(1);
+    run_flux_gather<double, true, false>(L, d, h->geom(), h->cfg.ncomp, h->gx, h->gy, h->gz, h->rvol, f, ms,
+                                         DiffSrc<double>{}, wl);
 }
 
 int need_dyn(asam_ctx* h) {

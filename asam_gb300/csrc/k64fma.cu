@@ -23,13 +23,11 @@ void launch_fcn(const Launch& L, const Dims& d, const GeomT<double>& g, int ncom
   k_face_flux<double, 2><<<gs_grid(L, d.n_wf()), kBlock, 0, L.stream>>>(d, g, ncomp, cz, mz, phi, gz);
   const asam::WallIn<double> wl{c, c + (size_t)rho_pos * d.npad()};
   if (df)
-    k_flux_gather<double, false, true><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol, f,
-                                                                                        MomSrc<double>{}, *df, wl);
+    run_flux_gather<double, false, true>(L, d, g, ncomp, gx, gy, gz, rvol, f, MomSrc<double>{}, *df, wl);
   else
-    k_flux_gather<double><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol, f,
-                                                                          MomSrc<double>{}, asam::DiffSrc<double>{},
-                                                                          wl);
-  count_launches(5);
+    run_flux_gather<double, false, false>(L, d, g, ncomp, gx, gy, gz, rvol, f, MomSrc<double>{},
+                                          asam::DiffSrc<double>{}, wl);
+  count_launches(4);
 }
 
 void launch_fcn_mom(const Launch& L, const Dims& d, const GeomT<double>& g, int ncomp, int rho_pos, const double* c,
@@ -43,12 +41,10 @@ void launch_fcn_mom(const Launch& L, const Dims& d, const GeomT<double>& g, int 
   k_face_flux<double, 2><<<gs_grid(L, d.n_wf()), kBlock, 0, L.stream>>>(d, g, ncomp, cz, mz, phi, gz);
   const asam::WallIn<double> wl{c, c + (size_t)rho_pos * d.npad()};
   if (df)
-    k_flux_gather<double, true, true><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol, f,
-                                                                                       ms, *df, wl);
+    run_flux_gather<double, true, true>(L, d, g, ncomp, gx, gy, gz, rvol, f, ms, *df, wl);
   else
-    k_flux_gather<double, true><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol, f, ms,
-                                                                                asam::DiffSrc<double>{}, wl);
-  count_launches(5);
+    run_flux_gather<double, true, false>(L, d, g, ncomp, gx, gy, gz, rvol, f, ms, asam::DiffSrc<double>{}, wl);
+  count_launches(4);
 }
 
 void launch_jac(const Launch& L, const Dims& d, const GeomT<double>& g, const double* rho, const double* rvol,

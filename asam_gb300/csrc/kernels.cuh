@@ -52,19 +52,55 @@ __device__ __forceinline__ T k2f(T hL, T hC, T hR) {
   const T e = eps_t<T>();
   return (hC / (hL + hC + e)) * (hR / (hL + hC + hR + e));
 }
+// a < b on the integer units (a comparison is an FP64 instruction of 64 cycles
+// as well): false for a quiet NaN a, as in 0/0 at a slope of -Eps; b a number
+__device__ __forceinline__ bool less(double a, double b) {
+  if (((unsigned)__double2hiint(a) & 0x7ff80000u) == 0x7ff80000u) return false;
+  long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  x ^= (long long)((unsigned long long)(x >> 63) >> 1);
+  y ^= (long long)((unsigned long long)(y >> 63) >> 1);
+  return x < y;
+}
+__device__ __forceinline__ bool less(float a, float b) { return a < b; }
+__device__ __forceinline__ bool positive(double a) { return __double_as_longlong(a) > 0; }
+__device__ __forceinline__ bool negative(double a) {
+  return (unsigned long long)__double_as_longlong(a) > 0x8000000000000000ull;
+}
+__device__ __forceinline__ bool positive(float a) { return a > 0.0f; }
+__device__ __forceinline__ bool negative(float a) { return a < 0.0f; }
+
 template <typename T>
 __device__ __forceinline__ T koren(T r, T k1, T k2) {
   T a = k1 * r + k2;
-  T m = a < (T)1 ? a : (T)1;
-  m = r < m ? r : m;
-  return (T)0 > m ? (T)0 : m;
+  T m = less(a, (T)1) ? a : (T)1;
+  m = less(r, m) ? r : m;
+  return negative(m) ? (T)0 : m;
 }
+
+// RN(x + Eps): from |x| = 2^-45 on Eps is less than half a unit in the last
+// place (of the next smaller number, too), so the sum is x
+__device__ __forceinline__ double add_eps(double x) {
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if (h >= (1023u - 45u) << 20) return x;
+  return (h | (unsigned)__double2loint(x)) == 0 ? asam::kEps : x + asam::kEps;
+}
+__device__ __forceinline__ float add_eps(float x) { return x + eps_t<float>(); }
+// products and quotients on the integer units (FP64; the same bits)
+__device__ __forceinline__ double mul_i(double a, double b) { return fpi::mul_rn(a, b); }
+__device__ __forceinline__ float mul_i(float a, float b) { return a * b; }
+__device__ __forceinline__ double div_i(double a, double b) { return fpi::div_rn(a, b); }
+__device__ __forceinline__ float div_i(float a, float b) { return a / b; }
+// a divisor with its reciprocal, for several quotients
+__device__ __forceinline__ unsigned long long recip_i(double d) { return fpi::recip(d); }
+__device__ __forceinline__ float recip_i(float d) { return 1.0f / d; }
+__device__ __forceinline__ double quot_i(double x, double d, unsigned long long R) { return fpi::quot_rn(x, d, R); }
+__device__ __forceinline__ float quot_i(float x, float d, float r) { return div_rn(x, d, r); }
 
 using asam::GeomT;
 
-// phi = c/(Rho+Eps) over the padded box, all components.  One IEEE
-// reciprocal of Rho+Eps per cell, then the correctly rounded quotient per
-// component (div_rn), identical to the reference's c/(Rho+Eps).
+// phi = c/(Rho+Eps) over the padded box, all components.  One reciprocal of
+// Rho+Eps per cell, then the correctly rounded quotient per component,
+// identical to the reference's c/(Rho+Eps); both on the integer units.
 template <typename T>
 __global__ void k_phi(Dims d, int ncomp, int rho_pos, const T* __restrict__ c, T* __restrict__ phi) {
   const size_t n = d.npad();
@@ -72,8 +108,9 @@ __global__ void k_phi(Dims d, int ncomp, int rho_pos, const T* __restrict__ c, T
   const T* rho = c + (size_t)rho_pos * n;
   for (size_t P = blockIdx.x * (size_t)blockDim.x + threadIdx.x; P < n; P += (size_t)gridDim.x * blockDim.x) {
     const T rp = rho[P] + e;
-    const T rr = (T)1 / rp;
-    for (int ic = 0; ic < ncomp; ++ic) phi[ic * n + P] = div_rn(c[ic * n + P], rp, rr);
+    const auto rr = recip_i(rp);
+#pragma unroll 2
+    for (int ic = 0; ic < ncomp; ++ic) phi[ic * n + P] = quot_i(c[ic * n + P], rp, rr);
   }
 }
 
@@ -163,6 +200,11 @@ __global__ void k_face_coef(Dims d, GeomT<T> g, T* __restrict__ coef, unsigned c
 // flux the reference's loop computes for the upwind interior cell of the face
 // (zero when the upwind cell is a halo cell or the velocity is zero):
 //   Half*(ABS(u)+-u)*F*(cC + Fo/(Fo+Eps)*PhiLim(r,k1,k2,...))   (:875-894)
+// Bound by the FP64 unit (64 cycles of a sub-partition per warp instruction):
+// the slope quotient, the comparisons and two of the products run on the
+// integer units, an Eps that cannot change its sum is not added, and a ratio
+// of 1 is not multiplied, which leaves 5 to 8 FP64 instructions a face and
+// component of about 25.
 template <typename T, int AXIS>
 __global__ void k_face_flux(Dims d, GeomT<T> g, int ncomp, const T* __restrict__ coef,
                             const unsigned char* __restrict__ mask, const T* __restrict__ phi,
@@ -173,21 +215,28 @@ __global__ void k_face_flux(Dims d, GeomT<T> g, int ncomp, const T* __restrict__
   const int ez = AXIS == 2 ? nz + 1 : nz;
   const size_t nface = (size_t)ex * ey * ez;
   const size_t n = d.npad();
-  const T e = eps_t<T>();
   for (size_t f = blockIdx.x * (size_t)blockDim.x + threadIdx.x; f < nface; f += (size_t)gridDim.x * blockDim.x) {
     const T pref_s = coef[f];
     if (pref_s == (T)0) {
       for (int ic = 0; ic < ncomp; ++ic) gout[ic * nface + f] = (T)0;
       continue;
     }
-    const bool right = pref_s > (T)0;
+    const bool right = positive(pref_s);
     const T pref = right ? pref_s : -pref_s;
     const T ratio = coef[nface + f], k1 = coef[2 * nface + f], k2 = coef[3 * nface + f];
+    const bool unit = ratio == (T)1;
     const unsigned char m = mask[f];
-    const int a = (int)(f % ex);
-    const size_t rest = f / ex;
-    const int b = (int)(rest % ey);
-    const int cc = (int)(rest / ey);
+    int a, b, cc;
+    if (nface < (size_t)0xffffffffu) {
+      const unsigned fu = (unsigned)f, rest = fu / (unsigned)ex;
+      a = (int)(fu - rest * (unsigned)ex);
+      cc = (int)(rest / (unsigned)ey);
+      b = (int)(rest - (unsigned)cc * (unsigned)ey);
+    } else {
+      a = (int)(f % ex);
+      b = (int)((f / ex) % ey);
+      cc = (int)((f / ex) / ey);
+    }
     int ci, cj, ck;
     if (AXIS == 0) {
       ci = a + !right; cj = b + 1; ck = cc + 1;
@@ -224,15 +273,12 @@ __global__ void k_face_flux(Dims d, GeomT<T> g, int ncomp, const T* __restrict__
         if (m & 4) cL = ((FR - FL) * cC + FL * cL) / FR;
         if (m & 8) cR = ((FL - FR) * cC + FR * cR) / FL;
       }
-      T flux;
-      if (right) {
-        const T r = (cR - cC + e) / ((cC - cL) + e);
-        flux = pref * (cC + ratio * (koren(r, k1, k2) * (cC - cL)));
-      } else {
-        const T r = (cC - cL + e) / ((cR - cC) + e);
-        flux = pref * (cC + ratio * (koren(r, k1, k2) * (cC - cR)));
-      }
-      gout[ic * nface + f] = flux;
+      // r = (cR-cC+Eps)/((cC-cL)+Eps), slope cC-cL; from the right mirrored
+      const T dR = cR - cC, dL = cC - cL;
+      const T eR = add_eps(dR), eL = add_eps(dL);
+      const T r = div_i(right ? eR : eL, right ? eL : eR);
+      const T slope = mul_i(koren(r, k1, k2), right ? dL : -dR);
+      gout[ic * nface + f] = mul_i(pref, unit ? cC + slope : cC + ratio * slope);
     }
   }
 }
@@ -241,25 +287,26 @@ __global__ void k_face_flux(Dims d, GeomT<T> g, int ncomp, const T* __restrict__
 // interior face between padded cells (i,j,k) and their +1 neighbour along
 // axis, with DUU = F/(F+Eps) of IniJacAccGrav (MULTI/JacAccGrav_Mod.f90:297):
 //   DUU*F/(F+Eps)*(p(+1)-p)/(Metr*(d(+1)+d+Eps)), evaluated left to right.
+// An area from 2^-45 on is unchanged by Eps, both ratios are 1 and the products
+// with them exact.
+template <typename T>
+__device__ __forceinline__ T pgrad_ratio(T F, T dp, T den) {
+  const T Fe = add_eps(F);
+  if (Fe == F && F > (T)0) return div_i(dp, den);
+  const T du = div_i(F, Fe);
+  return div_i(div_i(du * F, Fe) * dp, den);
+}
 template <typename T>
 __device__ __forceinline__ T pgrad_face(const Dims& d, const GeomT<T>& g, const MomSrc<T>& ms, int axis, int i, int j,
                                         int k) {
   const T e = eps_t<T>();
-  if (axis == 0) {
-    const T F = g.fu[d.FU(i, j, k)];
-    const T du = F / (F + e);
-    return du * F / (F + e) * (ms.p[d.P(i + 1, j, k)] - ms.p[d.P(i, j, k)]) /
-           (ms.mxy[j - 1] * (ms.dx[i] + ms.dx[i - 1] + e));
-  }
-  if (axis == 1) {
-    const T F = g.fv[d.FV(i, j, k)];
-    const T du = F / (F + e);
-    return du * F / (F + e) * (ms.p[d.P(i, j + 1, k)] - ms.p[d.P(i, j, k)]) /
-           (ms.myx[i - 1] * (ms.dy[j] + ms.dy[j - 1] + e));
-  }
-  const T F = g.fw[d.FW(i, j, k)];
-  const T du = F / (F + e);
-  return du * F / (F + e) * (ms.p[d.P(i, j, k + 1)] - ms.p[d.P(i, j, k)]) / (ms.dz[k] + ms.dz[k - 1] + e);
+  if (axis == 0)
+    return pgrad_ratio(g.fu[d.FU(i, j, k)], ms.p[d.P(i + 1, j, k)] - ms.p[d.P(i, j, k)],
+                       ms.mxy[j - 1] * (ms.dx[i] + ms.dx[i - 1] + e));
+  if (axis == 1)
+    return pgrad_ratio(g.fv[d.FV(i, j, k)], ms.p[d.P(i, j + 1, k)] - ms.p[d.P(i, j, k)],
+                       ms.myx[i - 1] * (ms.dy[j] + ms.dy[j - 1] + e));
+  return pgrad_ratio(g.fw[d.FW(i, j, k)], ms.p[d.P(i, j, k + 1)] - ms.p[d.P(i, j, k)], ms.dz[k] + ms.dz[k - 1] + e);
 }
 
 // Grad of PGradComputeCFull's neighbour loop on a periodic side ('iw', 'ie',
@@ -297,8 +344,9 @@ __device__ __forceinline__ T buoy_rho_face(const Dims& d, const GeomT<T>& g, con
                                            int k) {
   const T e = eps_t<T>();
   const T F = g.fw[d.FW(i, j, k)];
-  return F / (F + e) * (ms.dz[k - 1] * ms.rho[d.P(i, j, k)] + ms.dz[k] * ms.rho[d.P(i, j, k + 1)]) /
-         (ms.dz[k - 1] + ms.dz[k] + e);
+  const T s = ms.dz[k - 1] * ms.rho[d.P(i, j, k)] + ms.dz[k] * ms.rho[d.P(i, j, k + 1)];
+  const T Fe = add_eps(F), den = ms.dz[k - 1] + ms.dz[k] + e;
+  return Fe == F && F > (T)0 ? div_i(s, den) : div_i(div_i(F, Fe) * s, den);
 }
 
 // Gather of the face fluxes into the cell right-hand side in the exact order
@@ -310,6 +358,41 @@ __device__ __forceinline__ T buoy_rho_face(const Dims& d, const GeomT<T>& g, con
 // kMom adds the momentum sources of ms (closed or periodic x/y sides); kDiff the diffusion
 // fluxes of df with DiffusionCompute's second zero-volume mask (the halo
 // cells of a periodic side included, before ExchangeFlux reads them).
+// The cells one in from every side of the block have none of the side terms:
+// k_flux_plain takes them (half of the registers), and this kernel, whose
+// 170 registers leave an SM eight warps, the halo cells and the outermost
+// interior ones, enumerated without gaps.
+//
+// Halo and outermost interior cells of a block with at least two cells along
+// every axis: the planes k = 0, 1, nz, nz+1, then of the other planes the rows
+// j = 0, 1, ny, ny+1, then of the other rows the cells i = 0, 1, nx, nx+1; a
+// thinner block has no other cells.
+__host__ __device__ inline bool flux_all_edges(const Dims& d) { return d.nx < 2 || d.ny < 2 || d.nz < 2; }
+__host__ __device__ inline size_t flux_edges(const Dims& d) {
+  if (flux_all_edges(d)) return d.npad();
+  return 4 * ((size_t)d.NX() * d.NY() + (size_t)d.NX() * (d.nz - 2) + (size_t)(d.ny - 2) * (d.nz - 2));
+}
+__device__ __forceinline__ void flux_edge_cell(const Dims& d, size_t q, int& i, int& j, int& k) {
+  auto side = [](int s, int m) { return s < 2 ? s : m - 2 + s; };  // 0, 1, m, m+1
+  const size_t nk = 4 * (size_t)d.NX() * d.NY(), nj = 4 * (size_t)d.NX() * (d.nz - 2);
+  if (q < nk) {
+    const unsigned p = (unsigned)q, r = p / (unsigned)d.NX();
+    i = (int)(p - r * d.NX());
+    j = (int)(r % (unsigned)d.NY());
+    k = side((int)(r / (unsigned)d.NY()), d.nz);
+  } else if (q < nk + nj) {
+    const unsigned p = (unsigned)(q - nk), r = p / (unsigned)d.NX();
+    i = (int)(p - r * d.NX());
+    j = side((int)(r & 3u), d.ny);
+    k = 2 + (int)(r >> 2);
+  } else {
+    const unsigned p = (unsigned)(q - nk - nj), r = p >> 2;
+    i = side((int)(p & 3u), d.nx);
+    j = 2 + (int)(r % (unsigned)(d.ny - 2));
+    k = 2 + (int)(r / (unsigned)(d.ny - 2));
+  }
+}
+
 template <typename T, bool kMom = false, bool kDiff = false>
 __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict__ gx, const T* __restrict__ gy,
                               const T* __restrict__ gz, const T* __restrict__ rvol, T* __restrict__ f,
@@ -319,12 +402,18 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
   const size_t n = d.npad();
   const size_t nfx = (size_t)(nx + 1) * ny * nz, nfy = (size_t)nx * (ny + 1) * nz, nfz = (size_t)nx * ny * (nz + 1);
   const T e = eps_t<T>();
-  for (size_t P = blockIdx.x * (size_t)blockDim.x + threadIdx.x; P < n; P += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(P % NX);
-    const int j = (int)((P / NX) % NY);
-    const int k = (int)(P / ((size_t)NX * NY));
+  const bool all = flux_all_edges(d);
+  const size_t nedge = flux_edges(d);
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nedge; q += (size_t)gridDim.x * blockDim.x) {
+    int i, j, k;
+    if (all)
+      d.ijk(q, i, j, k);
+    else
+      flux_edge_cell(d, q, i, j, k);
+    const size_t P = d.P(i, j, k);
     const T V = g.volc[P];
     const T Ve = V + e, rV = rvol[P];
+    const auto RV = recip_i(Ve);
     const bool ii = i >= 1 && i <= nx, jj = j >= 1 && j <= ny, kk = k >= 1 && k <= nz;
     if (ii && jj && kk) {
       const size_t fxL = d.UF(i - 1, j, k), fxR = d.UF(i, j, k);
@@ -337,23 +426,27 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
       const bool exW = d.per_x && i == 1, exE = d.per_x && i == nx;
       const bool exS = d.per_y && j == 1, exN = d.per_y && j == ny;
       const bool exB = d.per_z && k == 1, exT = d.per_z && k == nz;
+      // directions of the six faces' flow, tested once for all components
+      const bool puL = positive(uL), nuL = negative(uL), puR = positive(uR), nuR = negative(uR);
+      const bool pvL = positive(vL), nvL = negative(vL), pvR = positive(vR), nvR = negative(vR);
+      const bool pwL = positive(wL), nwL = negative(wL), pwR = positive(wR), nwR = negative(wR);
       for (int ic = 0; ic < ncomp; ++ic) {
         const T* GX = gx + ic * nfx;
         const T* GY = gy + ic * nfy;
         const T* GZ = gz + ic * nfz;
         T a = (T)0;
-        if (wL > (T)0) a = a + GZ[fzL];  // FluxZR of the cell below
-        if (vL > (T)0) a = a + GY[fyL];  // FluxYR of the cell south
-        if (uL > (T)0) a = a + GX[fxL];  // FluxXR of the cell west
-        if (uL < (T)0) a = a - GX[fxL];  // own x-left
-        if (uR > (T)0) a = a - GX[fxR];  // own x-right
-        if (vL < (T)0) a = a - GY[fyL];
-        if (vR > (T)0) a = a - GY[fyR];
-        if (wL < (T)0) a = a - GZ[fzL];
-        if (wR > (T)0) a = a - GZ[fzR];
-        if (uR < (T)0) a = a + GX[fxR];  // FluxXL of the cell east
-        if (vR < (T)0) a = a + GY[fyR];
-        if (wR < (T)0) a = a + GZ[fzR];
+        if (pwL) a = a + GZ[fzL];  // FluxZR of the cell below
+        if (pvL) a = a + GY[fyL];  // FluxYR of the cell south
+        if (puL) a = a + GX[fxL];  // FluxXR of the cell west
+        if (nuL) a = a - GX[fxL];  // own x-left
+        if (puR) a = a - GX[fxR];  // own x-right
+        if (nvL) a = a - GY[fyL];
+        if (pvR) a = a - GY[fyR];
+        if (nwL) a = a - GZ[fzL];
+        if (pwR) a = a - GZ[fzR];
+        if (nuR) a = a + GX[fxR];  // FluxXL of the cell east
+        if (nvR) a = a + GY[fyR];
+        if (nwR) a = a + GZ[fzR];
         if (wl.c) {  // inflow through the outer walls' faces, W, E, S, N, B, T (:975-1044)
           const T* cc = wl.c + ic * n;
           const T half = (T)0.5;
@@ -382,7 +475,7 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
             a = a + half * (fabs(wR) - wR) * cc[H] / (wl.rho[H] + e) * g.fw[d.FW(i, j, nz)];
           }
         }
-        a = div_rn(a * V, Ve, rV);
+        a = quot_i(a * V, Ve, RV);
         if (kDiff) {  // f(R) - Flux, f(L) + Flux per face, x then y then z; then the mask
           const T* ph = df.phi + ic * n;
           const T pc = ph[P];
@@ -492,7 +585,7 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
           }
           a = a + hv;
         }
-        T fv = div_rn(a, Ve, rV);
+        T fv = quot_i(a, Ve, RV);
         if (kMom && ms.buoy) {  // fL(iz+1) - RhoLoc*Grav, fR(iz) - RhoLoc*Grav
           if (ic == ms.pos[4] && k >= 2) fv = fv - buoy_rho_face(d, g, ms, i, j, k - 1) * ms.grav;
           else if (ic == ms.pos[5] && k <= nz - 1) fv = fv - buoy_rho_face(d, g, ms, i, j, k) * ms.grav;
@@ -548,6 +641,99 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
         }
         f[ic * n + P] = div_rn(a, Ve, rV);
       }
+    }
+  }
+}
+
+// k_flux_gather's operations for the cells with 2 <= i <= nx-1 (j, k alike).
+// Bound by the FP64 unit and by the latency of its serial sum: the directions
+// of the six faces are tested once per cell, the two quotients by the volume
+// run on the integer units, and the faces of a pressure gradient whose area is
+// not tiny skip the ratios F/(F+Eps) = 1 (pgrad_face).
+template <typename T, bool kMom, bool kDiff>
+__global__ void __launch_bounds__(256, kMom || kDiff ? 2 : 3) k_flux_plain(Dims d, GeomT<T> g, int ncomp, const T* __restrict__ gx,
+                                                    const T* __restrict__ gy, const T* __restrict__ gz,
+                                                    T* __restrict__ f, MomSrc<T> ms, DiffSrc<T> df) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int NX = d.NX(), NY = d.NY();
+  const unsigned px = nx - 2, py = ny - 2;
+  const size_t n = d.npad(), np = (size_t)px * py * (nz - 2);
+  const size_t nfx = (size_t)(nx + 1) * ny * nz, nfy = (size_t)nx * (ny + 1) * nz, nfz = (size_t)nx * ny * (nz + 1);
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < np; q += (size_t)gridDim.x * blockDim.x) {
+    int i, j, k;
+    if (np < (size_t)0xffffffffu) {
+      const unsigned p = (unsigned)q, r = p / px;
+      i = (int)(p - r * px) + 2;
+      k = (int)(r / py) + 2;
+      j = (int)(r - (unsigned)(k - 2) * py) + 2;
+    } else {
+      const size_t r = q / px;
+      i = (int)(q - r * px) + 2;
+      k = (int)(r / py) + 2;
+      j = (int)(r - (size_t)(k - 2) * py) + 2;
+    }
+    const size_t P = d.P(i, j, k);
+    const T V = g.volc[P], Ve = V + eps_t<T>();
+    const auto RV = recip_i(Ve);
+    const size_t fx = d.UF(i - 1, j, k), fy = d.VF(i, j - 1, k), fz = d.WF(i, j, k - 1);
+    const size_t dz = (size_t)nx * ny;
+    const T uL = g.uf[fx], uR = g.uf[fx + 1], vL = g.vf[fy], vR = g.vf[fy + nx], wL = g.wf[fz], wR = g.wf[fz + dz];
+    // directions of the six faces' flow, tested once for all components
+    const unsigned m = (unsigned)positive(uL) | (unsigned)negative(uL) << 1 | (unsigned)positive(uR) << 2 |
+                       (unsigned)negative(uR) << 3 | (unsigned)positive(vL) << 4 | (unsigned)negative(vL) << 5 |
+                       (unsigned)positive(vR) << 6 | (unsigned)negative(vR) << 7 | (unsigned)positive(wL) << 8 |
+                       (unsigned)negative(wL) << 9 | (unsigned)positive(wR) << 10 | (unsigned)negative(wR) << 11;
+#pragma unroll 2
+    for (int ic = 0; ic < ncomp; ++ic) {
+      const T* GX = gx + ic * nfx + fx;
+      const T* GY = gy + ic * nfy + fy;
+      const T* GZ = gz + ic * nfz + fz;
+      const T xl = GX[0], xr = GX[1], yl = GY[0], yr = GY[nx], zl = GZ[0], zr = GZ[dz];
+      T a = (T)0;
+      if (m & 256) a = a + zl;  // FluxZR of the cell below
+      if (m & 16) a = a + yl;   // FluxYR of the cell south
+      if (m & 1) a = a + xl;    // FluxXR of the cell west
+      if (m & 2) a = a - xl;    // own x-left
+      if (m & 4) a = a - xr;    // own x-right
+      if (m & 32) a = a - yl;
+      if (m & 64) a = a - yr;
+      if (m & 512) a = a - zl;
+      if (m & 1024) a = a - zr;
+      if (m & 8) a = a + xr;    // FluxXL of the cell east
+      if (m & 128) a = a + yr;
+      if (m & 2048) a = a + zr;
+      a = quot_i(a * V, Ve, RV);
+      if (kDiff) {  // f(R) - Flux, f(L) + Flux per face, x then y then z; then the mask
+        const T* ph = df.phi + ic * n;
+        const T pc = ph[P];
+        a = a - (T)2 * df.kx[fx] * (pc - ph[P - 1]);
+        a = a + (T)2 * df.kx[fx + 1] * (ph[P + 1] - pc);
+        a = a - (T)2 * df.ky[fy] * (pc - ph[P - (size_t)NX]);
+        a = a + (T)2 * df.ky[fy + nx] * (ph[P + (size_t)NX] - pc);
+        a = a - (T)2 * df.kz[fz] * (pc - ph[P - (size_t)NX * NY]);
+        a = a + (T)2 * df.kz[fz + dz] * (ph[P + (size_t)NX * NY] - pc);
+        a = quot_i(a * V, Ve, RV);
+      }
+      if (kMom && ms.pgrad) {  // uRhsL(ix+1) - Two*VolC(ix+1)*Grad, uRhsR(ix) - Two*VolC(ix)*Grad
+        int axis = -1, lo = 0;
+        if (ic == ms.pos[0]) axis = 0, lo = 1;
+        else if (ic == ms.pos[1]) axis = 0;
+        else if (ic == ms.pos[2]) axis = 1, lo = 1;
+        else if (ic == ms.pos[3]) axis = 1;
+        else if (ic == ms.pos[4]) axis = 2, lo = 1;
+        else if (ic == ms.pos[5]) axis = 2;
+        if (axis >= 0) {
+          const T gr = pgrad_face(d, g, ms, axis, i - (axis == 0 ? lo : 0), j - (axis == 1 ? lo : 0),
+                                  k - (axis == 2 ? lo : 0));
+          a = a - (T)2 * V * gr;
+        }
+      }
+      T fv = quot_i(a, Ve, RV);
+      if (kMom && ms.buoy) {  // fL(iz+1) - RhoLoc*Grav, fR(iz) - RhoLoc*Grav
+        if (ic == ms.pos[4]) fv = fv - buoy_rho_face(d, g, ms, i, j, k - 1) * ms.grav;
+        else if (ic == ms.pos[5]) fv = fv - buoy_rho_face(d, g, ms, i, j, k) * ms.grav;
+      }
+      f[ic * n + P] = fv;
     }
   }
 }

@@ -23,6 +23,20 @@ inline int gs_grid(const asam::Launch& L, size_t n) {
   if (g < 1) g = 1;
   return (int)g;
 }
+// the gather of the face fluxes: the cells off the sides, then the others
+template <typename T, bool kMom, bool kDiff>
+void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::GeomT<T>& g, int ncomp, const T* gx,
+                     const T* gy, const T* gz, const T* rvol, T* f, const asam::MomSrc<T>& ms,
+                     const asam::DiffSrc<T>& df, const asam::WallIn<T>& wl) {
+  if (d.nx > 2 && d.ny > 2 && d.nz > 2) {
+    k_flux_plain<T, kMom, kDiff><<<gs_grid(L, (size_t)(d.nx - 2) * (d.ny - 2) * (d.nz - 2)), kBlock, 0, L.stream>>>(
+        d, g, ncomp, gx, gy, gz, f, ms, df);
+    asam::count_launches(1);
+  }
+  k_flux_gather<T, kMom, kDiff><<<gs_grid(L, flux_edges(d)), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol, f, ms, df,
+                                                                                wl);
+  asam::count_launches(1);
+}
 }  // namespace
 
 #define ASAM_DEFINE_LAUNCHERS(T, TM)                                                                               \
@@ -48,12 +62,9 @@ inline int gs_grid(const asam::Launch& L, size_t n) {
   void launch_flux_gather(const Launch& L, const Dims& d, const GeomT<T>& g, int ncomp, const T* gx, const T* gy,  \
                           const T* gz, const T* rvol, T* f, const DiffSrc<T>* df, const WallIn<T>& wl) {           \
     if (df)                                                                                                        \
-      k_flux_gather<T, false, true><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol,  \
-                                                                                   f, MomSrc<T>{}, *df, wl);       \
+      run_flux_gather<T, false, true>(L, d, g, ncomp, gx, gy, gz, rvol, f, MomSrc<T>{}, *df, wl);                  \
     else                                                                                                           \
-      k_flux_gather<T><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, g, ncomp, gx, gy, gz, rvol, f,            \
-                                                                      MomSrc<T>{}, DiffSrc<T>{}, wl);              \
-    count_launches(1);                                                                                             \
+      run_flux_gather<T, false, false>(L, d, g, ncomp, gx, gy, gz, rvol, f, MomSrc<T>{}, DiffSrc<T>{}, wl);        \
   }                                                                                                                \
   void launch_diff_coef(const Launch& L, const Dims& d, const GeomT<T>& g, const T* dh, const T* dv, T* kx, T* ky,  \
                         T* kz) {                                                                                   \
