@@ -540,27 +540,6 @@ __device__ inline T matvec2_at(const Lev2T<T>& P, size_t mo, const T* __restrict
   return y;
 }
 
-// One zebra half-sweep over the x-lines of parity c of one plane: the line
-// right-hand side in the forward or backward operation order of
-// GaussSeidel_2D, then Solve_1D with the precomputed factors.  The forward
-// elimination streams the eight inputs of each row (b, the two neighbour
-// lines, their couplings, the sub-diagonal of the previous row, the pivot
-// and its reciprocal) through a per-thread ring of kRing rows in shared
-// memory with cp.async, kAhead rows ahead of the recurrence; the copies read
-// only the other parity's lines and the matrix, never this thread's column.
-// The back substitution loads x and w four rows ahead in two register sets.
-// Ring depth by value type: the same 64 KB per CTA hold 4 FP64 rows or 8 FP32
-// rows, so the FP32 copy keeps twice as many rows in flight.
-template <typename T>
-struct RingCfg {
-  static constexpr int ring = 4, ahead = 3;
-};
-template <>
-struct RingCfg<float> {
-  static constexpr int ring = 8, ahead = 7;
-};
-constexpr int kFields = 8;
-
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -657,52 +636,69 @@ __device__ void line_half_lanes(const Lev2T<T>& P, size_t mo, const T* __restric
   }
 }
 
-// FP64: the line right-hand sides of one half-sweep formed by the whole block
-// and left in x of the lines to be solved, before their recurrences.  A GB300
-// sub-partition takes 64 cycles per FP64 warp instruction, dependent or not, so
-// a warp that forms its own right-hand sides (four operations a row) and then
-// runs the recurrence (seven) pays all eleven one after the other while the
-// block's other warps wait: 704 cycles a row against 448.  With more lines
-// than four warps the solving warps fill all four sub-partitions by
-// themselves and the split would only move the same work (kSplitLines).
-constexpr int kSplitLines = 128;
-template <typename T>
-__device__ __forceinline__ bool split_rhs(int nl) {
-  return sizeof(T) == 8 && nl <= kSplitLines;
-}
-template <typename T, bool kWrap>
-__device__ __forceinline__ void rhs_half(const Lev2T<T>& P, size_t mo, const T* __restrict__ b, T* x, int c, int fwd) {
+// The line right-hand sides of one half-sweep, b minus the two neighbour lines
+// in the forward or backward operation order of GaussSeidel_2D, formed by the
+// whole block and left in x of the lines to be solved, before their
+// recurrences.  A GB300 sub-partition takes 64 cycles per FP64 warp
+// instruction, dependent or not, so a warp that forms its own right-hand sides
+// (four operations a row) and then runs the recurrence (seven) pays all eleven
+// one after the other while the block's other warps wait.
+// kU entries a thread at a time: 4 where the operands come from L2, 1 for FP64
+// in shared memory (the FP64 unit is the limit there).
+template <typename T, bool kWrap, int kU>
+__device__ __forceinline__ void rhs_half(const Lev2T<T>& P, size_t mo, const T* b, T* x, int c, int fwd) {
   const int c1 = P.c1, c2 = P.c2, h = P.h, w = P.w;
   const T* lx = P.lx + mo;
   const T* ux = P.ux + mo;
-  const int nl = (c2 - c + 1) / 2;
+  const int nl = (c2 - c + 1) / 2, tot = nl * c1, bd = blockDim.x;
   const bool wrap = kWrap && P.wxl && c2 >= 2 && ((c2 - 1) & 1);
   const size_t wk = kWrap ? (mo / P.ps) * (size_t)c1 : 0;
-  for_plane(nl, (size_t)nl * c1, [&](size_t, int i, int q) {
-    const int j = 2 * q + c;
-    const int o = i * w, oth = o + (1 - c) * h;
-    const int e = o + c * h + q;
-    const T bv = b[e];
-    T ml = (T)0, mr = (T)0;  // a missing neighbour: t - 0 leaves every bit of t
-    if (j > 0) {
-      const int a = oth + ((j - 1) >> 1);
-      ml = lx[a] * x[a];
-    } else if (wrap) {
-      ml = P.wxl[wk + i] * x[o + slot(0, h, 0, c2 - 1)];
+  const int wlast = (int)slot(0, h, 0, c2 - 1);
+  int i = (int)threadIdx.x / nl, q = (int)threadIdx.x - i * nl;
+  const int di = bd / nl, dq = bd - di * nl;
+  for (int e = threadIdx.x; e < tot; e += kU * bd) {
+    T bv[kU], cl[kU], xl[kU], cr[kU], xr[kU];
+    int pos[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      pos[u] = -1;
+      // a missing neighbour: 0*0, and t - 0 leaves every bit of t
+      bv[u] = cl[u] = xl[u] = cr[u] = xr[u] = (T)0;
+      if (e + u * bd < tot) {
+        const int j = 2 * q + c, o = i * w, oth = o + (1 - c) * h;
+        pos[u] = o + c * h + q;
+        bv[u] = b[pos[u]];
+        const bool wl = wrap && j == 0, wr = wrap && j == c2 - 1;
+        if (j > 0) cl[u] = lx[oth + ((j - 1) >> 1)], xl[u] = x[oth + ((j - 1) >> 1)];
+        if (wl) cl[u] = P.wxl[wk + i], xl[u] = x[o + wlast];
+        if (j < c2 - 1) cr[u] = ux[pos[u]], xr[u] = x[oth + ((j + 1) >> 1)];
+        if (wr) cr[u] = P.wxh[wk + i], xr[u] = x[o];
+      }
+      i += di;
+      q += dq;
+      if (q >= nl) {
+        q -= nl;
+        ++i;
+      }
     }
-    if (j < c2 - 1) {
-      mr = ux[e] * x[oth + ((j + 1) >> 1)];
-    } else if (wrap) {
-      mr = P.wxh[wk + i] * x[o];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const T ml = cl[u] * xl[u], mr = cr[u] * xr[u];
+      if (pos[u] >= 0) x[pos[u]] = fwd ? (bv[u] - ml) - mr : (bv[u] - mr) - ml;
     }
-    x[e] = fwd ? (bv - ml) - mr : (bv - mr) - ml;
-  });
+  }
   __syncthreads();
 }
 
+// One zebra half-sweep over the x-lines of parity c of one plane whose level
+// streams from global memory: the right-hand sides, then Solve_1D with the
+// precomputed factors, a thread per line.  A thread loads the operands of a
+// batch of rows into registers while it solves the batch before: with one
+// warp per sub-partition nothing else covers the L2 latency, and the row ring in
+// shared memory that fed it before (eight cp.async a row) cost more
+// instructions than the row itself.
 template <typename T, bool kWrap = false>
-__device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __restrict__ b, T* __restrict__ x, int c,
-                                       int fwd, T* __restrict__ ring, int rs) {
+__device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* b, T* x, int c, int fwd) {
   if constexpr (sizeof(T) == 4) {  // few lines: K lanes per line (the whole block takes part in the shuffles)
     const int nl = (P.c2 - c + 1) / 2;
     int K = 1;
@@ -712,106 +708,76 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __
       return;
     }
   }
-  const bool split = split_rhs<T>((P.c2 - c + 1) / 2);
-  if (split) rhs_half<T, kWrap>(P, mo, b, x, c, fwd);
-  const int c1 = P.c1, c2 = P.c2, h = P.h, w = P.w;
-  const T* __restrict__ lx = P.lx + mo;
-  const T* __restrict__ ux = P.ux + mo;
-  const T* __restrict__ lz = P.lz + mo;
-  const T* __restrict__ ft = P.ft + mo;
-  const T* __restrict__ frt = P.frt + mo;
-  const T* __restrict__ fw = P.fw + mo;
-  constexpr int kRing = RingCfg<T>::ring, kAhead = RingCfg<T>::ahead;
-  const int nl = (c2 - c + 1) / 2;
-  // slots of the ring: rs threads take part (rs = min(block, the lines of one
-  // parity rounded up to a warp)), so a narrow plane leaves the shared memory
-  // to its resident levels
-  const int bd = rs, tid = threadIdx.x;
-  if (tid >= rs) return;
-  for (int q = tid; q < nl; q += bd) {
-    const int j = 2 * q + c;
-    const size_t col = (size_t)c * h + q;
-    const bool hasL = j > 0, hasR = j < c2 - 1;
-    const size_t colL = hasL ? (size_t)(1 - c) * h + ((j - 1) >> 1) : col;
-    const size_t colR = hasR ? (size_t)(1 - c) * h + ((j + 1) >> 1) : col;
-    // periodic-Laplacian hierarchy: line 0's left neighbour is line c2-1 and
-    // line c2-1's right neighbour is line 0, across the periodic side; used
-    // only when the two have different parities (no line reads a line of its
-    // own half-sweep).  The wrap neighbour and its coupling take the ring
-    // slots of the missing neighbour, so they stream ahead like the others.
-    const bool wrap = kWrap && P.wxl && c2 >= 2 && ((c2 - 1) & 1);
-    const bool wL = wrap && j == 0, wR = wrap && j == c2 - 1;
-    const bool useL = !split && (hasL || wL), useR = !split && (hasR || wR);
-    const size_t wk = (mo / P.ps) * (size_t)c1;
-    const size_t xL0 = wL ? slot(0, h, 0, c2 - 1) : colL, xR0 = wR ? slot(0, h, 0, 0) : colR;
-    const T* rb = split ? x : b;
-    auto issue = [&](int i) {
-      T* sl = ring + (size_t)(i % kRing) * kFields * bd + tid;
-      const bool ok = i < c1;
-      const size_t io = ok ? (size_t)i : 0, o = io * w;
-      const size_t om = i > 0 && ok ? o - w : o;
-      cp_async_elem(sl + 0 * bd, rb + col + o, ok);
-      if (!split) {
-        cp_async_elem(sl + 1 * bd, x + xL0 + o, ok && useL);
-        cp_async_elem(sl + 2 * bd, x + xR0 + o, ok && useR);
-        cp_async_elem(sl + 3 * bd, wL ? P.wxl + wk + io : lx + colL + o, ok && useL);
-        cp_async_elem(sl + 4 * bd, wR ? P.wxh + wk + io : ux + col + o, ok && useR);
-      }
-      cp_async_elem(sl + 5 * bd, lz + col + om, ok && i > 0);
-      cp_async_elem(sl + 6 * bd, ft + col + o, ok);
-      cp_async_elem(sl + 7 * bd, frt + col + o, ok);
-      cp_commit();
-    };
-    for (int r = 0; r < kAhead; ++r) issue(r);
+  rhs_half<T, kWrap, 4>(P, mo, b, x, c, fwd);
+  const int c1 = P.c1, w = P.w;
+  const int nl = (P.c2 - c + 1) / 2;
+  constexpr int kB = sizeof(T) == 8 ? 4 : 8;
+  struct Batch {
+    T t[kB], lz[kB], ft[kB], frt[kB];
+  };
+  for (int q = threadIdx.x; q < nl; q += blockDim.x) {
+    const size_t col = (size_t)c * P.h + q;
+    T* xp = x + col;
+    const T *lzp = P.lz + mo + col, *ftp = P.ft + mo + col, *frtp = P.frt + mo + col, *fwp = P.fw + mo + col;
     T prev = (T)0;
-    for (int i = 0; i < c1; ++i) {
-      issue(i + kAhead);
-      cp_wait<kAhead>();
-      const T* sl = ring + (size_t)(i % kRing) * kFields * bd + tid;
-      T t = sl[0];
-      if (fwd) {
-        if (useL) t = t - sl[3 * bd] * sl[1 * bd];
-        if (useR) t = t - sl[4 * bd] * sl[2 * bd];
-      } else {
-        if (useR) t = t - sl[4 * bd] * sl[2 * bd];
-        if (useL) t = t - sl[3 * bd] * sl[1 * bd];
+    auto load = [&](Batch& B, int r0) {
+#pragma unroll
+      for (int r = 0; r < kB; ++r) {
+        const int i = min(r0 + r, c1 - 1), o = i * w;
+        B.t[r] = xp[o];
+        B.lz[r] = i > 0 ? lzp[o - w] : (T)0;
+        B.ft[r] = ftp[o];
+        B.frt[r] = frtp[o];
       }
-      if (i > 0) t = t - sl[5 * bd] * prev;
-      const T y = div_rn(t, sl[6 * bd], sl[7 * bd]);
-      x[col + (size_t)i * w] = y;
-      prev = y;
+    };
+    auto solve = [&](const Batch& B, int r0) {
+#pragma unroll
+      for (int r = 0; r < kB; ++r) {
+        if (r0 + r < c1) {
+          const T m = B.lz[r] * prev;  // row 0: t - 0*0
+          prev = div_rn(B.t[r] - m, B.ft[r], B.frt[r]);
+          xp[(r0 + r) * w] = prev;
+        }
+      }
+    };
+    {
+      Batch A, B;
+      load(A, 0);
+      for (int r0 = 0; r0 < c1; r0 += 2 * kB) {
+        load(B, r0 + kB);
+        solve(A, r0);
+        load(A, r0 + 2 * kB);
+        solve(B, r0 + kB);
+      }
     }
-    cp_wait<0>();
     // back substitution b(i) = b(i) - w(i)*b(i+1), rows c1-2 .. 0
     const int nb = c1 - 1;
-    T xa[4], wa[4], xb[4], wb[4];
-    auto load4 = [&](T* xs, T* ws, int r0) {
+    constexpr int kC = 8;
+    T xa[kC], wa[kC], xb[kC], wb[kC];
+    auto load_back = [&](T* xs, T* ws, int r0) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = c1 - 2 - (r0 + r);
+      for (int r = 0; r < kC; ++r) {
+        const int o = max(nb - 1 - (r0 + r), 0) * w;
+        xs[r] = xp[o];
+        ws[r] = fwp[o];
+      }
+    };
+    auto solve_back = [&](const T* xs, const T* ws, int r0) {
+#pragma unroll
+      for (int r = 0; r < kC; ++r) {
+        const int i = nb - 1 - (r0 + r);
         if (i >= 0) {
-          xs[r] = x[col + (size_t)i * w];
-          ws[r] = fw[col + (size_t)i * w];
+          prev = xs[r] - ws[r] * prev;
+          xp[i * w] = prev;
         }
       }
     };
-    auto solve4 = [&](const T* xs, const T* ws, int r0) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = c1 - 2 - (r0 + r);
-        if (i >= 0) {
-          const T v = xs[r] - ws[r] * prev;
-          x[col + (size_t)i * w] = v;
-          prev = v;
-        }
-      }
-    };
-    if (nb > 0) load4(xa, wa, 0);
-    for (int r0 = 0; r0 < nb; r0 += 8) {
-      load4(xb, wb, r0 + 4);
-      solve4(xa, wa, r0);
-      load4(xa, wa, r0 + 8);
-      solve4(xb, wb, r0 + 4);
+    load_back(xa, wa, 0);
+    for (int r0 = 0; r0 < nb; r0 += 2 * kC) {
+      load_back(xb, wb, r0 + kC);
+      solve_back(xa, wa, r0);
+      load_back(xa, wa, r0 + 2 * kC);
+      solve_back(xb, wb, r0 + kC);
     }
   }
 }
@@ -820,14 +786,14 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* __
 // Plane levels resident in shared memory.
 //
 // What bounds a plane's multigrid is the serial row recurrence of its line
-// solves plus a fixed cost per half-sweep: filling the row ring from L2, the
-// first loads of the back substitution, the restriction's round trips.  A
+// solves plus a fixed cost per half-sweep: the first loads of the forward and
+// the back substitution from L2, the restriction's round trips.  A
 // 64x32 block runs 2240 half-sweeps per V-cycle and the coarse plane levels
 // have rows and lines in the tens, so the fixed cost was half of the time.
 // The plane levels that fit (from the coarsest up, all of them for a plane of
 // up to about 2800 FP64 entries) are therefore copied to shared memory once
 // per plane solve, and their smoothing, residuals and transfers touch nothing
-// else; a level that does not fit streams through the ring as before.
+// else; a level that does not fit streams from global memory.
 //
 // One resident level, in units of T from its offset: the arrays d, uz, lz,
 // fw, ft, frt, ux, lx, x, b of n = padded(ps) values each, then (kWrap) wxl, wxh.
@@ -907,8 +873,7 @@ __device__ __forceinline__ void res_copy(const Lev2T<T>& G, int off, int k) {
 // line_half on a resident level: the same relaxation with its operands in
 // shared memory.  The next row's operands are loaded while this row's
 // recurrence runs, so an FP64 row costs the recurrence alone (five dependent
-// operations forward and two backward).  A missing neighbour contributes
-// t - 0*0, which leaves every bit of t.
+// operations forward and two backward; 370 and 150 cycles measured).
 template <typename T, bool kWrap>
 __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd) {
   if constexpr (sizeof(T) == 4) {
@@ -920,81 +885,26 @@ __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd)
       return;
     }
   }
-  const int c1 = S.c1, c2 = S.c2, h = S.h, w = S.w;
-  const int nl = (c2 - c + 1) / 2;
-  const bool split = split_rhs<T>(nl);
-  if (split) rhs_half<T, kWrap>(S, 0, S.b, S.x, c, fwd);
-  struct Row {
-    T b, xl, xr, cl, cr, lz, ft, frt;
-  };
+  rhs_half<T, kWrap, sizeof(T) == 8 ? 1 : 4>(S, 0, S.b, S.x, c, fwd);
+  const int c1 = S.c1, h = S.h, w = S.w;
+  const int nl = (S.c2 - c + 1) / 2;
   for (int q = threadIdx.x; q < nl; q += blockDim.x) {
-    const int j = 2 * q + c;
     const int col = c * h + q;
-    const bool hasL = j > 0, hasR = j < c2 - 1;
-    const int colL = hasL ? (1 - c) * h + ((j - 1) >> 1) : col;
-    const int colR = hasR ? (1 - c) * h + ((j + 1) >> 1) : col;
-    const bool wrap = kWrap && S.wxl && c2 >= 2 && ((c2 - 1) & 1);
-    const bool wL = wrap && j == 0, wR = wrap && j == c2 - 1;
-    const bool useL = hasL || wL, useR = hasR || wR;
-    const T* xL = S.x + (wL ? (int)slot(0, h, 0, c2 - 1) : colL);
-    const T* xR = S.x + (wR ? 0 : colR);
-    const T* cL = wL ? S.wxl : S.lx + colL;
-    const T* cR = wR ? S.wxh : S.ux + col;
-    const int sL = wL ? 1 : w, sR = wR ? 1 : w;
-    const T* bp = S.b + col;
     const T* lzp = S.lz + col;
     const T* ftp = S.ft + col;
     const T* frtp = S.frt + col;
     T* xp = S.x + col;
-    T prev = (T)0;
-    if (split) {
-      T t = xp[0], lz = (T)0, ft = ftp[0], frt = frtp[0];
-      for (int i = 0; i < c1; ++i) {
-        const T m = lz * prev;
-        const int in = (i + 1 < c1 ? i + 1 : i) * w;
-        const T tn = xp[in], lzn = lzp[in - (i + 1 < c1 ? w : 0)], ftn = ftp[in], frtn = frtp[in];
-        prev = div_rn(t - m, ft, frt);
-        xp[i * w] = prev;
-        t = tn;
-        lz = lzn;
-        ft = ftn;
-        frt = frtn;
-      }
-    } else {
-      auto load = [&](int i, Row& r) {
-        const int o = i * w;
-        r.b = bp[o];
-        r.xl = useL ? xL[o] : (T)0;
-        r.cl = useL ? cL[i * sL] : (T)0;
-        r.xr = useR ? xR[o] : (T)0;
-        r.cr = useR ? cR[i * sR] : (T)0;
-        r.lz = i > 0 ? lzp[o - w] : (T)0;
-        r.ft = ftp[o];
-        r.frt = frtp[o];
-      };
-      auto rhs = [&](const Row& r) {
-        const T ml = r.cl * r.xl, mr = r.cr * r.xr;
-        return fwd ? (r.b - ml) - mr : (r.b - mr) - ml;
-      };
-      Row cur, nxt;
-      load(0, cur);
-      load(c1 > 1 ? 1 : 0, nxt);
-      T t = rhs(cur);
-      T lz = (T)0, ft = cur.ft, frt = cur.frt;
-      for (int i = 0; i < c1; ++i) {
-        const T m = lz * prev;
-        Row nn;
-        load(i + 2 < c1 ? i + 2 : c1 - 1, nn);
-        const T tt = t - m;
-        const T y = div_rn(tt, ft, frt);
-        t = rhs(nxt);
-        lz = nxt.lz;
-        ft = nxt.ft;
-        frt = nxt.frt;
-        nxt = nn;
-        xp[i * w] = y;
-        prev = y;
-      }
+    T prev = (T)0, t = xp[0], lz = (T)0, ft = ftp[0], frt = frtp[0];
+    for (int i = 0; i < c1; ++i) {
+      const T m = lz * prev;  // row 0: t - 0*0
+      const int in = (i + 1 < c1 ? i + 1 : i) * w;
+      const T tn = xp[in], lzn = lzp[in - (i + 1 < c1 ? w : 0)], ftn = ftp[in], frtn = frtp[in];
+      prev = div_rn(t - m, ft, frt);
+      xp[i * w] = prev;
+      t = tn;
+      lz = lzn;
+      ft = ftn;
+      frt = frtn;
     }
     const T* fwp = S.fw + col;
     T ya = (T)0, wa = (T)0;
@@ -1023,10 +933,10 @@ __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd)
 __device__ __forceinline__ int gs_half_sweeps(int gi) { return gi > 0 ? 2 * gi + 1 : 0; }
 
 template <typename T, bool kWrap = false>
-__device__ void gs2d(const Lev2T<T>& P, size_t mo, const T* b, T* x, int gi, T* ring, int rs) {
+__device__ void gs2d(const Lev2T<T>& P, size_t mo, const T* b, T* x, int gi) {
   const int nh = P.c2 > 1 ? gs_half_sweeps(gi) : 1;
   for (int hs = 0; hs < nh; ++hs) {  // a single line is solved once
-    line_half<T, kWrap>(P, mo, b, x, hs & 1, P.c2 == 1 || (!(hs & 1) && hs + 1 < nh), ring, rs);
+    line_half<T, kWrap>(P, mo, b, x, hs & 1, P.c2 == 1 || (!(hs & 1) && hs + 1 < nh));
     __syncthreads();
   }
 }
@@ -1040,21 +950,51 @@ __device__ __noinline__ void gs2d_res(const Lev2T<T>& G, int off, int gi) {
   }
 }
 
+// MatVecT_2D at a fine entry without branches, for the residual: a missing
+// neighbour's coefficient and value are 0 and add 0*0 (which can turn a -0 into
+// +0 only, lost in the sum of residuals that starts from +0)
+template <typename T, bool kWrap>
+__device__ __forceinline__ T matvec2_flat(const Lev2T<T>& P, size_t mo, const T* x, int s, int i, int j, int k) {
+  const int c1 = P.c1, c2 = P.c2, w = P.w, h = P.h, row = i * w;
+  const bool up = i > 0, dn = i < c1 - 1, lf = j > 0, rt = j < c2 - 1;
+  const int sl = row + (lf ? (int)slot(0, h, 0, j - 1) : 0), sr = row + (rt ? (int)slot(0, h, 0, j + 1) : 0);
+  const T lzv = up ? P.lz[mo + s - w] : (T)0, xu = up ? x[s - w] : (T)0;
+  const T dv = P.d[mo + s], xc = x[s];
+  const T uzv = dn ? P.uz[mo + s] : (T)0, xd = dn ? x[s + w] : (T)0;
+  const T lxv = lf ? P.lx[mo + sl] : (T)0, xl = lf ? x[sl] : (T)0;
+  const T uxv = rt ? P.ux[mo + s] : (T)0, xr = rt ? x[sr] : (T)0;
+  T y = lzv * xu + dv * xc + uzv * xd;
+  y = y + lxv * xl + uxv * xr;
+  if (kWrap && P.wxl && (j == 0 || j == c2 - 1)) {  // periodic-Laplacian hierarchy: across the periodic x side
+    const size_t kc = (size_t)k * c1;
+    if (j == 0) y = y + P.wxl[kc + i] * x[row + slot(0, h, 0, c2 - 1)];
+    if (j == c2 - 1) y = y + P.wxh[kc + i] * x[row];
+  }
+  return y;
+}
+
 // Restriction of the residual: the coarse right-hand side is the sum of the
 // four fine residuals b - A x in the reference's order (one pass: the residual
-// itself is not stored), the coarse iterate starts from 0
-template <typename T, bool kWrap>
+// itself is not stored, and the four are evaluated without branches so that
+// all their loads are in flight), the coarse iterate starts from 0
+// kU residuals at a time: FP64 in shared memory one (the FP64 unit is the limit)
+template <typename T, bool kWrap, int kU>
 __device__ __forceinline__ void restrict2d(const Lev2T<T>& P, size_t mo, const T* b, const T* x, int k, int cw, int ch,
                                            int cc2, size_t cps, T* bq, T* xq) {
   for_plane(cw, cps, [&](size_t s, int a, int r) {
     const int bb = line_of(r, ch, cc2);
     if (bb < 0) return;
     T v = (T)0;
-    for (int i1 = 2 * a; i1 <= 2 * a + 1 && i1 < P.c1; ++i1)
-      for (int i2 = 2 * bb; i2 <= 2 * bb + 1 && i2 < P.c2; ++i2) {
-        const size_t e = slot(P.w, P.h, i1, i2);
-        v = v + (b[e] - matvec2_at<T, kWrap>(P, mo, x, e, i1, i2, k));
-      }
+#pragma unroll kU
+    for (int r = 0; r < 4; ++r) {
+      const int i1 = 2 * a + (r >> 1), i2 = 2 * bb + (r & 1);
+      const bool in = i1 < P.c1 && i2 < P.c2;
+      if (kU == 1 && !in) continue;
+      const int i1c = in ? i1 : 2 * a, i2c = in ? i2 : 2 * bb;
+      const int e = (int)slot(P.w, P.h, i1c, i2c);
+      const T d = b[e] - matvec2_flat<T, kWrap>(P, mo, x, e, i1c, i2c, k);
+      v = v + (in ? d : (T)0);
+    }
     bq[s] = v;
     xq[s] = (T)0;
   });
@@ -1062,7 +1002,7 @@ __device__ __forceinline__ void restrict2d(const Lev2T<T>& P, size_t mo, const T
 template <typename T, bool kWrap>
 __device__ __noinline__ void restrict2d_res(const Lev2T<T>& G, int off, const Lev2T<T>& Gc, int offc) {
   const Lev2T<T> S = res_level(G, off), C = res_level(Gc, offc);
-  restrict2d<T, kWrap>(S, 0, S.b, S.x, 0, C.w, C.h, C.c2, C.ps, C.b, C.x);
+  restrict2d<T, kWrap, sizeof(T) == 8 ? 1 : 4>(S, 0, S.b, S.x, 0, C.w, C.h, C.c2, C.ps, C.b, C.x);
 }
 
 // x of level F corrected by x of the next coarser level P
@@ -1077,7 +1017,7 @@ __device__ __forceinline__ void prolong2d(int fw, int fh, int fc2, size_t fps, T
 // Multigrid_2D (TriDiagT_Mod.f90:490-551) on plane k of a 3D level, inside one
 // CTA; the plane levels from mr on are resident at roff[level]
 template <typename T, bool kWrap = false>
-__device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, T* ring, int rs, int mr, const int* roff) {
+__device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, int mr, const int* roff) {
   const int nl = A.nl;
   int gi = 1;
   auto xg = [&](int lv) { return lv == 0 ? x0 : A.pl[lv].x + (size_t)k * A.pl[lv].ps; };
@@ -1086,7 +1026,7 @@ __device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, T* r
     if (lv >= mr)
       gs2d_res<T, kWrap>(A.pl[lv], roff[lv], gi);
     else
-      gs2d<T, kWrap>(A.pl[lv], (size_t)k * A.pl[lv].ps, bg(lv), xg(lv), gi, ring, rs);
+      gs2d<T, kWrap>(A.pl[lv], (size_t)k * A.pl[lv].ps, bg(lv), xg(lv), gi);
   };
   for (int lv = 0; lv < nl; ++lv) {
     smooth(lv);
@@ -1106,7 +1046,7 @@ __device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, T* r
         bq = Q.b + (size_t)k * Q.ps;
         xq = Q.x + (size_t)k * Q.ps;
       }
-      restrict2d<T, kWrap>(P, (size_t)k * P.ps, bg(lv), xg(lv), k, Q.w, Q.h, Q.c2, Q.ps, bq, xq);
+      restrict2d<T, kWrap, sizeof(T) == 8 ? 2 : 4>(P, (size_t)k * P.ps, bg(lv), xg(lv), k, Q.w, Q.h, Q.c2, Q.ps, bq, xq);
     }
     __syncthreads();
   }
@@ -1133,16 +1073,25 @@ __device__ void mg2d(const Lev3T<T>& A, int k, T* x0, const T* b0, int gi2, T* r
 // 3D level L: each CTA forms its plane's right-hand side (forward or backward
 // operation order of the reference) and runs Solve_2D on it.  mr: the first
 // resident plane level (0: the whole plane solve runs in shared memory, only
-// x goes back; A.nl: none); rs: threads of the ring.
+// x goes back; A.nl: none).
+// A half-sweep of a small level takes tens of microseconds, of which starting
+// the kernel and copying the matrix to shared memory are several: the level's
+// descriptor is a kernel parameter, and the half-sweeps that follow one another
+// are launched with programmatic serialisation, so that the next one's blocks
+// start on idle SMs and copy their matrix (which no half-sweep writes) while
+// this one runs; they wait for it before they touch x or b.
 template <typename T, bool kWrap = false>
-__global__ void __launch_bounds__(kPlaneBlock, 2) k_plane_half(const Lev3T<T>* __restrict__ lvs, int L, int color, int fwd,
-                                                             int mult_iter2, int gi2, int mr, int rs) {
+__global__ void __launch_bounds__(kPlaneBlock, 2) k_plane_half(const __grid_constant__ Lev3T<T> lev, int color, int fwd,
+                                                             int mult_iter2, int gi2, int mr) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ Lev3T<T> A;
   __shared__ int roff[kMaxLev + 1];
-  T* ring = reinterpret_cast<T*>(plane_smem);  // kRing * kFields * rs values of T (mr > 0), then the resident levels
+  static_assert(sizeof(Lev3T<T>) % 8 == 0, "copied by 8-byte words");
+  for (int q = threadIdx.x; q < (int)(sizeof(Lev3T<T>) / 8); q += blockDim.x)
+    reinterpret_cast<unsigned long long*>(&A)[q] = reinterpret_cast<const unsigned long long*>(&lev)[q];
+  __syncthreads();
   if (threadIdx.x == 0) {
-    A = lvs[L];
-    int o = mr > 0 ? RingCfg<T>::ring * kFields * rs : 0;
+    int o = 0;
     for (int lv = mr; lv < A.nl; ++lv) {
       roff[lv] = o;
       o += res_elems<T>(A.pl[lv].c1, A.pl[lv].ps, A.pl[lv].wxl != nullptr);
@@ -1155,6 +1104,7 @@ __global__ void __launch_bounds__(kPlaneBlock, 2) k_plane_half(const Lev3T<T>* _
     if (k >= A.m3) break;
     for (int lv = mr; lv < A.nl; ++lv) res_copy(A.pl[lv], roff[lv], k);
     cp_commit();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the half-sweep before (no-op after an ordinary launch)
     const size_t off = (size_t)k * P0.ps, ps = P0.ps;
     T *x0 = A.x + off, *t0 = A.t + off;
     if (mr == 0) {
@@ -1162,29 +1112,47 @@ __global__ void __launch_bounds__(kPlaneBlock, 2) k_plane_half(const Lev3T<T>* _
       x0 = S.x;
       t0 = S.b;
     }
-    for_plane(P0.w, ps, [&](size_t s, int, int r) {
-      if (line_of(r, P0.h, P0.c2) < 0) return;
-      const size_t e = off + s;
-      T v = A.b[e];
-      if (fwd) {
-        if (k > 0) v = v - A.l3[e - ps] * A.x[e - ps];
-        if (k < A.m3 - 1) v = v - A.u3[e] * A.x[e + ps];
-      } else {
-        if (k < A.m3 - 1) v = v - A.u3[e] * A.x[e + ps];
-        if (k > 0) v = v - A.l3[e - ps] * A.x[e - ps];
+    // the plane's right-hand side, four slots a thread at a time (padded slots
+    // hold zeros everywhere and stay zero)
+    const bool lo = k > 0, hi = k < A.m3 - 1;
+    const bool wrap = kWrap && A.wyl && A.m3 >= 2 && ((A.m3 - 1) & 1);
+    const T *pb = A.b + off, *pl = A.l3 + off - (lo ? ps : 0), *pu = A.u3 + off, *px = A.x + off;
+    const T *xm = px - (lo ? ps : 0), *xp = px + (hi ? ps : 0);
+    constexpr int kU = sizeof(T) == 8 ? 2 : 4;
+    for (size_t s0 = threadIdx.x; s0 < ps; s0 += kU * (size_t)blockDim.x) {
+      T v[kU], cl[kU], vl[kU], cu[kU], vu[kU], xc[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const size_t s = s0 + u * (size_t)blockDim.x;
+        if (s >= ps) continue;
+        v[u] = pb[s];
+        if (lo) cl[u] = pl[s], vl[u] = xm[s];
+        if (hi) cu[u] = pu[s], vu[u] = xp[s];
+        if (mr == 0) xc[u] = px[s];
       }
-      // periodic-Laplacian hierarchy: the plane across the periodic y side
-      // (only when planes 0 and m3-1 have different parities)
-      if (kWrap && A.wyl && A.m3 >= 2 && ((A.m3 - 1) & 1)) {
-        if (k == 0) v = v - A.wyl[s] * A.x[(size_t)(A.m3 - 1) * ps + s];
-        if (k == A.m3 - 1) v = v - A.wyh[s] * A.x[s];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const size_t s = s0 + u * (size_t)blockDim.x;
+        if (s >= ps) continue;
+        T t = v[u];
+        if (fwd) {
+          if (lo) t = t - cl[u] * vl[u];
+          if (hi) t = t - cu[u] * vu[u];
+        } else {
+          if (hi) t = t - cu[u] * vu[u];
+          if (lo) t = t - cl[u] * vl[u];
+        }
+        // periodic-Laplacian hierarchy: the plane across the periodic y side
+        // (only when planes 0 and m3-1 have different parities)
+        if (wrap && k == 0) t = t - A.wyl[s] * A.x[(size_t)(A.m3 - 1) * ps + s];
+        if (wrap && k == A.m3 - 1) t = t - A.wyh[s] * A.x[s];
+        t0[s] = t;
+        if (mr == 0) x0[s] = xc[u];
       }
-      t0[s] = v;
-      if (mr == 0) x0[s] = A.x[e];
-    });
+    }
     cp_wait<0>();
     __syncthreads();
-    for (int it = 0; it < mult_iter2; ++it) mg2d<T, kWrap>(A, k, x0, t0, gi2, ring, rs, mr, roff);
+    for (int it = 0; it < mult_iter2; ++it) mg2d<T, kWrap>(A, k, x0, t0, gi2, mr, roff);
     if (mr == 0) {  // x0 is final: the last smoother ended with a block barrier
       for_plane(P0.w, ps, [&](size_t s, int, int r) {
         if (line_of(r, P0.h, P0.c2) >= 0) A.x[off + s] = x0[s];
@@ -2080,25 +2048,23 @@ int proj_build(asam_ctx* h) {
 // memory: as many as fit, from the coarsest up, in one CTA's share of an SM
 // (two CTAs per SM when there are more planes than SMs)
 struct PlanePlan {
-  int mr, rs;
+  int mr;
   size_t smem;
 };
 template <typename T>
 PlanePlan plane_plan(const Lev3T<T>& A, int np) {
   const size_t cap = np > 152 ? kPlaneSmem2 : kPlaneSmem1;
-  const int rs = std::min(kPlaneBlock, (A.pl[0].h + 31) / 32 * 32);
-  const size_t ring = (size_t)RingCfg<T>::ring * kFields * rs * sizeof(T);
   size_t used = 0;
   int mr = A.nl;
   while (mr > 0) {
     const Lev2T<T>& P = A.pl[mr - 1];
     if (P.ps > cap / (10 * sizeof(T))) break;
     const size_t add = (size_t)res_elems<T>(P.c1, P.ps, P.wxl != nullptr) * sizeof(T);
-    if (used + add + (mr > 1 ? ring : 0) > cap) break;
+    if (used + add > cap) break;
     used += add;
     --mr;
   }
-  return PlanePlan{mr, rs, used + (mr > 0 ? ring : 0)};
+  return PlanePlan{mr, used};
 }
 
 // Solve_3D from a zero start on level 0 (VCycleCG's MatrixT branch): lv[0].b
@@ -2113,11 +2079,23 @@ void vcycle_run(asam_ctx* h, std::vector<Lev3T<T>>& lv, Lev3T<T>* d_lv, int gi2,
   cudaMemsetAsync(lv[0].x, 0, sizeof(T) * len0(s), st);
   auto gs3 = [&](int L, int gi) {
     const Lev3T<T>& A = lv[L];
+    bool after_half = false;
     auto half = [&](int c, int fwd) {
       const int np = (A.m3 - c + 1) / 2;
       if (np <= 0) return;
       const PlanePlan pp = plane_plan(A, np);
-      k_plane_half<T, kWrap><<<np, kPlaneBlock, pp.smem, st>>>(d_lv, L, c, fwd, mi2, gi2, pp.mr, pp.rs);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(np);
+      cfg.blockDim = dim3(kPlaneBlock);
+      cfg.dynamicSmemBytes = pp.smem;
+      cfg.stream = st;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at.val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = after_half ? 1 : 0;  // the launch before in the stream is a half-sweep
+      cudaLaunchKernelEx(&cfg, k_plane_half<T, kWrap>, A, c, fwd, mi2, gi2, pp.mr);
+      after_half = true;
       ++nl;
     };
     if (A.m3 > 1) {
