@@ -797,9 +797,7 @@ int forward_record(asam_ctx* h, const double* c, double dt, double tol, std::vec
     }
     int rc = fcn_dev(h, cur, h->rhs);
     if (rc) return rc;
-    launch_scale_host(L, len, dt, h->rhs);
-    for (int js = 0; js < is; ++js)
-      launch_axpy_host(L, len, h->beta[is * 4 + js], h->incr + (size_t)js * len, h->rhs);
+    launch_lincomb(L, len, h->rhs, &dt, is, h->beta + is * 4, h->incr, h->rhs);
     double* x = h->incr + (size_t)is * len;
     CK(cudaMemsetAsync(x, 0, len * sizeof(double), L.stream));
     int it = 200;
@@ -807,8 +805,7 @@ int forward_record(asam_ctx* h, const double* c, double dt, double tol, std::vec
     rc = bicgstab_dev<double>(h, h->val, x, h->rhs, &it, &t, h->w64, true);
     if (rc != kOk && rc != kNotConverged) return rc;
     launch_exchange_cell(L, d, nc, x);
-    CK(cudaMemcpyAsync(cur, h->cold, len * sizeof(double), cudaMemcpyDeviceToDevice, L.stream));
-    for (int js = 0; js <= is; ++js) launch_axpy_host(L, len, h->alpha[is * 4 + js], h->incr + (size_t)js * len, cur);
+    launch_lincomb(L, len, h->cold, nullptr, is + 1, h->alpha + is * 4, h->incr, cur);
   }
   return check_launch();
 }

@@ -210,6 +210,7 @@ enum ScalarOp {
   OP_RNORM_HALF = 5,  // rnorm = sqrt(sum); converged-at-half-step flag
   OP_OMEGA = 6,       // omega = dot_a / sum   (dot_a = (t,r), sum = (t,t))
   OP_RNORM_FULL = 7,  // rnorm = sqrt(sum); converged flag
+  OP_RNORM0_RHO = 8,  // OP_RNORM0 and OP_RHO of one sum (the shadow residual is the residual)
 };
 // Which device scalar scales an update.
 enum ScalarSel { SEL_ALPHA = 0, SEL_OMEGA = 1, SEL_BETA = 2 };

@@ -4,6 +4,7 @@
 // host only reads the convergence flag twice per iteration.
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -305,17 +306,21 @@ void gs_schedule_free(asam_ctx* h) {
 // pipelined wavefront), zero halo, exchange.  The FP32 inner solver of the
 // refined mode may use the vertical-column line solve instead of the sweeps.
 template <typename T>
-void psolve_dev(asam_ctx* h, const T* val, const T* in, T* out, Work<T>& w) {
+void psolve_dev(asam_ctx* h, const T* val, const T* in, T* out, Work<T>& w, bool own) {
   const Launch& L = h->L;
   const Dims& d = h->d;
   const int nc = h->cfg.ncomp;
-  cudaMemcpyAsync(w.bbuf, in, h->len * sizeof(T), cudaMemcpyDeviceToDevice, L.stream);
-  launch_exchange_cell(L, d, nc, w.bbuf);
+  // own: in is a vector of the Krylov solver, whose periodic halos nothing but
+  // this preconditioner reads (dot products run over interior cells, products
+  // over the preconditioned vectors), so it is exchanged in place
+  T* rhs = own ? const_cast<T*>(in) : w.bbuf;
+  if (!own) cudaMemcpyAsync(w.bbuf, in, h->len * sizeof(T), cudaMemcpyDeviceToDevice, L.stream);
+  launch_exchange_cell(L, d, nc, rhs);
   const bool inner = sizeof(T) == sizeof(float);  // FP32 inner solver of the refined mode
   const int nsweep = 1 + (inner ? h->cfg.inner_gs_iter : h->cfg.gs_iter);
   if (inner && h->cfg.inner_precond != 0) {  // 1: z lines, 2: x lines, 3: y lines
     const int axis = h->cfg.inner_precond == 1 ? 2 : h->cfg.inner_precond == 2 ? 0 : 1;
-    launch_line_psolve(L, d, nc, val, w.bbuf, out, w.tbuf, axis, (const T*)h->xl_w, (const T*)h->xl_r);
+    launch_line_psolve(L, d, nc, val, rhs, out, w.tbuf, axis, (const T*)h->xl_w, (const T*)h->xl_r);
   } else if (inner && h->gs_order) {
     const GsTileSched sch{h->gs_order,
                           h->gs_nticket,
@@ -325,9 +330,9 @@ void psolve_dev(asam_ctx* h, const T* val, const T* in, T* out, Work<T>& w) {
                           reinterpret_cast<unsigned*>(h->gs_counter + 1),
                           gs_group_of(h->cfg),
                           h->gs_spin > 0 ? h->gs_spin : kGsSpinLimit};
-    launch_gs_persist(L, d, nc, val, w.bbuf, out, w.tbuf, nsweep, sch);
+    launch_gs_persist(L, d, nc, val, rhs, out, w.tbuf, nsweep, sch);
   } else {
-    launch_gs_sweeps(L, d, nc, val, w.bbuf, out, w.tbuf, nsweep, gs_group_of(h->cfg));
+    launch_gs_sweeps(L, d, nc, val, rhs, out, w.tbuf, nsweep, gs_group_of(h->cfg));
   }
   launch_zero_halo(L, d, nc, out);
   launch_exchange_cell(L, d, nc, out);
@@ -396,10 +401,22 @@ void prepare_inner(asam_ctx* h) {
   }
 }
 
+// x into two or three arrays
+template <typename T>
+__global__ void k_copy3(size_t len, const T* x, T* y0, T* y1, T* y2) {
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x) {
+    const T v = x[q];
+    if (y0) y0[q] = v;
+    y1[q] = v;
+    y2[q] = v;
+  }
+}
+
 // BiCGStabMet_Vec4CellSp (MODULE/SpMatrix4CellPar_Mod.f90:245-348) on the device.
+// loaded: the caller has put b into w.r, w.rt and w.p (x = 0).
 template <typename T>
 int bicgstab_dev(asam_ctx* h, const T* val, T* x, const T* b, int* maxiter, double* tol, Work<T>& w,
-                 bool x_is_zero) {
+                 bool x_is_zero, bool loaded) {
   const Launch& L = h->L;
   const Dims& d = h->d;
   const int nc = h->cfg.ncomp;
@@ -407,32 +424,32 @@ int bicgstab_dev(asam_ctx* h, const T* val, T* x, const T* b, int* maxiter, doub
   memset(h->sc_host, 0, sizeof(KrylovScalars));
   h->sc_host->tol = *tol;
   CK(cudaMemcpyAsync(h->sc, h->sc_host, sizeof(KrylovScalars), cudaMemcpyHostToDevice, L.stream));
-  if (x_is_zero) {  // r = b - A*0 = b exactly
-    CK(cudaMemcpyAsync(w.r, b, len * sizeof(T), cudaMemcpyDeviceToDevice, L.stream));
-  } else {
+  if (!x_is_zero) {
     launch_matvec(L, d, nc, val, x, w.r, 0);
     launch_xpay_host(L, len, b, (T)-1, w.r);
   }
-  CK(cudaMemcpyAsync(w.rt, w.r, len * sizeof(T), cudaMemcpyDeviceToDevice, L.stream));
-  launch_dot(L, d, nc, w.r, w.r, h->partial, h->sc, OP_RNORM0, nullptr);
+  if (!loaded) {  // r~ = p = r, and r = b - A*0 = b exactly for x = 0
+    k_copy3<T><<<std::min((size_t)L.sm_count * 16, (len + 255) / 256), 256, 0, L.stream>>>(
+        len, x_is_zero ? b : w.r, x_is_zero ? w.r : nullptr, w.rt, w.p);
+    count_launches(1);
+  }
+  launch_dot(L, d, nc, w.r, w.r, h->partial, h->sc, OP_RNORM0_RHO, nullptr);  // |r0| and (r~, r)
   if (sizeof(T) == sizeof(float)) prepare_inner(h);
   const int prec = sizeof(T) == sizeof(float) ? 1 : 0;
   auto half1 = [&](bool first) {
-    launch_dot(L, d, nc, w.rt, w.r, h->partial, h->sc, OP_RHO, nullptr);
-    if (first) {
-      cudaMemcpyAsync(w.p, w.r, len * sizeof(T), cudaMemcpyDeviceToDevice, L.stream);
-    } else {
+    if (!first) {
+      launch_dot(L, d, nc, w.rt, w.r, h->partial, h->sc, OP_RHO, nullptr);
       launch_beta(L, h->sc);
       launch_pupdate(L, len, h->sc, w.r, w.v, w.p);
     }
-    psolve_dev<T>(h, val, w.p, w.ph, w);
+    psolve_dev<T>(h, val, w.p, w.ph, w, true);
     launch_matvec_dot(L, d, nc, val, w.ph, w.v, w.rt, h->partial, h->sc, OP_ALPHA);  // v = A ph, (r~, v)
     launch_axpy_dot(L, d, nc, h->sc, SEL_ALPHA, -1.0, w.v, w.r, h->partial, OP_RNORM_HALF);  // r -= alpha v, (r, r)
   };
   // second half without the update of x (launched after it: x is the
   // caller's array, and nothing in the half reads alpha/omega after it)
   auto half2 = [&]() {
-    psolve_dev<T>(h, val, w.r, w.rh, w);
+    psolve_dev<T>(h, val, w.r, w.rh, w, true);
     // t = A rh with (t, r) and (t, t); r -= omega t with (r, r)
     launch_matvec_dot2(L, d, nc, val, w.rh, w.t, w.r, h->partial, h->sc, OP_STORE_A, OP_OMEGA);
     launch_axpy_dot(L, d, nc, h->sc, SEL_OMEGA, -1.0, w.t, w.r, h->partial, OP_RNORM_FULL);
@@ -484,16 +501,17 @@ int bicgstab_refined(asam_ctx* h, double* x, const double* b, int* maxiter, doub
   const int nc = h->cfg.ncomp;
   const size_t len = h->len;
   double* r = h->w64.r;
-  if (x_is_zero) {  // r = b - A*0 = b
-    CK(cudaMemcpyAsync(r, b, len * sizeof(double), cudaMemcpyDeviceToDevice, L.stream));
-  } else {
+  if (!x_is_zero) {
     launch_matvec(L, d, nc, h->val, x, r, 0);
     launch_xpay_host(L, len, b, -1.0, r);
   }
-  launch_dot(L, d, nc, r, r, h->partial, h->sc, OP_STORE_A, h->red_out);
+  const double* r0 = x_is_zero ? b : r;  // r = b - A*0 = b
+  launch_dot(L, d, nc, r0, r0, h->partial, h->sc, OP_STORE_A, h->red_out);
   double rr0 = 0;
   int rc = reduce_to_host(h, &rr0);
   if (rc) return rc;
+  // x = 0 is first written by the first correction
+  if (x_is_zero && !(rr0 > 0.0)) CK(cudaMemsetAsync(x, 0, len * sizeof(double), L.stream));
   if (std::isnan(rr0)) {
     set_last_error("NaN in the stage system", __FILE__, __LINE__);
     return kNanDetected;
@@ -510,18 +528,21 @@ int bicgstab_refined(asam_ctx* h, double* x, const double* b, int* maxiter, doub
   const int max_outer = 8;
   for (int outer = 0; outer < max_outer; ++outer) {
     // the inner system is A d = r/|r| (unit scale in FP32); x += |r| d
-    launch_convert_f64_to_f32_scaled(L, len, r, 1.0 / rnorm, h->b32);
+    launch_convert_f64_to_f32_scaled3(L, len, outer == 0 ? r0 : r, 1.0 / rnorm, h->w32.r, h->w32.rt, h->w32.p);
     CK(cudaMemsetAsync(h->x32, 0, len * sizeof(float), L.stream));
     int it = h->cfg.bicgstab_maxiter;
     double tin = 0.5 * target / rnorm;
     if (tin < 1e-6) tin = 1e-6;
     if (tin > 1e-2) tin = 1e-2;
-    rc = bicgstab_dev<float>(h, h->val32, h->x32, h->b32, &it, &tin, h->w32, true);
+    rc = bicgstab_dev<float>(h, h->val32, h->x32, nullptr, &it, &tin, h->w32, true, true);
     // an inner breakdown or iteration limit still leaves a usable correction:
     // the outer FP64 residual decides
     if (rc != kOk && rc != kNotConverged && rc != kBreakdown) return rc;
     total_inner += it < 0 ? -it : (it > h->cfg.bicgstab_maxiter ? it / 2 : it);
-    launch_add_f32_to_f64(L, len, h->x32, rnorm, x);                             // x += |r| * correction
+    if (outer == 0 && x_is_zero)
+      launch_set_f32_to_f64(L, len, h->x32, rnorm, x);
+    else
+      launch_add_f32_to_f64(L, len, h->x32, rnorm, x);  // x += |r| * correction
     asam_fma::launch_resid_dot(L, d, nc, h->val, x, b, r, h->partial, h->sc, OP_STORE_A, h->red_out);  // r, r.r
     double rr = 0;
     rc = reduce_to_host(h, &rr);
@@ -573,8 +594,10 @@ int jac_dev(asam_ctx* h, const double* c, double dt) {
   return check_launch();
 }
 
+// x_is_zero: the start value is 0, x need not hold it
 int solve_dev(asam_ctx* h, double* x, const double* b, int* maxiter, double* tol, bool x_is_zero) {
   if (h->cfg.precision == ASAM_PREC_FP32_REFINED) return bicgstab_refined(h, x, b, maxiter, tol, x_is_zero);
+  if (x_is_zero) CK(cudaMemsetAsync(x, 0, h->len * sizeof(double), h->L.stream));
   return bicgstab_dev<double>(h, h->val, x, b, maxiter, tol, h->w64, x_is_zero);
 }
 
@@ -597,10 +620,8 @@ int ros_step_dev(asam_ctx* h, double* c, double dt, int* iters, double* resid) {
     }
     int rc = fcn_dev(h, c, h->rhs);
     if (rc) return rc;
-    launch_scale_host(L, len, dt, h->rhs);
-    for (int js = 0; js < is; ++js) launch_axpy_host(L, len, h->beta[is * 4 + js], h->incr + (size_t)js * len, h->rhs);
+    launch_lincomb(L, len, h->rhs, &dt, is, h->beta + is * 4, h->incr, h->rhs);
     double* x = h->incr + (size_t)is * len;
-    CK(cudaMemsetAsync(x, 0, len * sizeof(double), L.stream));
     int it = h->cfg.bicgstab_maxiter;
     double tol = h->cfg.bicgstab_tol;
     rc = solve_dev(h, x, h->rhs, &it, &tol, true);
@@ -609,9 +630,7 @@ int ros_step_dev(asam_ctx* h, double* c, double dt, int* iters, double* resid) {
     if (iters) iters[is] = it;
     if (resid) resid[is] = tol;
     launch_exchange_cell(L, d, nc, x);
-    launch_exchange_cell(L, d, nc, x);
-    CK(cudaMemcpyAsync(c, h->cold, len * sizeof(double), cudaMemcpyDeviceToDevice, L.stream));
-    for (int js = 0; js <= is; ++js) launch_axpy_host(L, len, h->alpha[is * 4 + js], h->incr + (size_t)js * len, c);
+    launch_lincomb(L, len, h->cold, nullptr, is + 1, h->alpha + is * 4, h->incr, c);
   }
   int rc = check_launch();
   return rc ? rc : status;
@@ -645,11 +664,12 @@ int stage_out_end(asam_ctx* h, double* p, size_t n, double* dev) {
   return kOk;
 }
 
-template void psolve_dev<double>(asam_ctx*, const double*, const double*, double*, Work<double>&);
-template void psolve_dev<float>(asam_ctx*, const float*, const float*, float*, Work<float>&);
+template void psolve_dev<double>(asam_ctx*, const double*, const double*, double*, Work<double>&, bool);
+template void psolve_dev<float>(asam_ctx*, const float*, const float*, float*, Work<float>&, bool);
 template int bicgstab_dev<double>(asam_ctx*, const double*, double*, const double*, int*, double*, Work<double>&,
-                                  bool);
-template int bicgstab_dev<float>(asam_ctx*, const float*, float*, const float*, int*, double*, Work<float>&, bool);
+                                  bool, bool);
+template int bicgstab_dev<float>(asam_ctx*, const float*, float*, const float*, int*, double*, Work<float>&, bool,
+                                 bool);
 
 }  // namespace asam
 

@@ -138,10 +138,10 @@ int reduce_to_host(asam_ctx* h, double* out);
 bool is_device_ptr(const void* p);
 bool device_array(const void* p);  // device memory, false without a CUDA driver
 template <typename T>
-void psolve_dev(asam_ctx* h, const T* val, const T* in, T* out, Work<T>& w);
+void psolve_dev(asam_ctx* h, const T* val, const T* in, T* out, Work<T>& w, bool own = false);
 template <typename T>
 int bicgstab_dev(asam_ctx* h, const T* val, T* x, const T* b, int* maxiter, double* tol, Work<T>& w,
-                 bool x_is_zero);
+                 bool x_is_zero, bool loaded = false);
 int fcn_dev(asam_ctx* h, const double* c, double* f);
 int jac_dev(asam_ctx* h, const double* c, double dt);
 int solve_dev(asam_ctx* h, double* x, const double* b, int* maxiter, double* tol, bool x_is_zero);

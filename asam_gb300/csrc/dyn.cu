@@ -333,10 +333,8 @@ int ros_step_dyn(asam_ctx* h, double* c, double dt, int* iters, double* resid, i
       if ((rc = asam_lapl_compute(h, h->beta0, dt))) return rc;
     }
     fcn_dyn_dev(h, c, s->pre, h->rhs);
-    launch_scale_host(L, len, dt, h->rhs);
-    for (int js = 0; js < is; ++js) launch_axpy_host(L, len, h->beta[is * 4 + js], h->incr + (size_t)js * len, h->rhs);
+    launch_lincomb(L, len, h->rhs, &dt, is, h->beta + is * 4, h->incr, h->rhs);
     double* x = h->incr + (size_t)is * len;
-    CK(cudaMemsetAsync(x, 0, len * sizeof(double), L.stream));
     int it = h->cfg.bicgstab_maxiter;
     double tol = h->cfg.bicgstab_tol;
     rc = solve_dev(h, x, h->rhs, &it, &tol, true);
@@ -366,8 +364,7 @@ int ros_step_dyn(asam_ctx* h, double* c, double dt, int* iters, double* resid, i
       count_launches(1);
     }
     launch_exchange_cell(L, d, nc, x);
-    CK(cudaMemcpyAsync(c, h->cold, len * sizeof(double), cudaMemcpyDeviceToDevice, L.stream));
-    for (int js = 0; js <= is; ++js) launch_axpy_host(L, len, h->alpha[is * 4 + js], h->incr + (size_t)js * len, c);
+    launch_lincomb(L, len, h->cold, nullptr, is + 1, h->alpha + is * 4, h->incr, c);
   }
   // the transport operators of later calls see the new velocity
   launch_face_coef(L, d, h->geom(), h->coef_x, h->coef_y, h->coef_z, h->mask_x, h->mask_y, h->mask_z);

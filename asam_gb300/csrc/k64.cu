@@ -24,6 +24,39 @@ __global__ void k_cvt_d2f_scaled(size_t len, const double* __restrict__ x, doubl
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x)
     y[q] = (float)(s * x[q]);
 }
+// the same into the inner solver's residual, shadow residual and search direction
+__global__ void k_cvt_d2f_scaled3(size_t len, const double* __restrict__ x, double s, float* __restrict__ y0,
+                                  float* __restrict__ y1, float* __restrict__ y2) {
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x) {
+    const float v = (float)(s * x[q]);
+    y0[q] = v;
+    y1[q] = v;
+    y2[q] = v;
+  }
+}
+// y = 0 + s * x: k_add_f2d on a zero y
+__global__ void k_set_f2d(size_t len, const float* __restrict__ x, double s, double* __restrict__ y) {
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x)
+    y[q] = 0.0 + s * (double)x[q];
+}
+// out = s*base (base itself unless kScale), then out = a_j x_j + out for every
+// term: a stage's right-hand side or state in one pass over its arrays instead
+// of a copy or a scaling and a pass per term, with the same roundings
+struct LinTerms {
+  int n;
+  double a[4];
+  const double* x[4];
+};
+template <bool kScale>
+__global__ void k_lincomb(size_t len, LinTerms t, const double* base, double s, double* out) {
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x) {
+    double v = kScale ? s * base[q] : base[q];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < t.n) v = t.a[j] * t.x[j][q] + v;
+    out[q] = v;
+  }
+}
 // slots 7 and 8 of the DIA storage: 1/diagonal (correctly rounded) and its
 // 64-bit reciprocal
 __global__ void k_recip_diag(size_t n, double* __restrict__ val) {
@@ -61,6 +94,29 @@ void launch_add_f32_to_f64(const Launch& L, size_t len, const float* x, double s
 }
 void launch_convert_f64_to_f32_scaled(const Launch& L, size_t len, const double* x, double s, float* y) {
   k_cvt_d2f_scaled<<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, x, s, y);
+  count_launches(1);
+}
+void launch_convert_f64_to_f32_scaled3(const Launch& L, size_t len, const double* x, double s, float* y0, float* y1,
+                                       float* y2) {
+  k_cvt_d2f_scaled3<<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, x, s, y0, y1, y2);
+  count_launches(1);
+}
+void launch_set_f32_to_f64(const Launch& L, size_t len, const float* x, double s, double* y) {
+  k_set_f2d<<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, x, s, y);
+  count_launches(1);
+}
+void launch_lincomb(const Launch& L, size_t len, const double* base, const double* scale, int nterm, const double* a,
+                    const double* x, double* out) {
+  LinTerms t{};
+  for (int j = 0; j < nterm; ++j)
+    if (a[j] != 0.0) {
+      t.a[t.n] = a[j];
+      t.x[t.n++] = x + (size_t)j * len;
+    }
+  if (scale)
+    k_lincomb<true><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, t, base, *scale, out);
+  else
+    k_lincomb<false><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, t, base, 1.0, out);
   count_launches(1);
 }
 void launch_resid_dot(const Launch& L, const Dims& d, int ncomp, const double* val, const double* x, const double* b,

@@ -2034,6 +2034,7 @@ __global__ void k_dot_final(const double* __restrict__ partial, int npart, asam:
     case OP_STORE_A: sc->dot_a = s; break;
     case OP_STORE_B: sc->dot_b = s; break;
     case OP_RNORM0: sc->rnorm0 = sqrt(s); break;
+    case OP_RNORM0_RHO: sc->rnorm0 = sqrt(s); [[fallthrough]];
     case OP_RHO:
       sc->rho_old = sc->rho;
       sc->rho = s;

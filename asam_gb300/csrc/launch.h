@@ -69,6 +69,12 @@ void launch_convert_f64_to_f32(const Launch&, size_t len, const double* x, float
 void launch_convert_f32_to_f64(const Launch&, size_t len, const float* x, double* y);
 void launch_add_f32_to_f64(const Launch&, size_t len, const float* x, double s, double* y);
 void launch_convert_f64_to_f32_scaled(const Launch&, size_t len, const double* x, double s, float* y);
+void launch_convert_f64_to_f32_scaled3(const Launch&, size_t len, const double* x, double s, float* y0, float* y1,
+                                       float* y2);
+void launch_set_f32_to_f64(const Launch&, size_t len, const float* x, double s, double* y);
+// out = base (scaled by *scale when given) + sum of the nterm <= 4 terms a[j]*x_j, x_j at x + j*len
+void launch_lincomb(const Launch&, size_t len, const double* base, const double* scale, int nterm, const double* a,
+                    const double* x, double* out);
 void launch_resid_dot(const Launch&, const Dims&, int ncomp, const double* val, const double* x, const double* b,
                       double* r, double* partial, KrylovScalars* sc, int op, double* out);
 

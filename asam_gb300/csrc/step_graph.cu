@@ -222,7 +222,7 @@ int record_bicgstab(asam_ctx* h, const T* val, T* x, const T* b, Work<T>& w, Bod
   const long long n1 = thread_launches();
   launch_dot(h->L, d, nc, w.rt, w.r, h->partial, h->sc, OP_RHO, nullptr);
   launch_pupdate_auto(h->L, len, h->sc, w.r, w.v, w.p);
-  psolve_dev<T>(h, val, w.p, w.ph, w);
+  psolve_dev<T>(h, val, w.p, w.ph, w, true);
   launch_matvec_dot(h->L, d, nc, val, w.ph, w.v, w.rt, h->partial, h->sc, OP_ALPHA);
   launch_axpy_dot(h->L, d, nc, h->sc, SEL_ALPHA, -1.0, w.v, w.r, h->partial, OP_RNORM_HALF);
   launch_xupdate_half(h->L, len, h->sc, w.ph, x);
@@ -233,7 +233,7 @@ int record_bicgstab(asam_ctx* h, const T* val, T* x, const T* b, Work<T>& w, Bod
   if ((rc = begin_conditional(s1, s2, cudaGraphCondTypeIf, ih))) return rc;
   h->L.stream = s2;
   const long long n2 = thread_launches();
-  psolve_dev<T>(h, val, w.r, w.rh, w);
+  psolve_dev<T>(h, val, w.r, w.rh, w, true);
   launch_matvec_dot2(h->L, d, nc, val, w.rh, w.t, w.r, h->partial, h->sc, OP_STORE_A, OP_OMEGA);
   launch_axpy_dot(h->L, d, nc, h->sc, SEL_OMEGA, -1.0, w.t, w.r, h->partial, OP_RNORM_FULL);
   launch_xupdate(h->L, len, h->sc, 1, w.ph, w.rh, x);
@@ -315,8 +315,7 @@ int record_step(asam_ctx* h, double* c, double dt, BodyCounts* bc) {
     int rc;
     if (is == 0 && (rc = jac_dev(h, c, dt))) return rc;
     if ((rc = fcn_dev(h, c, h->rhs))) return rc;
-    launch_scale_host(L, len, dt, h->rhs);
-    for (int js = 0; js < is; ++js) launch_axpy_host(L, len, h->beta[is * 4 + js], h->incr + (size_t)js * len, h->rhs);
+    launch_lincomb(L, len, h->rhs, &dt, is, h->beta + is * 4, h->incr, h->rhs);
     double* x = h->incr + (size_t)is * len;
     CK(cudaMemsetAsync(x, 0, len * sizeof(double), L.stream));
     const bool refined = h->cfg.precision == ASAM_PREC_FP32_REFINED;
@@ -326,9 +325,7 @@ int record_step(asam_ctx* h, double* c, double dt, BodyCounts* bc) {
     CK(cudaMemcpyAsync(h->stage_sc + is, refined ? h->ref_sc : h->sc, sizeof(KrylovScalars),
                        cudaMemcpyDeviceToDevice, L.stream));
     launch_exchange_cell(L, d, nc, x);
-    launch_exchange_cell(L, d, nc, x);
-    CK(cudaMemcpyAsync(c, h->cold, len * sizeof(double), cudaMemcpyDeviceToDevice, L.stream));
-    for (int js = 0; js <= is; ++js) launch_axpy_host(L, len, h->alpha[is * 4 + js], h->incr + (size_t)js * len, c);
+    launch_lincomb(L, len, h->cold, nullptr, is + 1, h->alpha + is * 4, h->incr, c);
   }
   return check_launch();
 }
