@@ -41,20 +41,45 @@ __global__ void k_set_f2d(size_t len, const float* __restrict__ x, double s, dou
 }
 // out = s*base (base itself unless kScale), then out = a_j x_j + out for every
 // term: a stage's right-hand side or state in one pass over its arrays instead
-// of a copy or a scaling and a pass per term, with the same roundings
+// of a copy or a scaling and a pass per term, with the same roundings.  Bound by
+// HBM: the number of terms is a template parameter so that a thread has the
+// loads of all terms and of two elements in flight.
 struct LinTerms {
   int n;
   double a[4];
   const double* x[4];
 };
-template <bool kScale>
+template <int kN, bool kScale>
 __global__ void k_lincomb(size_t len, LinTerms t, const double* base, double s, double* out) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x) {
-    double v = kScale ? s * base[q] : base[q];
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += 2 * stride) {
+    const size_t p = q + stride;
+    const bool two = p < len;
+    double v = base[q], w = two ? base[p] : 0.0, xv[kN + 1], xw[kN + 1];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < t.n) v = t.a[j] * t.x[j][q] + v;
+    for (int j = 0; j < kN; ++j) {
+      xv[j] = t.x[j][q];
+      xw[j] = two ? t.x[j][p] : 0.0;
+    }
+    if (kScale) v = s * v, w = s * w;
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+      v = t.a[j] * xv[j] + v;
+      w = t.a[j] * xw[j] + w;
+    }
     out[q] = v;
+    if (two) out[p] = w;
+  }
+}
+template <bool kScale>
+void run_lincomb(const asam::Launch& L, size_t len, const LinTerms& t, const double* base, double s, double* out) {
+  const int g = gs_grid(L, (len + 1) / 2);
+  switch (t.n) {
+    case 0: k_lincomb<0, kScale><<<g, kBlock, 0, L.stream>>>(len, t, base, s, out); break;
+    case 1: k_lincomb<1, kScale><<<g, kBlock, 0, L.stream>>>(len, t, base, s, out); break;
+    case 2: k_lincomb<2, kScale><<<g, kBlock, 0, L.stream>>>(len, t, base, s, out); break;
+    case 3: k_lincomb<3, kScale><<<g, kBlock, 0, L.stream>>>(len, t, base, s, out); break;
+    default: k_lincomb<4, kScale><<<g, kBlock, 0, L.stream>>>(len, t, base, s, out);
   }
 }
 // slots 7 and 8 of the DIA storage: 1/diagonal (correctly rounded) and its
@@ -114,9 +139,9 @@ void launch_lincomb(const Launch& L, size_t len, const double* base, const doubl
       t.x[t.n++] = x + (size_t)j * len;
     }
   if (scale)
-    k_lincomb<true><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, t, base, *scale, out);
+    run_lincomb<true>(L, len, t, base, *scale, out);
   else
-    k_lincomb<false><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, t, base, 1.0, out);
+    run_lincomb<false>(L, len, t, base, 1.0, out);
   count_launches(1);
 }
 void launch_resid_dot(const Launch& L, const Dims& d, int ncomp, const double* val, const double* x, const double* b,

@@ -651,7 +651,7 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
 // run on the integer units, and the faces of a pressure gradient whose area is
 // not tiny skip the ratios F/(F+Eps) = 1 (pgrad_face).
 template <typename T, bool kMom, bool kDiff>
-__global__ void __launch_bounds__(256, kMom || kDiff ? 2 : 3) k_flux_plain(Dims d, GeomT<T> g, int ncomp, const T* __restrict__ gx,
+__global__ void __launch_bounds__(256, kMom || kDiff ? 2 : 4) k_flux_plain(Dims d, GeomT<T> g, int ncomp, const T* __restrict__ gx,
                                                     const T* __restrict__ gy, const T* __restrict__ gz,
                                                     T* __restrict__ f, MomSrc<T> ms, DiffSrc<T> df) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -975,6 +975,24 @@ __global__ void k_jac(Dims d, GeomT<T> g, const T* __restrict__ rho, const T* __
   }
 }
 
+// RN(x + RN(s - x)): the reference's y = -1*x + y, y = x + y around the identity
+// source block.  For x/2 <= s <= 2x the difference is exact (Sterbenz) and the
+// sum gives s back, which holds for most entries of I - dt*J times a smooth x
+// and is tested on the integer units; the two FP64 sums are left to the others.
+__device__ __forceinline__ double add_identity(double s, double x) {
+  const long long bs = __double_as_longlong(s), bx = __double_as_longlong(x);
+  if (((unsigned long long)(bs - bx + (1ll << 52)) <= (1ull << 53) &&
+       ((unsigned)(bs >> 32) & 0x7fffffffu) - (2u << 20) < (2043u << 20)) ||
+      (bs | bx) == 0)
+    return s;
+  s = (-1.0) * x + s;
+  return x + s;
+}
+__device__ __forceinline__ float add_identity(float s, float x) {
+  s = (-1.0f) * x + s;
+  return x + s;
+}
+
 // ---------------------------------------------------------------------------
 // Stage operator: MatVecMet_Vec4CellSp (MODULE/SpMatrix4CellPar_Mod.f90:70-84):
 // y = T*x (SpAVec_SpDiag, CG/MatSpDiag_Mod.f90:87-108, row sums in diagonal
@@ -996,6 +1014,7 @@ __global__ void k_matvec(Dims d, int ncomp, const TM* __restrict__ val, const T*
     const T v4 = i < NX - 1 ? (T)val[4 * n + P + 1] : (T)0;
     const T v5 = j < NY - 1 ? (T)val[5 * n + P + sy] : (T)0;
     const T v6 = k < NZ - 1 ? (T)val[6 * n + P + sz] : (T)0;
+#pragma unroll 2  // two components' loads in flight (FP32: 0.30 against 0.36 ms at 256x256x128)
     for (int ic = 0; ic < ncomp; ++ic) {
       const T* xa = x + ic * n;
       T s = (T)0;
@@ -1006,11 +1025,7 @@ __global__ void k_matvec(Dims d, int ncomp, const TM* __restrict__ val, const T*
       if (i < NX - 1) s = s + v4 * xa[P + 1];
       if (j < NY - 1) s = s + v5 * xa[P + sy];
       if (k < NZ - 1) s = s + v6 * xa[P + sz];
-      if (!plain_spmv) {
-        const T xp = xa[P];
-        s = (T)(-1) * xp + s;
-        s = xp + s;
-      }
+      if (!plain_spmv) s = add_identity(s, xa[P]);
       y[ic * n + P] = s;
     }
   }
@@ -1990,9 +2005,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_matvec_dot(Dims d, int ncomp, con
       if (i < NX - 1) s = s + v4 * xa[P + 1];
       if (j < NY - 1) s = s + v5 * xa[P + sy];
       if (k < NZ - 1) s = s + v6 * xa[P + sz];
-      const T xp = xa[P];
-      s = (T)(-1) * xp + s;
-      s = xp + s;
+      s = add_identity(s, xa[P]);
       y[ic * n + P] = s;
       if (in) {
         if (kTwo) {
@@ -2385,9 +2398,7 @@ __global__ void k_resid_dot(Dims d, int ncomp, const T* __restrict__ val, const 
       if (i < NX - 1) s = s + v4 * xa[P + 1];
       if (j < NY - 1) s = s + v5 * xa[P + sy];
       if (k < NZ - 1) s = s + v6 * xa[P + sz];
-      const T xp = xa[P];
-      s = (T)(-1) * xp + s;
-      s = xp + s;
+      s = add_identity(s, xa[P]);
       const T rv = b[ic * n + P] + (T)(-1) * s;
       r[ic * n + P] = rv;
       if (interior) acc += (double)rv * (double)rv;
