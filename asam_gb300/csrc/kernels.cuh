@@ -1072,6 +1072,10 @@ constexpr int GS_TZ = 4;
 //      three products and differences and the quotient, which runs on the
 //      integer units (fp64_int.cuh; the same bits);
 //   3. the block stores x^s.
+// A tile takes some 10 us beside its wavefront's 7, most of it the launch and
+// the first loads, so the launches of consecutive tile levels use programmatic
+// serialisation: a level's blocks start, and load the matrix and b, while the
+// level before runs.
 // A line's row pitch of kGsTx + 5 gives the 16 lines of a half-warp, each at its
 // own hyperplane offset, 16 different banks.
 constexpr int kGsTx = 16;
@@ -1102,12 +1106,16 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
   const int g0 = blockIdx.z / nsweep * group;  // this block's components: g0 .. g0+ncomp-1
   const int ncomp = min(group, ncomp_all - g0);
   const int L = tau - 2 * s;
-  if (L < 0 || L >= nlev) return;
   const int K = blockIdx.y;
   const int Jlo = max(0, L - K - (ntx - 1));
   const int J = Jlo + (int)blockIdx.x;
   const int I = L - J - K;
-  if (J >= nty || I < 0 || I >= ntx) return;  // uniform over the block
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (L < 0 || L >= nlev || J >= nty || I < 0 || I >= ntx) {  // uniform over the block
+    // a launch ends after the one before it, even without a tile
+    if (blockIdx.x + blockIdx.y + blockIdx.z == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   const int NX = d.NX(), NY = d.NY(), NZ = d.NZ();
   const size_t n = d.npad();
   const size_t sy = (size_t)NX, sz = (size_t)NX * NY;
@@ -1123,6 +1131,10 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
     const size_t P = (size_t)i + sy * (size_t)j + sz * (size_t)k;
     const int e = lb * kGsPitch + a;
     constexpr int kArr = kGsLines * kGsPitch;
+    const bool u4 = in && s > 0 && i < NX - 1, u5 = in && s > 0 && j < NY - 1, u6 = in && s > 0 && k < NZ - 1;
+    const T c4 = u4 ? (T)val[4 * n + P + 1] : (T)0;
+    const T c5 = u5 ? (T)val[5 * n + P + sy] : (T)0;
+    const T c6 = u6 ? (T)val[6 * n + P + sz] : (T)0;
     if (in) {
       // a missing neighbour: coefficient and value 0, t - 0 leaves every bit of t
       coef[e] = k > 0 ? (T)val[0 * n + P - sz] : (T)0;
@@ -1130,21 +1142,22 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
       coef[e + 2 * kArr] = i > 0 ? (T)val[2 * n + P - 1] : (T)0;
       coef[e + 3 * kArr] = (T)val[3 * n + P];
       coef[e + 4 * kArr] = reinterpret_cast<const T*>(val + (sizeof(TM) == 8 ? 8 : 7) * n)[P];
-      const bool u4 = s > 0 && i < NX - 1, u5 = s > 0 && j < NY - 1, u6 = s > 0 && k < NZ - 1;
-      const T c4 = u4 ? (T)val[4 * n + P + 1] : (T)0;
-      const T c5 = u5 ? (T)val[5 * n + P + sy] : (T)0;
-      const T c6 = u6 ? (T)val[6 * n + P + sz] : (T)0;
+      for (int ic = 0; ic < ncomp; ++ic) comp[(size_t)ic * kGsComp + e] = b[(size_t)ic * n + P];
+    }
+    // up to here only the matrix and b were read, which no sweep writes
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (in) {
       const int lz = lb / GS_TY, ly = lb % GS_TY;
 #pragma unroll 2
       for (int ic = 0; ic < ncomp; ++ic) {
         const size_t q = (size_t)ic * n + P;
         T* cs = comp + (size_t)ic * kGsComp;
-        T t = b[q];
         const T x4 = u4 ? xo[q + 1] : (T)0, x5 = u5 ? xo[q + sy] : (T)0, x6 = u6 ? xo[q + sz] : (T)0;
         T* face = cs + kArr;  // faces: below [y][x], south [z][x], west [z][y]
         if (lz == 0) face[ly * kGsTx + a] = k > 0 ? xn[q - sz] : (T)0;
         if (ly == 0) face[4 * kGsTx + lz * kGsTx + a] = j > 0 ? xn[q - sy] : (T)0;
         if (a == 0) face[8 * kGsTx + lb] = i > 0 ? xn[q - 1] : (T)0;
+        T t = cs[e];
         if (u4) t = t - gs_mul(c4, x4);
         if (u5) t = t - gs_mul(c5, x5);
         if (u6) t = t - gs_mul(c6, x6);

@@ -9,6 +9,9 @@ namespace asam {
 struct Launch {
   cudaStream_t stream;
   int sm_count;
+  // kernels of one chain may be launched with programmatic serialisation (off
+  // while the bodies of conditional graph nodes are recorded)
+  bool chain = true;
 };
 
 #define ASAM_DECLARE_LAUNCHERS(T, TM)                                                                            \

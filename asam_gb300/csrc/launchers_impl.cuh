@@ -23,6 +23,25 @@ inline int gs_grid(const asam::Launch& L, size_t n) {
   if (g < 1) g = 1;
   return (int)g;
 }
+// A kernel whose blocks may start while the kernel launched before it in the
+// stream still runs (follows: that one is of the same chain); it waits with
+// griddepcontrol.wait before it reads what that one writes.
+template <typename... P, typename... A>
+void launch_chained(const asam::Launch& L, bool follows, void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                    A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = L.stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = follows && L.chain && L.stream != nullptr ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // the gather of the face fluxes: the cells off the sides, then the others
 template <typename T, bool kMom, bool kDiff>
 void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::GeomT<T>& g, int ncomp, const T* gx,
@@ -123,8 +142,8 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
         k_gs_pipe_smem<TM, T><<<grid, threads, smem, L.stream>>>(d, ncomp, group, val, b, out, work, tau, nsweep,  \
                                                                  ntx, nty, ntz, nlev);                             \
       else                                                                                                         \
-        gs_kernel<<<grid, threads, smem, L.stream>>>(d, ncomp, group, val, b, out, work, tau, nsweep, ntx, nty,    \
-                                                            ntz, nlev);                                            \
+        launch_chained(L, tau > 0, gs_kernel, grid, threads, smem, d, ncomp, group, val, b, out, work, tau, nsweep,\
+                       ntx, nty, ntz, nlev);                                                                       \
       count_launches(1);                                                                                           \
     }                                                                                                              \
   }                                                                                                                \

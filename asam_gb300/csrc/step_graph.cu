@@ -208,6 +208,12 @@ int record_bicgstab(asam_ctx* h, const T* val, T* x, const T* b, Work<T>& w, Bod
   const int nc = h->cfg.ncomp;
   const size_t len = h->len;
   const cudaStream_t s0 = h->L.stream, s1 = h->cap_stream[0], s2 = h->cap_stream[1];
+  struct NoChain {  // ordinary launches in the bodies of conditional nodes
+    bool& chain;
+    bool was;
+    explicit NoChain(bool& c) : chain(c), was(c) { c = false; }
+    ~NoChain() { chain = was; }
+  } no_chain(h->L.chain);
   CK(cudaMemcpyAsync(w.r, b, len * sizeof(T), cudaMemcpyDeviceToDevice, s0));
   CK(cudaMemcpyAsync(w.rt, w.r, len * sizeof(T), cudaMemcpyDeviceToDevice, s0));
   launch_dot(h->L, d, nc, w.r, w.r, h->partial, h->sc, OP_RNORM0, nullptr);
