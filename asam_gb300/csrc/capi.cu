@@ -800,6 +800,8 @@ __global__ void k_probe_div(unsigned long long n, unsigned long long seed, int s
     auto same = [](double u, double v) { return __double_as_longlong(u) == __double_as_longlong(v) || (isnan(u) && isnan(v)); };
     if (!same(fpi::mul_rn(a, b), __dmul_rn(a, b))) ++cnt;
     if (!same(fpi::div_rn(a, b), __ddiv_rn(a, b))) ++cnt;
+    if (!same(fpi::quot_rn(a, b, fpi::recip(b)), __ddiv_rn(a, b))) ++cnt;
+    if (!same(fpi::quot_chain(a, b, fpi::recip(b)), __ddiv_rn(a, b))) ++cnt;
   }
   if (cnt) atomicAdd(bad, cnt);
 }

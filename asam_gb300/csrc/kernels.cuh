@@ -2266,7 +2266,7 @@ __device__ __forceinline__ void tri_tile_store(const T (*tile)[kTriPitch], T* __
   }
 }
 // the pivot with its reciprocal, quotients by it and the product off its chain
-__device__ __forceinline__ unsigned long long tri_recip(double t) { return fpi::recip(t); }
+__device__ __forceinline__ unsigned long long tri_recip(double t) { return fpi::recip_quick(t); }
 __device__ __forceinline__ double tri_quot(double x, double t, unsigned long long R) { return fpi::quot_rn(x, t, R); }
 __device__ __forceinline__ double tri_mul(double a, double b) { return fpi::mul_rn(a, b); }
 __device__ __forceinline__ unsigned long long tri_recip(float) { return 0; }

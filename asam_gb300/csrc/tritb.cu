@@ -795,7 +795,7 @@ __global__ void k_tb_coarse_cells(int n3, int n2, int n1, TbFields g, int c3, in
 //   [0..3]   adjugate of t(i): (t22, -t12), (-t21, t11)  (Div_2's numerators)
 //   [4..7]   l(i-1), the coupling to the previous row (0 in row 0)
 //   [8..11]  w(i) (0 in the last row)
-//   [12]     Det(t(i)); [13] its reciprocal for fpi::quot_rn
+//   [12]     Det(t(i)); [13] its reciprocal for fpi::quot_chain
 constexpr int kTbFac = 14;
 
 __global__ void k_tb_factor(size_t nline, int n1, const double* __restrict__ d, const double* __restrict__ u,
@@ -886,7 +886,7 @@ __device__ __forceinline__ void tb_half(int tr, int n2, int n1, const double* __
       const double v = __dsub_rn(t, __dadd_rn(__dmul_rn(l.x, c1), __dmul_rn(l.y, c2)));
       const double vo = other(v);
       const double num = __dadd_rn(__dmul_rn(ad.x, r ? vo : v), __dmul_rn(ad.y, r ? v : vo));
-      y = fpi::quot_rn(num, dr.x, (unsigned long long)__double_as_longlong(dr.y));
+      y = fpi::quot_chain(num, dr.x, (unsigned long long)__double_as_longlong(dr.y));
       if (live) xp[2 * i] = y;
       const double yo = other(y);
       c1 = r ? yo : y;
