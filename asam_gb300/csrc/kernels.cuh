@@ -1090,7 +1090,7 @@ inline size_t gs_tile_elems(int ncomp) { return (size_t)kGsCoef + (size_t)ncomp 
 __device__ __forceinline__ double gs_mul(double a, double b) { return fpi::mul_rn(a, b); }
 __device__ __forceinline__ float gs_mul(float a, float b) { return a * b; }
 __device__ __forceinline__ double gs_quot(double t, double d, double r) {
-  return fpi::quot_rn(t, d, (unsigned long long)__double_as_longlong(r));
+  return fpi::quot_chain(t, d, (unsigned long long)__double_as_longlong(r));
 }
 __device__ __forceinline__ float gs_quot(float t, float d, float r) { return div_rn(t, d, r); }
 
