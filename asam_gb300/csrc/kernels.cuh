@@ -1031,6 +1031,56 @@ __global__ void k_matvec(Dims d, int ncomp, const TM* __restrict__ val, const T*
   }
 }
 
+// The same product for FP32 and boxes of even padded width: a thread takes two
+// neighbouring cells, whose operands in the other rows and planes are aligned
+// pairs (NX even makes every row, plane and component start even).  The
+// one-cell kernel is bound by its load instructions, seven per cell and
+// component, most of them hits; here they are seven per two cells
+// (256x256x128, 10 components: 283 against 306 us).
+// The operations of a cell are those of the one-cell kernel.
+__global__ void __launch_bounds__(256) k_matvec_pairs(Dims d, int ncomp, const float* __restrict__ val,
+                                                      const float* __restrict__ x, float* __restrict__ y,
+                                                      int plain_spmv) {
+  const int NX = d.NX(), NY = d.NY(), NZ = d.NZ();
+  const size_t n = d.npad();
+  const size_t sy = (size_t)NX, sz = (size_t)NX * NY;
+  auto pair = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
+  for (size_t h = blockIdx.x * (size_t)blockDim.x + threadIdx.x; h < n / 2; h += (size_t)gridDim.x * blockDim.x) {
+    const size_t P = 2 * h;
+    int i, j, k;
+    d.ijk(P, i, j, k);
+    const bool zm = k > 0, ym = j > 0, xm = i > 0, xp = i + 1 < NX - 1, yp = j < NY - 1, zp = k < NZ - 1;
+    const float2 none = make_float2(0.f, 0.f);
+    const float2 v0 = zm ? pair(val + 0 * n + P - sz) : none;
+    const float2 v1 = ym ? pair(val + 1 * n + P - sy) : none;
+    const float v2a = xm ? val[2 * n + P - 1] : 0.f, v2b = val[2 * n + P];
+    const float2 v3 = pair(val + 3 * n + P);
+    const float v4a = val[4 * n + P + 1], v4b = xp ? val[4 * n + P + 2] : 0.f;
+    const float2 v5 = yp ? pair(val + 5 * n + P + sy) : none;
+    const float2 v6 = zp ? pair(val + 6 * n + P + sz) : none;
+#pragma unroll 2
+    for (int ic = 0; ic < ncomp; ++ic) {
+      const float* xa = x + ic * n + P;
+      const float2 c = pair(xa);
+      const float2 xzm = zm ? pair(xa - sz) : none, xym = ym ? pair(xa - sy) : none;
+      const float2 xyp = yp ? pair(xa + sy) : none, xzp = zp ? pair(xa + sz) : none;
+      const float xl = xm ? xa[-1] : 0.f, xr = xp ? xa[2] : 0.f;
+      float s = 0.f, t = 0.f;
+      if (zm) s = s + v0.x * xzm.x, t = t + v0.y * xzm.y;
+      if (ym) s = s + v1.x * xym.x, t = t + v1.y * xym.y;
+      if (xm) s = s + v2a * xl;
+      t = t + v2b * c.x;
+      s = s + v3.x * c.x, t = t + v3.y * c.y;
+      s = s + v4a * c.y;
+      if (xp) t = t + v4b * xr;
+      if (yp) s = s + v5.x * xyp.x, t = t + v5.y * xyp.y;
+      if (zp) s = s + v6.x * xzp.x, t = t + v6.y * xzp.y;
+      if (!plain_spmv) s = add_identity(s, c.x), t = add_identity(t, c.y);
+      *reinterpret_cast<float2*>(y + ic * n + P) = make_float2(s, t);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Gauss-Seidel preconditioner GaussSeidel_SpDiag (CG/MatSpDiag_Mod.f90:191-235),
 // restated as: sweep 0 solves (L+D)x=b; sweeps 1..IterG solve
@@ -1683,6 +1733,112 @@ __global__ void __launch_bounds__(32 * xl_warps<T>()) k_xline_factor(Dims d, con
   }
 }
 
+// The same recurrences on whole rows in shared memory: a CTA takes nrow
+// consecutive rows of the box with all their components, copies the three
+// coefficient rows once for all of them and the right-hand sides (cp.async,
+// lanes along x), runs one thread per (component, row) forward and back without
+// leaving shared memory, and stores the solution.  Memory bounds it: the
+// right-hand side is read and the solution written once (the chunked kernel
+// also writes and reads the forward result, and waits for a memory round trip
+// in every chunk).  Row pitch NX | 1, so that the threads of a warp, one row
+// apart, fall on different banks.  kXlU entries at a time in registers: their
+// loads do not wait behind the chain.
+constexpr int kXlBlock = 256, kXlU = 8;
+inline __host__ __device__ int xl_pitch(int NX) { return NX | 1; }
+template <typename T>
+inline size_t xl_row_bytes(int NX, int ncomp) {
+  return (size_t)(3 + ncomp) * xl_pitch(NX) * sizeof(T);
+}
+template <typename TM, typename T>
+__global__ void __launch_bounds__(kXlBlock) k_xline_rows(Dims d, int ncomp, const TM* __restrict__ val,
+                                                        const T* __restrict__ fw, const T* __restrict__ fr,
+                                                        const T* __restrict__ b, T* __restrict__ x, int nrow) {
+  extern __shared__ __align__(16) unsigned char xl_smem_raw[];
+  const int NX = d.NX(), S = xl_pitch(NX);
+  const size_t n = d.npad();
+  const int r0 = blockIdx.x * nrow, nr = min(nrow, d.NY() * d.NZ() - r0);
+  T* sa = reinterpret_cast<T*>(xl_smem_raw);  // a, 1/den, w of every row, then b (g, x) of every (component, row)
+  T* sr = sa + nrow * S;
+  T* sw = sr + nrow * S;
+  T* sb = sw + nrow * S;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  auto copy_row = [&](T* dst, const T* src, int skip) {  // src may not be read below index skip
+    for (int i = lane; i < NX; i += 32) cp_async_elem(dst + i, src + max(i, skip), i >= skip);
+  };
+  for (int t = warp; t < (2 + ncomp) * nr; t += nwarp) {
+    const int m = t / nr, q = t - m * nr;
+    const size_t P = (size_t)(r0 + q) * NX;
+    if (m == 0)
+      copy_row(sa + q * S, val + 2 * n + P - 1, 1);
+    else if (m == 1)
+      copy_row(sr + q * S, fr + P, 0);
+    else
+      copy_row(sb + ((m - 2) * nrow + q) * S, b + (size_t)(m - 2) * n + P, 0);
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  for (int q = warp; q < nr; q += nwarp) copy_row(sw + q * S, fw + (size_t)(r0 + q) * NX, 0);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  __syncthreads();
+  const int ch = threadIdx.x, q = ch % nrow;
+  const bool solves = ch < ncomp * nrow && q < nr;
+  T* g = sb + ch * S;
+  if (solves) {
+    const T *a = sa + q * S, *r = sr + q * S;
+    T prev = (T)0;
+    int k = 0;
+    for (; k + kXlU <= NX; k += kXlU) {
+      T av[kXlU], rv[kXlU], bv[kXlU];
+#pragma unroll
+      for (int u = 0; u < kXlU; ++u) {
+        av[u] = a[k + u];
+        rv[u] = r[k + u];
+        bv[u] = g[k + u];
+      }
+#pragma unroll
+      for (int u = 0; u < kXlU; ++u) {
+        prev = (bv[u] - av[u] * prev) * rv[u];
+        g[k + u] = prev;
+      }
+    }
+    for (; k < NX; ++k) {
+      prev = (g[k] - a[k] * prev) * r[k];
+      g[k] = prev;
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  if (solves) {
+    const T* w = sw + q * S;
+    T next = g[NX - 1];
+    int k = NX - 2;
+    for (; k - kXlU + 1 >= 0; k -= kXlU) {
+      T wv[kXlU], gv[kXlU];
+#pragma unroll
+      for (int u = 0; u < kXlU; ++u) {
+        wv[u] = w[k - u];
+        gv[u] = g[k - u];
+      }
+#pragma unroll
+      for (int u = 0; u < kXlU; ++u) {
+        next = gv[u] - wv[u] * next;
+        g[k - u] = next;
+      }
+    }
+    for (; k >= 0; --k) {
+      next = g[k] - w[k] * next;
+      g[k] = next;
+    }
+  }
+  __syncthreads();
+  for (int t = warp; t < ncomp * nr; t += nwarp) {
+    const int m = t / nr, qq = t - m * nr;
+    const T* src = sb + (m * nrow + qq) * S;
+    T* dst = x + (size_t)m * n + (size_t)(r0 + qq) * NX;
+    for (int i = lane; i < NX; i += 32) dst[i] = src[i];
+  }
+}
+
 template <typename TM, typename T>
 __global__ void __launch_bounds__(32 * xl_warps<T>()) k_xline_solve(Dims d, int ncomp, const TM* __restrict__ val,
                                                                    const T* __restrict__ fw,
@@ -1743,25 +1899,41 @@ __global__ void __launch_bounds__(32 * xl_warps<T>()) k_xline_solve(Dims d, int 
   }
 }
 
-// zero the whole halo layer (PSolveSp, MODULE/Vector4Cell_Mod.f90:732-737)
+// zero the whole halo layer (PSolveSp, MODULE/Vector4Cell_Mod.f90:732-737):
+// one thread per halo cell (the two z planes, the two y walls between them,
+// the ends of the other rows), one component per blockIdx.y.  Bound by its
+// single-sector stores (256x256x128, 3 FP32 components: 3.9 us; 31 when looked
+// for among all cells).
+inline size_t halo_cells(const asam::Dims& d) {
+  return 2 * ((size_t)d.NX() * d.NY() + (size_t)d.NX() * d.nz + (size_t)d.ny * d.nz);
+}
 template <typename T>
-__global__ void k_zero_halo(Dims d, int ncomp, T* __restrict__ x) {
-  const int NX = d.NX(), NY = d.NY(), NZ = d.NZ();
-  const size_t n = d.npad();
-  for (size_t P = blockIdx.x * (size_t)blockDim.x + threadIdx.x; P < n; P += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(P % NX);
-    const int j = (int)((P / NX) % NY);
-    const int k = (int)(P / ((size_t)NX * NY));
-    if (i == 0 || i == NX - 1 || j == 0 || j == NY - 1 || k == 0 || k == NZ - 1)
-      for (int ic = 0; ic < ncomp; ++ic) x[ic * n + P] = (T)0;
+__global__ void k_zero_halo(Dims d, unsigned tot, T* __restrict__ x) {
+  const unsigned NX = d.NX(), NY = d.NY(), nzp = 2 * NX * NY, nyw = 2 * NX * d.nz;
+  const size_t sy = NX, sz = (size_t)NX * NY;
+  T* a = x + (size_t)blockIdx.y * d.npad();
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x) {
+    size_t P;
+    if (q < nzp) {
+      P = q < NX * NY ? q : (size_t)(d.nz) * sz + q;  // the planes k = 0 and nz + 1
+    } else if (q - nzp < nyw) {
+      const unsigned r = q - nzp, row = r / NX, i = r - row * NX, k = row / 2 + 1;
+      P = i + (row & 1 ? sy * (NY - 1) : 0) + sz * k;
+    } else {
+      const unsigned r = q - nzp - nyw, row = r / 2, k = row / d.ny + 1, j = row % d.ny + 1;
+      P = (r & 1 ? NX - 1 : 0) + sy * j + sz * k;
+    }
+    a[P] = (T)0;
   }
 }
 
-// periodic halo fill (ExchangeCell of a single periodic block)
+// periodic halo fill (ExchangeCell of a single periodic block), one component
+// per blockIdx.y: the two copies of a thread are all that it waits for (10
+// FP32 components at 128x112x72: 4.0 us, 10.0 with a loop over the components)
 template <typename T>
-__global__ void k_exchange_cell(Dims d, int ncomp, T* __restrict__ c) {
+__global__ void k_exchange_cell(Dims d, T* __restrict__ c) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const size_t n = d.npad();
+  T* a = c + (size_t)blockIdx.y * d.npad();
   const size_t nxf = d.per_x ? (size_t)ny * nz : 0;
   const size_t nyf = d.per_y ? (size_t)nx * nz : 0;
   const size_t nzf = d.per_z ? (size_t)nx * ny : 0;
@@ -1780,11 +1952,8 @@ __global__ void k_exchange_cell(Dims d, int ncomp, T* __restrict__ c) {
       int i = (int)(r % nx) + 1, j = (int)(r / nx) + 1;
       lo = d.P(i, j, 0); lo_src = d.P(i, j, nz); hi = d.P(i, j, nz + 1); hi_src = d.P(i, j, 1);
     }
-    for (int ic = 0; ic < ncomp; ++ic) {
-      T* a = c + ic * n;
-      a[lo] = a[lo_src];
-      a[hi] = a[hi_src];
-    }
+    a[lo] = a[lo_src];
+    a[hi] = a[hi_src];
   }
 }
 
@@ -1948,7 +2117,8 @@ __device__ __forceinline__ double block_sum(double v, double* ws) {
 
 // One warp per interior x-row of one component at a time (lanes along x, so
 // every load is coalesced and no per-element index division is needed).
-template <typename T>
+// kTwo: (y, y) as well, in the second half of partial, from the same pass.
+template <typename T, bool kTwo>
 __global__ void k_dot_partial(Dims d, int ncomp, const T* __restrict__ x, const T* __restrict__ y,
                               double* __restrict__ partial) {
   const int nx = d.nx, ny = d.ny;
@@ -1958,7 +2128,7 @@ __global__ void k_dot_partial(Dims d, int ncomp, const T* __restrict__ x, const 
   const size_t sy = (size_t)d.NX(), sz = (size_t)d.NX() * d.NY();
   const int lane = threadIdx.x & 31;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  DotAcc<T> acc;
+  DotAcc<T> acc, acc2;
   for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < nrow; r += nw) {
     const int ic = (int)(r / rows_c);
     const int jk = (int)(r - ic * rows_c);
@@ -1971,15 +2141,26 @@ __global__ void k_dot_partial(Dims d, int ncomp, const T* __restrict__ x, const 
       const T x0 = xr[i], x1 = xr[i + 32], x2 = xr[i + 64], x3 = xr[i + 96];
       const T y0 = yr[i], y1 = yr[i + 32], y2 = yr[i + 64], y3 = yr[i + 96];
       acc.add(x0, y0);
+      if constexpr (kTwo) acc2.add(y0, y0);
       acc.add(x1, y1);
+      if constexpr (kTwo) acc2.add(y1, y1);
       acc.add(x2, y2);
+      if constexpr (kTwo) acc2.add(y2, y2);
       acc.add(x3, y3);
+      if constexpr (kTwo) acc2.add(y3, y3);
     }
-    for (; i < nx; i += 32) acc.add(xr[i], yr[i]);
+    for (; i < nx; i += 32) {
+      acc.add(xr[i], yr[i]);
+      if constexpr (kTwo) acc2.add(yr[i], yr[i]);
+    }
   }
   __shared__ double ws[RED_BLOCK / 32];
   const double t = block_sum(acc.value(), ws);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  if constexpr (kTwo) {
+    const double t2 = block_sum(acc2.value(), ws);
+    if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = t2;
+  }
 }
 
 // SpMV fused with the dot products that read its result (BiCGStab's
@@ -2108,6 +2289,7 @@ template <typename T>
 __global__ void __launch_bounds__(RED_BLOCK) k_axpy_dot(Dims d, int ncomp, const asam::KrylovScalars* sc, int sel,
                                                         double sign, const T* __restrict__ x, T* __restrict__ y,
                                                         double* __restrict__ partial) {
+  constexpr int kU = 4;  // cells a lane whose loads are in flight together
   const T a = (T)(sign * pick(sc, sel));
   const int NX = d.NX(), NY = d.NY();
   const long long rows_c = (long long)NY * d.NZ();
@@ -2122,13 +2304,24 @@ __global__ void __launch_bounds__(RED_BLOCK) k_axpy_dot(Dims d, int ncomp, const
     const int j = (int)(jk % NY), k = (int)(jk / NY);
     const bool row_in = j >= 1 && j <= d.ny && k >= 1 && k <= d.nz;
     const size_t base = (size_t)ic * n + (size_t)jk * NX;
-    for (int i = lane; i < NX; i += 32) {
-      T v = y[base + i];
-      if (a != (T)0) {
-        v = a * x[base + i] + v;
-        y[base + i] = v;
+    for (int i0 = lane; i0 < NX; i0 += 32 * kU) {
+      T v[kU], xv[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int i = min(i0 + 32 * u, NX - 1);
+        v[u] = y[base + i];
+        xv[u] = a != (T)0 ? x[base + i] : (T)0;
       }
-      if (row_in && i >= 1 && i <= d.nx) acc.add(v, v);
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int i = i0 + 32 * u;
+        if (i >= NX) break;
+        if (a != (T)0) {
+          v[u] = a * xv[u] + v[u];
+          y[base + i] = v[u];
+        }
+        if (row_in && i >= 1 && i <= d.nx) acc.add(v[u], v[u]);
+      }
     }
   }
   __shared__ double ws[RED_BLOCK / 32];

@@ -23,6 +23,32 @@ inline int gs_grid(const asam::Launch& L, size_t n) {
   if (g < 1) g = 1;
   return (int)g;
 }
+// The FP32 vectors and matrix are the context's own allocations, so an even
+// padded width alone makes every pair aligned; FP64 vectors may be the caller's.
+template <typename TM, typename T>
+void run_matvec(const asam::Launch& L, const asam::Dims& d, int ncomp, const TM* val, const T* x, T* y, int plain) {
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (d.NX() % 2 == 0) {
+      k_matvec_pairs<<<gs_grid(L, d.npad() / 2), kBlock, 0, L.stream>>>(d, ncomp, val, x, y, plain);
+      return;
+    }
+  }
+  k_matvec<TM, T><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, ncomp, val, x, y, plain);
+}
+// Rows per CTA of k_xline_rows: as many as fill one warp with recurrences (a
+// step of a warp costs the same for 10 threads as for 32; 256x256x128 with 10
+// components: 204 us at 3 rows, 228 at 4, 224 at 2), within the shared memory
+// of four CTAs per SM (512x128x64: 138 us at 2 rows, 159 at 4) and leaving two
+// CTAs for every SM (61x47x33: 7.6 against 14.7 us).  0 where one row with all
+// its components does not fit: the chunked k_xline_solve.
+constexpr int kXlSmemMax = 227 * 1024, kXlSmemAim = 55 * 1024;
+template <typename T>
+inline int xl_rows(const asam::Launch& L, const asam::Dims& d, int ncomp) {
+  const size_t row = xl_row_bytes<T>(d.NX(), ncomp);
+  if (row > kXlSmemMax) return 0;
+  const int r = std::min((int)(kXlSmemAim / row), 32 / ncomp);
+  return std::max(1, std::min(r, d.NY() * d.NZ() / (2 * L.sm_count)));
+}
 // A kernel whose blocks may start while the kernel launched before it in the
 // stream still runs (follows: that one is of the same chain); it waits with
 // griddepcontrol.wait before it reads what that one writes.
@@ -103,7 +129,7 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
     count_launches(1);                                                                                             \
   }                                                                                                                \
   void launch_matvec(const Launch& L, const Dims& d, int ncomp, const TM* val, const T* x, T* y, int plain) {      \
-    k_matvec<TM, T><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, ncomp, val, x, y, plain);                    \
+    run_matvec<TM, T>(L, d, ncomp, val, x, y, plain);                                                              \
     count_launches(1);                                                                                             \
   }                                                                                                                \
   void launch_gs_sweeps(const Launch& L, const Dims& d, int ncomp, const TM* val, const T* b, T* out, T* work,     \
@@ -174,10 +200,17 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
   void launch_line_psolve(const Launch& L, const Dims& d, int ncomp, const TM* val, const T* b, T* x, T* w,       \
                           int axis, const T* fw, const T* fr) {                                                    \
     if (axis == 0) {                                                                                               \
-      const int wpb = xl_warps<T>();                                                                               \
-      const long long tasks = (long long)((d.NY() * d.NZ() + 31) / 32) * ncomp;                                   \
-      k_xline_solve<TM, T><<<(unsigned)((tasks + wpb - 1) / wpb), 32 * wpb, 0, L.stream>>>(d, ncomp, val, fw, fr,  \
-                                                                                             b, x);                \
+      const int nrow = xl_rows<T>(L, d, ncomp);                                                                    \
+      if (nrow > 0) {                                                                                              \
+        cudaFuncSetAttribute(k_xline_rows<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXlSmemMax);        \
+        k_xline_rows<TM, T><<<(d.NY() * d.NZ() + nrow - 1) / nrow, kXlBlock, nrow * xl_row_bytes<T>(d.NX(), ncomp),\
+                              L.stream>>>(d, ncomp, val, fw, fr, b, x, nrow);                                      \
+      } else {                                                                                                     \
+        const int wpb = xl_warps<T>();                                                                             \
+        const long long tasks = (long long)((d.NY() * d.NZ() + 31) / 32) * ncomp;                                  \
+        k_xline_solve<TM, T><<<(unsigned)((tasks + wpb - 1) / wpb), 32 * wpb, 0, L.stream>>>(d, ncomp, val, fw,    \
+                                                                                             fr, b, x);            \
+      }                                                                                                            \
     } else {                                                                                                       \
       const size_t ncols = (size_t)d.NX() * (axis == 2 ? d.NY() : d.NZ());                                         \
       k_line_psolve<TM, T><<<(unsigned)((ncols + 127) / 128), 128, 0, L.stream>>>(d, ncomp, axis, val, b, x, w);   \
@@ -191,13 +224,15 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
     count_launches(1);                                                                                             \
   }                                                                                                                \
   void launch_zero_halo(const Launch& L, const Dims& d, int ncomp, T* x) {                                         \
-    k_zero_halo<T><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, ncomp, x); count_launches(1);                                    \
+    const size_t tot = halo_cells(d);                                                                              \
+    k_zero_halo<T><<<dim3(gs_grid(L, tot), ncomp), kBlock, 0, L.stream>>>(d, (unsigned)tot, x);                    \
+    count_launches(1);                                                                                             \
   }                                                                                                                \
   void launch_exchange_cell(const Launch& L, const Dims& d, int ncomp, T* c) {                                     \
     size_t tot = (d.per_x ? (size_t)d.ny * d.nz : 0) + (d.per_y ? (size_t)d.nx * d.nz : 0) +                       \
                  (d.per_z ? (size_t)d.nx * d.ny : 0);                                                              \
     if (tot == 0) return;                                                                                          \
-    k_exchange_cell<T><<<gs_grid(L, tot), kBlock, 0, L.stream>>>(d, ncomp, c); count_launches(1);                                     \
+    k_exchange_cell<T><<<dim3(gs_grid(L, tot), ncomp), kBlock, 0, L.stream>>>(d, c); count_launches(1);            \
   }                                                                                                                \
   void launch_bound_cond(const Launch& L, const Dims& d, int ncomp, int comp0, const BcKinds& bc, T* c) {        \
     size_t tot = (d.per_x ? 0 : (size_t)d.ny * d.nz) + (d.per_y ? 0 : (size_t)d.nx * d.nz) +                       \
@@ -210,7 +245,7 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
   }                                                                                                                \
   void launch_dot(const Launch& L, const Dims& d, int ncomp, const T* x, const T* y, double* partial,              \
                   KrylovScalars* sc, int op, double* out) {                                                        \
-    k_dot_partial<T><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, x, y, partial); count_launches(1);                               \
+    k_dot_partial<T, false><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, x, y, partial); count_launches(1);                               \
     k_dot_final<<<1, RED_BLOCK, 0, L.stream>>>(partial, RED_GRID, sc, op, out); count_launches(1);                                    \
   }                                                                                                                \
   void launch_axpy_sc(const Launch& L, size_t len, const KrylovScalars* sc, int sel, double sign, const T* x,       \
@@ -234,8 +269,10 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
                           double* partial, KrylovScalars* sc, int op1, int op2) {                                  \
     if (sizeof(T) == sizeof(float)) {                                                                              \
       launch_matvec(L, d, ncomp, val, x, y, 0);                                                                    \
-      launch_dot(L, d, ncomp, y, a, partial, sc, op1, nullptr);                                                    \
-      launch_dot(L, d, ncomp, y, y, partial, sc, op2, nullptr);                                                    \
+      k_dot_partial<T, true><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, a, y, partial);                       \
+      k_dot_final<<<1, RED_BLOCK, 0, L.stream>>>(partial, RED_GRID, sc, op1, nullptr);                             \
+      k_dot_final<<<1, RED_BLOCK, 0, L.stream>>>(partial + RED_GRID, RED_GRID, sc, op2, nullptr);                  \
+      count_launches(3);                                                                                           \
       return;                                                                                                      \
     }                                                                                                              \
     const int g = fused_grid(L, d.npad());                                                                         \
