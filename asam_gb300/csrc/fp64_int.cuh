@@ -182,4 +182,16 @@ __device__ __forceinline__ double quot_rn(double x, double d, u64 R) {
 }
 __device__ __forceinline__ double div_rn(double x, double d) { return quot_rn(x, d, recip_quick(d)); }
 
+// A double whose products and quotients run on the integer units and whose
+// sums on the FP64 unit, for expressions that are written out as the reference
+// writes them.
+struct Num {
+  double v;
+  __device__ __forceinline__ Num(double x) : v(x) {}
+  friend __device__ __forceinline__ Num operator*(Num a, Num b) { return mul_rn(a.v, b.v); }
+  friend __device__ __forceinline__ Num operator/(Num a, Num b) { return div_rn(a.v, b.v); }
+  friend __device__ __forceinline__ Num operator+(Num a, Num b) { return __dadd_rn(a.v, b.v); }
+  friend __device__ __forceinline__ Num operator-(Num a, Num b) { return __dsub_rn(a.v, b.v); }
+};
+
 }  // namespace fpi
