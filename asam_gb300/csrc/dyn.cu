@@ -116,23 +116,26 @@ __global__ void k_shift_bound(Dims d, GeomT<double> g, Pos6 pos, const int* __re
 // VelCellToFaceComputeLR (ADVECT/VelocityCellFace_Mod.f90:1692-1722 interior,
 // the 'iw'/'pw' neighbour branches :1384-1689 for periodic sides, and the
 // outer-wall branches :1723-1892): one thread per face of uF, vF, wF.
+// Its quotients and products (four and five a face) run on the integer units
+// (256x256x64: 0.44 instead of 1.05 ms).
 __global__ void k_cell_to_face(Dims d, GeomT<double> g, Pos6 pos, BcKinds bc, const double* __restrict__ c,
                                double* __restrict__ uf, double* __restrict__ vf, double* __restrict__ wf) {
+  using fpi::Num;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const size_t n = d.npad();
   const size_t nu = d.n_uf(), nv = d.n_vf(), nw = d.n_wf();
-  const double e = kEps;
+  const fpi::Num e = kEps;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nu + nv + nw;
        q += (size_t)gridDim.x * blockDim.x) {
     if (q < nu) {
       const int i = (int)(q % (nx + 1)), j = (int)((q / (nx + 1)) % ny) + 1, k = (int)(q / ((size_t)(nx + 1) * ny)) + 1;
       double val;
       if ((i >= 1 && i <= nx - 1) || d.per_x) {
-        const double F = g.fu[d.FU(i, j, k)];
-        const double VR = g.volc[d.P(i + 1, j, k)] * F / (F + g.fu[d.FU(i + 1, j, k)] + e);
-        const double VL = g.volc[d.P(i, j, k)] * F / (F + g.fu[d.FU(i - 1, j, k)] + e);
-        val = (VR * c[pos.p[0] * n + d.P(i + 1, j, k)] + VL * c[pos.p[1] * n + d.P(i, j, k)]) / (VL + VR + e) * F /
-              (F + e);
+        const Num F = g.fu[d.FU(i, j, k)];
+        const Num VR = Num(g.volc[d.P(i + 1, j, k)]) * F / (F + g.fu[d.FU(i + 1, j, k)] + e);
+        const Num VL = Num(g.volc[d.P(i, j, k)]) * F / (F + g.fu[d.FU(i - 1, j, k)] + e);
+        val = ((VR * c[pos.p[0] * n + d.P(i + 1, j, k)] + VL * c[pos.p[1] * n + d.P(i, j, k)]) / (VL + VR + e) * F /
+               (F + e)).v;
       } else if (i == 0) {
         val = bc.k[pos.p[0]][0] == kBcZeroGrad ? c[pos.p[0] * n + d.P(1, j, k)] : 0.0;
       } else {
@@ -144,11 +147,11 @@ __global__ void k_cell_to_face(Dims d, GeomT<double> g, Pos6 pos, BcKinds bc, co
       const int i = (int)(r % nx) + 1, j = (int)((r / nx) % (ny + 1)), k = (int)(r / ((size_t)nx * (ny + 1))) + 1;
       double val;
       if ((j >= 1 && j <= ny - 1) || d.per_y) {
-        const double F = g.fv[d.FV(i, j, k)];
-        const double VR = g.volc[d.P(i, j + 1, k)] * F / (F + g.fv[d.FV(i, j + 1, k)] + e);
-        const double VL = g.volc[d.P(i, j, k)] * F / (F + g.fv[d.FV(i, j - 1, k)] + e);
-        val = (VR * c[pos.p[2] * n + d.P(i, j + 1, k)] + VL * c[pos.p[3] * n + d.P(i, j, k)]) / (VL + VR + e) * F /
-              (F + e);
+        const Num F = g.fv[d.FV(i, j, k)];
+        const Num VR = Num(g.volc[d.P(i, j + 1, k)]) * F / (F + g.fv[d.FV(i, j + 1, k)] + e);
+        const Num VL = Num(g.volc[d.P(i, j, k)]) * F / (F + g.fv[d.FV(i, j - 1, k)] + e);
+        val = ((VR * c[pos.p[2] * n + d.P(i, j + 1, k)] + VL * c[pos.p[3] * n + d.P(i, j, k)]) / (VL + VR + e) * F /
+               (F + e)).v;
       } else if (j == 0) {
         val = bc.k[pos.p[2]][2] == kBcZeroGrad ? c[pos.p[2] * n + d.P(i, 1, k)] : 0.0;
       } else {
@@ -160,11 +163,11 @@ __global__ void k_cell_to_face(Dims d, GeomT<double> g, Pos6 pos, BcKinds bc, co
       const int i = (int)(r % nx) + 1, j = (int)((r / nx) % ny) + 1, k = (int)(r / ((size_t)nx * ny));
       double val;
       if ((k >= 1 && k <= nz - 1) || d.per_z) {
-        const double F = g.fw[d.FW(i, j, k)];
-        const double VR = g.volc[d.P(i, j, k + 1)] * F / (F + g.fw[d.FW(i, j, k + 1)] + e);
-        const double VL = g.volc[d.P(i, j, k)] * F / (F + g.fw[d.FW(i, j, k - 1)] + e);
-        val = (VR * c[pos.p[4] * n + d.P(i, j, k + 1)] + VL * c[pos.p[5] * n + d.P(i, j, k)]) / (VL + VR + e) * F /
-              (F + e);
+        const Num F = g.fw[d.FW(i, j, k)];
+        const Num VR = Num(g.volc[d.P(i, j, k + 1)]) * F / (F + g.fw[d.FW(i, j, k + 1)] + e);
+        const Num VL = Num(g.volc[d.P(i, j, k)]) * F / (F + g.fw[d.FW(i, j, k - 1)] + e);
+        val = ((VR * c[pos.p[4] * n + d.P(i, j, k + 1)] + VL * c[pos.p[5] * n + d.P(i, j, k)]) / (VL + VR + e) * F /
+               (F + e)).v;
       } else if (k == 0) {
         val = bc.k[pos.p[4]][4] == kBcZeroGrad ? c[pos.p[4] * n + d.P(i, j, 1)] : 0.0;
       } else {
@@ -181,20 +184,21 @@ __global__ void k_cell_to_face(Dims d, GeomT<double> g, Pos6 pos, BcKinds bc, co
 __global__ void k_thermo(size_t n, const double* __restrict__ rho, const double* __restrict__ th,
                          const double* __restrict__ rv, const double* __restrict__ rc, const double* __restrict__ rr,
                          const double* __restrict__ ri, double* __restrict__ t, double* __restrict__ p) {
-  const double e = kEps;
+  using fpi::Num;
+  const Num e = kEps;
   for (size_t P = blockIdx.x * (size_t)blockDim.x + threadIdx.x; P < n; P += (size_t)gridDim.x * blockDim.x) {
     const double RhoLoc = rho[P];
     const double RhoVLoc = rv ? rv[P] : 0.0;
     const double rl = rc ? rc[P] : 0.0, rrr = rr ? rr[P] : 0.0;
     const double RhoLLoc = rl + rrr;
     const double RhoILoc = ri ? ri[P] : 0.0;
-    const double RhoDLoc = RhoLoc - RhoVLoc - RhoLLoc - RhoILoc + e;
-    const double Rm = kRd * RhoDLoc + kRv * RhoVLoc + e;
-    const double Cpml = kCpd * RhoDLoc + kCpv * RhoVLoc + kCpl * RhoLLoc + kCpi * RhoILoc + e;
-    const double KappaLoc = Rm / Cpml;
-    const double T = pow(kRd * th[P] / pow(kP0, KappaLoc), 1.0 / (1.0 - KappaLoc)) / Rm + e;
-    t[P] = T;
-    p[P] = (kRd * (RhoLoc - rl - rrr) + (kRv - kRd) * RhoVLoc) * T;
+    const Num RhoDLoc = RhoLoc - RhoVLoc - RhoLLoc - RhoILoc + e;
+    const Num Rm = kRd * RhoDLoc + Num(kRv) * RhoVLoc + e;
+    const Num Cpml = kCpd * RhoDLoc + Num(kCpv) * RhoVLoc + Num(kCpl) * RhoLLoc + Num(kCpi) * RhoILoc + e;
+    const double KappaLoc = (Rm / Cpml).v;
+    const Num T = pow((Num(kRd) * th[P] / pow(kP0, KappaLoc)).v, fpi::div_rn(1.0, 1.0 - KappaLoc)) / Rm + e;
+    t[P] = T.v;
+    p[P] = ((Num(kRd) * (RhoLoc - rl - rrr) + Num(kRv - kRd) * RhoVLoc) * T).v;
   }
 }
 

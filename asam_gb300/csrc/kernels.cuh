@@ -38,20 +38,6 @@ __device__ __forceinline__ float div_rn(float x, float d, float rinv) {
   return __fmaf_rn(e, rinv, q0);
 }
 
-// ---------------------------------------------------------------------------
-// Limiter and stencil coefficients: ADVECT/Advection_Mod.f90:2118-2134
-// (k1F, k2F, PhiLim with MethAdv='Koren').
-// ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T k1f(T hL, T hC, T hR) {
-  const T e = eps_t<T>();
-  return (hC / (hC + hR + e)) * ((hL + hC) / (hL + hC + hR + e));
-}
-template <typename T>
-__device__ __forceinline__ T k2f(T hL, T hC, T hR) {
-  const T e = eps_t<T>();
-  return (hC / (hL + hC + e)) * (hR / (hL + hC + hR + e));
-}
 // a < b on the integer units (a comparison is an FP64 instruction of 64 cycles
 // as well): false for a quiet NaN a, as in 0/0 at a slope of -Eps; b a number
 __device__ __forceinline__ bool less(double a, double b) {
@@ -68,14 +54,6 @@ __device__ __forceinline__ bool negative(double a) {
 }
 __device__ __forceinline__ bool positive(float a) { return a > 0.0f; }
 __device__ __forceinline__ bool negative(float a) { return a < 0.0f; }
-
-template <typename T>
-__device__ __forceinline__ T koren(T r, T k1, T k2) {
-  T a = k1 * r + k2;
-  T m = less(a, (T)1) ? a : (T)1;
-  m = less(r, m) ? r : m;
-  return negative(m) ? (T)0 : m;
-}
 
 // RN(x + Eps): from |x| = 2^-45 on Eps is less than half a unit in the last
 // place (of the next smaller number, too), so the sum is x
@@ -95,6 +73,26 @@ __device__ __forceinline__ unsigned long long recip_i(double d) { return fpi::re
 __device__ __forceinline__ float recip_i(float d) { return 1.0f / d; }
 __device__ __forceinline__ double quot_i(double x, double d, unsigned long long R) { return fpi::quot_rn(x, d, R); }
 __device__ __forceinline__ float quot_i(float x, float d, float r) { return div_rn(x, d, r); }
+
+// ---------------------------------------------------------------------------
+// Limiter and stencil coefficients: ADVECT/Advection_Mod.f90:2118-2134
+// (k1F, k2F, PhiLim with MethAdv='Koren').
+// ---------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ T k1f(T hL, T hC, T hR) {
+  return mul_i(div_i(hC, add_eps(hC + hR)), div_i(hL + hC, add_eps(hL + hC + hR)));
+}
+template <typename T>
+__device__ __forceinline__ T k2f(T hL, T hC, T hR) {
+  return mul_i(div_i(hC, add_eps(hL + hC)), div_i(hR, add_eps(hL + hC + hR)));
+}
+template <typename T>
+__device__ __forceinline__ T koren(T r, T k1, T k2) {
+  T a = k1 * r + k2;
+  T m = less(a, (T)1) ? a : (T)1;
+  m = less(r, m) ? r : m;
+  return negative(m) ? (T)0 : m;
+}
 
 using asam::GeomT;
 
@@ -120,6 +118,8 @@ __global__ void k_phi(Dims d, int ncomp, int rho_pos, const T* __restrict__ c, T
 //             - upwind cell right of it, 0 no flux in the reference's loop)
 //   coef[1] = F_other/(F_other+Eps), coef[2] = k1, coef[3] = k2 of the upwind cell
 //   mask bits: 1 VL<VC, 2 VR<VC (x only), 4 FL<FR, 8 FR<FL (blends of :868-871)
+// FP64: five quotients, the products and the comparisons on the integer units
+// (an axis of 256x256x64: 244 instead of 443 us).
 // with the upwind cell's VL, VC, VR, FL, FR as in ADVECT/Advection_Mod.f90:854-974.
 template <typename T, int AXIS>
 __global__ void k_face_coef(Dims d, GeomT<T> g, T* __restrict__ coef, unsigned char* __restrict__ mask) {
@@ -128,7 +128,6 @@ __global__ void k_face_coef(Dims d, GeomT<T> g, T* __restrict__ coef, unsigned c
   const int ey = AXIS == 1 ? ny + 1 : ny;
   const int ez = AXIS == 2 ? nz + 1 : nz;
   const size_t nface = (size_t)ex * ey * ez;
-  const T e = eps_t<T>();
   const T half = (T)0.5;
   for (size_t f = blockIdx.x * (size_t)blockDim.x + threadIdx.x; f < nface; f += (size_t)gridDim.x * blockDim.x) {
     const int a = (int)(f % ex);
@@ -150,8 +149,8 @@ __global__ void k_face_coef(Dims d, GeomT<T> g, T* __restrict__ coef, unsigned c
     const int s = AXIS == 0 ? i : (AXIS == 1 ? j : k);
     const int smax = AXIS == 0 ? nx : (AXIS == 1 ? ny : nz);
     int orient = 0;
-    if (vel > (T)0 && s >= 1) orient = 1;           // upwind = left cell, its right face
-    else if (vel < (T)0 && s + 1 <= smax) orient = -1;  // upwind = right cell, its left face
+    if (positive(vel) && s >= 1) orient = 1;           // upwind = left cell, its right face
+    else if (negative(vel) && s + 1 <= smax) orient = -1;  // upwind = right cell, its left face
     T c0 = (T)0, c1 = (T)0, c2 = (T)0, c3 = (T)0;
     unsigned char m = 0;
     if (orient != 0) {
@@ -172,20 +171,20 @@ __global__ void k_face_coef(Dims d, GeomT<T> g, T* __restrict__ coef, unsigned c
       }
       const T VL = g.volc[PC - stride], VC = g.volc[PC], VR = g.volc[PC + stride];
       if (orient > 0) {
-        c0 = half * (fabs(vel) + vel) * FR;
-        c1 = FL / (FL + e);
+        c0 = mul_i(mul_i(half, fabs(vel) + vel), FR);
+        c1 = div_i(FL, add_eps(FL));
         c2 = k1f(VL, VC, VR);
         c3 = k2f(VL, VC, VR);
       } else {
-        c0 = -(half * (fabs(vel) - vel) * FL);
-        c1 = FR / (FR + e);
+        c0 = -mul_i(mul_i(half, fabs(vel) - vel), FL);
+        c1 = div_i(FR, add_eps(FR));
         c2 = k1f(VR, VC, VL);
         c3 = k2f(VR, VC, VL);
       }
-      if (AXIS == 0 && VL < VC) m |= 1;
-      if (AXIS == 0 && VR < VC) m |= 2;
-      if (FL < FR) m |= 4;
-      if (FR < FL) m |= 8;
+      if (AXIS == 0 && less(VL, VC)) m |= 1;
+      if (AXIS == 0 && less(VR, VC)) m |= 2;
+      if (less(FL, FR)) m |= 4;
+      if (less(FR, FL)) m |= 8;
     }
     coef[0 * nface + f] = c0;
     coef[1 * nface + f] = c1;
@@ -825,14 +824,21 @@ __global__ void k_div(Dims d, GeomT<T> g, T* __restrict__ rhs) {
 // cell computing its column of the 7-diagonal matrix in the reference's
 // accumulation order.
 // ---------------------------------------------------------------------------
-// Half*(ABS(u)+/-u)*F/V/(Rho+Eps), both divisions correctly rounded from the
-// precomputed reciprocals of V (= VolC+Eps of that cell: rvol) and of
-// Rho+Eps (one per column), so the result is the reference's expression
-template <typename T>
-__device__ __forceinline__ T jac_term(T vel, bool plus, T F, T Vden, T rVden, T rhoe, T rrhoe) {
-  const T half = (T)0.5;
-  T s = plus ? (fabs(vel) + vel) : (fabs(vel) - vel);
-  return div_rn(div_rn(half * s * F, Vden, rVden), rhoe, rrhoe);
+// Half*(ABS(u)+/-u)*F/V/(Rho+Eps).  Half*(ABS(u)+/-u) is |u| for one sign of u
+// and 0 for the other, where the term is 0; the product and both quotients (one
+// by a divisor of the whole column) run on the integer units.  All of it on the FP64
+// unit, twelve terms a cell, was what the kernel took its time for (128x128x64:
+// 327 us, now 149).
+__device__ __forceinline__ bool not_positive(double a) {  // false for NaN
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  return b == 0 || (b >= 0x8000000000000000ull && b <= 0xfff0000000000000ull);
+}
+__device__ __forceinline__ bool not_positive(float a) { return a <= 0.0f; }
+template <typename T, typename R>
+__device__ __forceinline__ T jac_term(T vel, bool plus, T F, T Vden, T rhoe, R rrhoe) {
+  const T u = plus ? vel : -vel;
+  if (not_positive(u)) return (T)0;
+  return quot_i(div_i(mul_i(u, F), Vden), rhoe, rrhoe);
 }
 
 template <typename T>
@@ -850,72 +856,74 @@ __global__ void k_jac(Dims d, GeomT<T> g, const T* __restrict__ rho, const T* __
     const int k = (int)(P / ((size_t)NX * NY));
     const bool ii = i >= 1 && i <= nx, jj = j >= 1 && j <= ny, kk = k >= 1 && k <= nz;
     const T rP = rho[P];
-    const T rPe = rP + e, rrP = (T)1 / rPe;
-    const T VP = g.volc[P] + e, rVP = rvol[P];
+    const T rPe = add_eps(rP);
+    const auto RP = recip_i(rPe);
+    const T VP = add_eps(g.volc[P]);
     T v[7] = {(T)0, (T)0, (T)0, (T)0, (T)0, (T)0, (T)0};
     // face activity: interior faces, plus boundary faces of periodic sides
     auto actx = [&](int fi) { return jj && kk && fi >= 0 && fi <= nx && ((fi >= 1 && fi <= nx - 1) || d.per_x); };
     auto acty = [&](int fj) { return ii && kk && fj >= 0 && fj <= ny && ((fj >= 1 && fj <= ny - 1) || d.per_y); };
     auto actz = [&](int fk) { return ii && jj && fk >= 0 && fk <= nz && ((fk >= 1 && fk <= nz - 1) || d.per_z); };
     // off-diagonals (each a single term)
-    if (actx(i)) v[2] = v[2] + jac_term(g.uf[d.UF(i, j, k)], true, g.fu[d.FU(i, j, k)], g.volc[P + sx] + e, rvol[P + sx], rPe, rrP);
+    if (actx(i)) v[2] = v[2] + jac_term(g.uf[d.UF(i, j, k)], true, g.fu[d.FU(i, j, k)], add_eps(g.volc[P + sx]), rPe, RP);
     if (actx(i - 1))
-      v[4] = v[4] + jac_term(g.uf[d.UF(i - 1, j, k)], false, g.fu[d.FU(i - 1, j, k)], g.volc[P - sx] + e, rvol[P - sx], rPe, rrP);
-    if (acty(j)) v[1] = v[1] + jac_term(g.vf[d.VF(i, j, k)], true, g.fv[d.FV(i, j, k)], g.volc[P + sy] + e, rvol[P + sy], rPe, rrP);
+      v[4] = v[4] + jac_term(g.uf[d.UF(i - 1, j, k)], false, g.fu[d.FU(i - 1, j, k)], add_eps(g.volc[P - sx]), rPe, RP);
+    if (acty(j)) v[1] = v[1] + jac_term(g.vf[d.VF(i, j, k)], true, g.fv[d.FV(i, j, k)], add_eps(g.volc[P + sy]), rPe, RP);
     if (acty(j - 1))
-      v[5] = v[5] + jac_term(g.vf[d.VF(i, j - 1, k)], false, g.fv[d.FV(i, j - 1, k)], g.volc[P - sy] + e, rvol[P - sy], rPe, rrP);
-    if (actz(k)) v[0] = v[0] + jac_term(g.wf[d.WF(i, j, k)], true, g.fw[d.FW(i, j, k)], g.volc[P + sz] + e, rvol[P + sz], rPe, rrP);
+      v[5] = v[5] + jac_term(g.vf[d.VF(i, j - 1, k)], false, g.fv[d.FV(i, j - 1, k)], add_eps(g.volc[P - sy]), rPe, RP);
+    if (actz(k)) v[0] = v[0] + jac_term(g.wf[d.WF(i, j, k)], true, g.fw[d.FW(i, j, k)], add_eps(g.volc[P + sz]), rPe, RP);
     if (actz(k - 1))
-      v[6] = v[6] + jac_term(g.wf[d.WF(i, j, k - 1)], false, g.fw[d.FW(i, j, k - 1)], g.volc[P - sz] + e, rvol[P - sz], rPe, rrP);
+      v[6] = v[6] + jac_term(g.wf[d.WF(i, j, k - 1)], false, g.fw[d.FW(i, j, k - 1)], add_eps(g.volc[P - sz]), rPe, RP);
     // diagonal: interior loops x, y, z (face left of P then face right of P)
     T dg = (T)0;
     if (jj && kk && i - 1 >= 1 && i - 1 <= nx - 1)
-      dg = dg - jac_term(g.uf[d.UF(i - 1, j, k)], false, g.fu[d.FU(i - 1, j, k)], VP, rVP, rPe, rrP);
-    if (jj && kk && i >= 1 && i <= nx - 1) dg = dg - jac_term(g.uf[d.UF(i, j, k)], true, g.fu[d.FU(i, j, k)], VP, rVP, rPe, rrP);
+      dg = dg - jac_term(g.uf[d.UF(i - 1, j, k)], false, g.fu[d.FU(i - 1, j, k)], VP, rPe, RP);
+    if (jj && kk && i >= 1 && i <= nx - 1) dg = dg - jac_term(g.uf[d.UF(i, j, k)], true, g.fu[d.FU(i, j, k)], VP, rPe, RP);
     if (ii && kk && j - 1 >= 1 && j - 1 <= ny - 1)
-      dg = dg - jac_term(g.vf[d.VF(i, j - 1, k)], false, g.fv[d.FV(i, j - 1, k)], VP, rVP, rPe, rrP);
-    if (ii && kk && j >= 1 && j <= ny - 1) dg = dg - jac_term(g.vf[d.VF(i, j, k)], true, g.fv[d.FV(i, j, k)], VP, rVP, rPe, rrP);
+      dg = dg - jac_term(g.vf[d.VF(i, j - 1, k)], false, g.fv[d.FV(i, j - 1, k)], VP, rPe, RP);
+    if (ii && kk && j >= 1 && j <= ny - 1) dg = dg - jac_term(g.vf[d.VF(i, j, k)], true, g.fv[d.FV(i, j, k)], VP, rPe, RP);
     if (ii && jj && k - 1 >= 1 && k - 1 <= nz - 1)
-      dg = dg - jac_term(g.wf[d.WF(i, j, k - 1)], false, g.fw[d.FW(i, j, k - 1)], VP, rVP, rPe, rrP);
-    if (ii && jj && k >= 1 && k <= nz - 1) dg = dg - jac_term(g.wf[d.WF(i, j, k)], true, g.fw[d.FW(i, j, k)], VP, rVP, rPe, rrP);
+      dg = dg - jac_term(g.wf[d.WF(i, j, k - 1)], false, g.fw[d.FW(i, j, k - 1)], VP, rPe, RP);
+    if (ii && jj && k >= 1 && k <= nz - 1) dg = dg - jac_term(g.wf[d.WF(i, j, k)], true, g.fw[d.FW(i, j, k)], VP, rPe, RP);
     // neighbour branches W, E, S, N, B, T of a periodic block
     if (d.per_x && jj && kk) {
-      if (i == 0) dg = dg - jac_term(g.uf[d.UF(0, j, k)], true, g.fu[d.FU(0, j, k)], VP, rVP, rPe, rrP);
-      if (i == 1) dg = dg - jac_term(g.uf[d.UF(0, j, k)], false, g.fu[d.FU(0, j, k)], VP, rVP, rPe, rrP);
-      if (i == nx) dg = dg - jac_term(g.uf[d.UF(nx, j, k)], true, g.fu[d.FU(nx, j, k)], VP, rVP, rPe, rrP);
-      if (i == nx + 1) dg = dg - jac_term(g.uf[d.UF(nx, j, k)], false, g.fu[d.FU(nx, j, k)], VP, rVP, rPe, rrP);
+      if (i == 0) dg = dg - jac_term(g.uf[d.UF(0, j, k)], true, g.fu[d.FU(0, j, k)], VP, rPe, RP);
+      if (i == 1) dg = dg - jac_term(g.uf[d.UF(0, j, k)], false, g.fu[d.FU(0, j, k)], VP, rPe, RP);
+      if (i == nx) dg = dg - jac_term(g.uf[d.UF(nx, j, k)], true, g.fu[d.FU(nx, j, k)], VP, rPe, RP);
+      if (i == nx + 1) dg = dg - jac_term(g.uf[d.UF(nx, j, k)], false, g.fu[d.FU(nx, j, k)], VP, rPe, RP);
     }
     // outer walls 'ow'/'oe' (ADVECT/Advection_Mod.f90:2390-2410, 2469-2489): the
     // outflow through the wall face on the interior cell's diagonal
     if (!d.per_x && jj && kk) {
-      if (i == 1) dg = dg - jac_term(g.uf[d.UF(0, j, k)], false, g.fu[d.FU(0, j, k)], VP, rVP, rPe, rrP);
-      if (i == nx) dg = dg - jac_term(g.uf[d.UF(nx, j, k)], true, g.fu[d.FU(nx, j, k)], VP, rVP, rPe, rrP);
+      if (i == 1) dg = dg - jac_term(g.uf[d.UF(0, j, k)], false, g.fu[d.FU(0, j, k)], VP, rPe, RP);
+      if (i == nx) dg = dg - jac_term(g.uf[d.UF(nx, j, k)], true, g.fu[d.FU(nx, j, k)], VP, rPe, RP);
     }
     if (d.per_y && ii && kk) {
-      if (j == 0) dg = dg - jac_term(g.vf[d.VF(i, 0, k)], true, g.fv[d.FV(i, 0, k)], VP, rVP, rPe, rrP);
-      if (j == 1) dg = dg - jac_term(g.vf[d.VF(i, 0, k)], false, g.fv[d.FV(i, 0, k)], VP, rVP, rPe, rrP);
-      if (j == ny) dg = dg - jac_term(g.vf[d.VF(i, ny, k)], true, g.fv[d.FV(i, ny, k)], VP, rVP, rPe, rrP);
-      if (j == ny + 1) dg = dg - jac_term(g.vf[d.VF(i, ny, k)], false, g.fv[d.FV(i, ny, k)], VP, rVP, rPe, rrP);
+      if (j == 0) dg = dg - jac_term(g.vf[d.VF(i, 0, k)], true, g.fv[d.FV(i, 0, k)], VP, rPe, RP);
+      if (j == 1) dg = dg - jac_term(g.vf[d.VF(i, 0, k)], false, g.fv[d.FV(i, 0, k)], VP, rPe, RP);
+      if (j == ny) dg = dg - jac_term(g.vf[d.VF(i, ny, k)], true, g.fv[d.FV(i, ny, k)], VP, rPe, RP);
+      if (j == ny + 1) dg = dg - jac_term(g.vf[d.VF(i, ny, k)], false, g.fv[d.FV(i, ny, k)], VP, rPe, RP);
     }
     if (!d.per_y && ii && kk) {  // 'os'/'on'
-      if (j == 1) dg = dg - jac_term(g.vf[d.VF(i, 0, k)], false, g.fv[d.FV(i, 0, k)], VP, rVP, rPe, rrP);
-      if (j == ny) dg = dg - jac_term(g.vf[d.VF(i, ny, k)], true, g.fv[d.FV(i, ny, k)], VP, rVP, rPe, rrP);
+      if (j == 1) dg = dg - jac_term(g.vf[d.VF(i, 0, k)], false, g.fv[d.FV(i, 0, k)], VP, rPe, RP);
+      if (j == ny) dg = dg - jac_term(g.vf[d.VF(i, ny, k)], true, g.fv[d.FV(i, ny, k)], VP, rPe, RP);
     }
     if (d.per_z && ii && jj) {
-      if (k == 0) dg = dg - jac_term(g.wf[d.WF(i, j, 0)], true, g.fw[d.FW(i, j, 0)], VP, rVP, rPe, rrP);
-      if (k == 1) dg = dg - jac_term(g.wf[d.WF(i, j, 0)], false, g.fw[d.FW(i, j, 0)], VP, rVP, rPe, rrP);
-      if (k == nz) dg = dg - jac_term(g.wf[d.WF(i, j, nz)], true, g.fw[d.FW(i, j, nz)], VP, rVP, rPe, rrP);
-      if (k == nz + 1) dg = dg - jac_term(g.wf[d.WF(i, j, nz)], false, g.fw[d.FW(i, j, nz)], VP, rVP, rPe, rrP);
+      if (k == 0) dg = dg - jac_term(g.wf[d.WF(i, j, 0)], true, g.fw[d.FW(i, j, 0)], VP, rPe, RP);
+      if (k == 1) dg = dg - jac_term(g.wf[d.WF(i, j, 0)], false, g.fw[d.FW(i, j, 0)], VP, rPe, RP);
+      if (k == nz) dg = dg - jac_term(g.wf[d.WF(i, j, nz)], true, g.fw[d.FW(i, j, nz)], VP, rPe, RP);
+      if (k == nz + 1) dg = dg - jac_term(g.wf[d.WF(i, j, nz)], false, g.fw[d.FW(i, j, nz)], VP, rPe, RP);
     }
     if (!d.per_z && ii && jj) {  // 'ob'/'ot'
-      if (k == 1) dg = dg - jac_term(g.wf[d.WF(i, j, 0)], false, g.fw[d.FW(i, j, 0)], VP, rVP, rPe, rrP);
-      if (k == nz) dg = dg - jac_term(g.wf[d.WF(i, j, nz)], true, g.fw[d.FW(i, j, nz)], VP, rVP, rPe, rrP);
+      if (k == 1) dg = dg - jac_term(g.wf[d.WF(i, j, 0)], false, g.fw[d.FW(i, j, 0)], VP, rPe, RP);
+      if (k == nz) dg = dg - jac_term(g.wf[d.WF(i, j, nz)], true, g.fw[d.FW(i, j, nz)], VP, rPe, RP);
     }
     // JacDiffusionCompute (ADVECT/Diffusion_Mod.f90:1504-1708): per face with
     // a neighbour Temp = 2K; the off-diagonal of each column and its diagonal
     // (face left of P, then face right of P; x, y, z) get
     // Temp/(VolC_row+Eps)/(Rho_col+Eps)
     if (dkx) {
+      const T rrP = (T)1 / rPe;
       auto term = [&](T K, size_t Q) { return div_rn(div_rn((T)2 * K, g.volc[Q] + e, rvol[Q]), rPe, rrP); };
       if (actx(i - 1)) {
         const T K = dkx[d.UF(i - 1, j, k)];

@@ -62,6 +62,8 @@ namespace asam {
 
 namespace prj {
 
+using fpi::Num;
+
 constexpr int kMaxLev = 8;
 constexpr int kPlaneBlock = 256;
 constexpr int kRedGrid = 1024;
@@ -381,7 +383,6 @@ __global__ void k_coarse_1d(Fields g, Fields c, int s1, int s2, int s3) {
 // hierarchy take 2.6 ms instead of 7.6.
 __global__ void k_assemble(Fields c, Lev2 P, double* __restrict__ u3, double* __restrict__ l3, int full, double bd2,
                            Facs fc, double fac_anela) {
-  using fpi::Num;
   const int n1 = c.n1, n2 = c.n2, n3 = c.n3;
   const size_t tot = (size_t)n1 * n2 * n3;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
@@ -506,6 +507,11 @@ __global__ void k_factor(Lev2 P) {
 
 // MatVecT_2D at entry (i,j) of a plane (TriDiagT_Mod.f90:113-133, 405-431);
 // x is the plane's vector, mo the plane's offset in the matrix arrays
+// a product: FP64 on the integer units, beside the sums on the FP64 unit
+// (k_matvec3 of 256x256x64: 119 instead of 137 us)
+__device__ __forceinline__ double mulq(double a, double b) { return fpi::mul_rn(a, b); }
+__device__ __forceinline__ float mulq(float a, float b) { return a * b; }
+
 template <typename T, bool kWrap = false>
 __device__ inline T matvec2_at(const Lev2T<T>& P, size_t mo, const T* __restrict__ x, size_t s, int i, int j,
                                int k) {
@@ -516,13 +522,13 @@ __device__ inline T matvec2_at(const Lev2T<T>& P, size_t mo, const T* __restrict
   T y;
   if (c1 > 1) {
     if (i == 0)
-      y = d[s] * x[s] + uz[s] * x[s + w];
+      y = mulq(d[s], x[s]) + mulq(uz[s], x[s + w]);
     else if (i < c1 - 1)
-      y = lz[s - w] * x[s - w] + d[s] * x[s] + uz[s] * x[s + w];
+      y = mulq(lz[s - w], x[s - w]) + mulq(d[s], x[s]) + mulq(uz[s], x[s + w]);
     else
-      y = lz[s - w] * x[s - w] + d[s] * x[s];
+      y = mulq(lz[s - w], x[s - w]) + mulq(d[s], x[s]);
   } else {
-    y = d[s] * x[s];
+    y = mulq(d[s], x[s]);
   }
   if (c2 > 1) {
     const size_t row = (size_t)i * w;
@@ -530,19 +536,19 @@ __device__ inline T matvec2_at(const Lev2T<T>& P, size_t mo, const T* __restrict
     const T* lx = P.lx + mo;
     if (j == 0) {
       const size_t sr = row + slot(0, P.h, 0, j + 1);
-      y = y + ux[s] * x[sr];
+      y = y + mulq(ux[s], x[sr]);
     } else if (j < c2 - 1) {
       const size_t sl = row + slot(0, P.h, 0, j - 1), sr = row + slot(0, P.h, 0, j + 1);
-      y = y + lx[sl] * x[sl] + ux[s] * x[sr];
+      y = y + mulq(lx[sl], x[sl]) + mulq(ux[s], x[sr]);
     } else {
       const size_t sl = row + slot(0, P.h, 0, j - 1);
-      y = y + lx[sl] * x[sl];
+      y = y + mulq(lx[sl], x[sl]);
     }
   }
   if (kWrap && P.wxl && (j == 0 || j == c2 - 1)) {  // periodic-Laplacian hierarchy: across the periodic x side
     const size_t row = (size_t)i * w, kc = (size_t)k * c1;
     if (j == 0) y = y + P.wxl[kc + i] * x[row + slot(0, P.h, 0, c2 - 1)];
-    if (j == c2 - 1) y = y + P.wxh[kc + i] * x[row];
+    if (j == c2 - 1) y = y + mulq(P.wxh[kc + i], x[row]);
   }
   return y;
 }
@@ -1193,15 +1199,15 @@ __global__ void k_matvec3(const Lev3T<T>* __restrict__ lvs, int L, const T* __re
     T v = matvec2_at<T, kWrap>(P, (size_t)k * ps, x + (size_t)k * ps, s, i, j, k);
     if (A.m3 > 1) {
       if (k == 0)
-        v = v + A.u3[e] * x[e + ps];
+        v = v + mulq(A.u3[e], x[e + ps]);
       else if (k < A.m3 - 1)
-        v = v + A.l3[e - ps] * x[e - ps] + A.u3[e] * x[e + ps];
+        v = v + mulq(A.l3[e - ps], x[e - ps]) + mulq(A.u3[e], x[e + ps]);
       else
-        v = v + A.l3[e - ps] * x[e - ps];
+        v = v + mulq(A.l3[e - ps], x[e - ps]);
     }
     if (kWrap && A.wyl) {  // periodic-Laplacian hierarchy: across the periodic y side
-      if (k == 0) v = v + A.wyl[s] * x[(size_t)(A.m3 - 1) * ps + s];
-      if (k == A.m3 - 1) v = v + A.wyh[s] * x[s];
+      if (k == 0) v = v + mulq(A.wyl[s], x[(size_t)(A.m3 - 1) * ps + s]);
+      if (k == A.m3 - 1) v = v + mulq(A.wyh[s], x[s]);
     }
     y[e] = mode == 0 ? b[e] - v : (mode == 1 ? -v : v);
   }
@@ -1269,14 +1275,16 @@ __global__ void k_from_layout(Lev2 P, int nx, int ny, int nz, const double* __re
 }
 
 // ---------------------------------------------------------------------------
-// FGMRES vector kernels (padding entries of the layout stay 0)
+// FGMRES vector kernels (padding entries of the layout stay 0); the products of
+// the Gram-Schmidt pass on the integer units, its sums on the FP64 unit
+// (256x256x64: a dot product 19 instead of 25 us, an update 14 instead of 19)
 // ---------------------------------------------------------------------------
 __global__ void k_pdot_partial(const double* __restrict__ a, const double* __restrict__ b, size_t n,
                                double* __restrict__ partial) {
   __shared__ double sh[kRedBlock];
   double s = 0.0;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-    s = s + a[e] * b[e];
+    s = s + fpi::mul_rn(a[e], b[e]);
   sh[threadIdx.x] = s;
   __syncthreads();
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
@@ -1302,7 +1310,7 @@ __global__ void k_pdot_final(const double* __restrict__ partial, int n, double* 
 __global__ void k_axpy_negdev(double* __restrict__ y, const double* __restrict__ x, const double* h, size_t n) {
   const double a = -*h;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-    y[e] = a * x[e] + y[e];
+    y[e] = fpi::mul_rn(a, x[e]) + y[e];
 }
 // v = (1/*h)*v   (DSCALE(One/H(i+1,i)))
 __global__ void k_scale_recipdev(double* __restrict__ v, const double* h, size_t n) {
@@ -1374,7 +1382,7 @@ __global__ void k_update_vel(Dims d, GeomT<double> g, Wts wt, double* __restrict
   const double* mzx = wt.metr + ny + 2 * nz + nx;
   const double* mzy = wt.metr + ny + 2 * nz + 2 * nx;
   auto C = [&](int i, int j, int k) { return (size_t)(i - 1) + (size_t)nx * ((size_t)(j - 1) + (size_t)ny * (size_t)(k - 1)); };
-  auto pd = [&](int i, int j, int k) { const size_t q = C(i, j, k); return p[q] * wt.dut[q]; };
+  auto pd = [&](int i, int j, int k) { const size_t q = C(i, j, k); return fpi::mul_rn(p[q], wt.dut[q]); };
   const size_t nu = (size_t)(nx + 1) * ny * nz, nv = (size_t)nx * (ny + 1) * nz, nw = (size_t)nx * ny * (nz + 1);
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nu + nv + nw; e += (size_t)gridDim.x * blockDim.x) {
     if (e < nu) {
@@ -1388,9 +1396,9 @@ __global__ void k_update_vel(Dims d, GeomT<double> g, Wts wt, double* __restrict
         u[e] = u[e] + t;
       }
       if (i >= 1 && i <= nx - 1) {
-        const double t = 2.0 * beta0 * dtp * wt.duu[e] * (pd(i + 1, j, k) - pd(i, j, k)) /
-                         ((wt.dx[i] + wt.dx[i - 1]) * mxy[j - 1] * mxz[k - 1]);
-        u[e] = u[e] - t;
+        const Num t = Num(2.0 * beta0 * dtp) * wt.duu[e] * (pd(i + 1, j, k) - pd(i, j, k)) /
+                         ((Num(wt.dx[i]) + wt.dx[i - 1]) * mxy[j - 1] * mxz[k - 1]);
+        u[e] = u[e] - t.v;
       }
     } else if (e < nu + nv) {
       const size_t ee = e - nu;
@@ -1404,9 +1412,9 @@ __global__ void k_update_vel(Dims d, GeomT<double> g, Wts wt, double* __restrict
         v[ee] = v[ee] + t;
       }
       if (j >= 1 && j <= ny - 1) {
-        const double t = 2.0 * beta0 * dtp * wt.duv[ee] * (pd(i, j + 1, k) - pd(i, j, k)) /
-                         ((wt.dy[j] + wt.dy[j - 1]) * myx[i - 1] * myz[k - 1]);
-        v[ee] = v[ee] - t;
+        const Num t = Num(2.0 * beta0 * dtp) * wt.duv[ee] * (pd(i, j + 1, k) - pd(i, j, k)) /
+                         ((Num(wt.dy[j]) + wt.dy[j - 1]) * myx[i - 1] * myz[k - 1]);
+        v[ee] = v[ee] - t.v;
       }
     } else {
       const size_t ee = e - nu - nv;
@@ -1424,8 +1432,8 @@ __global__ void k_update_vel(Dims d, GeomT<double> g, Wts wt, double* __restrict
         w[ee] = w[ee] + fwv / (fwv + asam::kEps) * t;
       }
       if (k >= 1 && k <= nz - 1) {
-        const double t = 2.0 * beta0 * dtp * wt.duw[ee] * (pd(i, j, k + 1) - pd(i, j, k)) / (wt.dz[k] + wt.dz[k - 1]);
-        w[ee] = w[ee] - fwv / (fwv + asam::kEps) * t;
+        const Num t = Num(2.0 * beta0 * dtp) * wt.duw[ee] * (pd(i, j, k + 1) - pd(i, j, k)) / (wt.dz[k] + wt.dz[k - 1]);
+        w[ee] = w[ee] - (Num(fwv) / (fwv + asam::kEps) * t).v;
       }
     }
   }
@@ -1450,23 +1458,23 @@ __global__ void k_update_incr(Dims d, GeomT<double> g, Wts wt, const double* __r
     const int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
     const size_t P = d.P(i, j, k);
     const double vC = g.volc[P];
-    const double fuR = g.fu[d.FU(i, j, k)], fuL = g.fu[d.FU(i - 1, j, k)];
-    const double fvR = g.fv[d.FV(i, j, k)], fvL = g.fv[d.FV(i, j - 1, k)];
-    const double fwR = g.fw[d.FW(i, j, k)], fwL = g.fw[d.FW(i, j, k - 1)];
+    const Num fuR = g.fu[d.FU(i, j, k)], fuL = g.fu[d.FU(i - 1, j, k)];
+    const Num fvR = g.fv[d.FV(i, j, k)], fvL = g.fv[d.FV(i, j - 1, k)];
+    const Num fwR = g.fw[d.FW(i, j, k)], fwL = g.fw[d.FW(i, j, k - 1)];
     const double uR = u[d.UF(i, j, k)], uL = u[d.UF(i - 1, j, k)];
     const double vR = v[d.VF(i, j, k)], vL = v[d.VF(i, j - 1, k)];
     const double wR = w[d.WF(i, j, k)], wL = w[d.WF(i, j, k - 1)];
     if (th_pos >= 0) {
-      const double s = fuR * wt.dtu[d.UF(i, j, k)] * uR - fuL * wt.dtu[d.UF(i - 1, j, k)] * uL +
-                       fvR * wt.dtv[d.VF(i, j, k)] * vR - fvL * wt.dtv[d.VF(i, j - 1, k)] * vL +
-                       fwR * wt.dtw[d.WF(i, j, k)] * wR - fwL * wt.dtw[d.WF(i, j, k - 1)] * wL;
+      const Num s = fuR * wt.dtu[d.UF(i, j, k)] * uR - fuL * wt.dtu[d.UF(i - 1, j, k)] * uL +
+                    fvR * wt.dtv[d.VF(i, j, k)] * vR - fvL * wt.dtv[d.VF(i, j - 1, k)] * vL +
+                    fwR * wt.dtw[d.WF(i, j, k)] * wR - fwL * wt.dtw[d.WF(i, j, k - 1)] * wL;
       double* c = incr + (size_t)th_pos * npad;
-      c[P] = c[P] - dtp * beta0 * wt.dtt[e] * s / (vC + asam::kEps);
+      c[P] = c[P] - (Num(dtp * beta0) * wt.dtt[e] * s / (vC + asam::kEps)).v;
     }
     if (rho_pos >= 0) {
-      const double s = fuR * uR - fuL * uL + fvR * vR - fvL * vL + fwR * wR - fwL * wL;
+      const Num s = fuR * uR - fuL * uL + fvR * vR - fvL * vL + fwR * wR - fwL * wL;
       double* c = incr + (size_t)rho_pos * npad;
-      c[P] = c[P] - dtp * beta0 * s / (vC + asam::kEps);
+      c[P] = c[P] - (Num(dtp * beta0) * s / (vC + asam::kEps)).v;
     }
   }
 }
@@ -1477,11 +1485,12 @@ __global__ void k_update_incr(Dims d, GeomT<double> g, Wts wt, const double* __r
 // The reference evaluates each face once from either cell; the two
 // evaluations are equal bit for bit (the sums are commutative, the product
 // and the quotient are taken in the same order), so the face terms are
-// computed once per face here: 5 divisions per cell instead of 14.
+// computed once per face here: 5 divisions per cell instead of 14, on the
+// integer units like the products.
 __global__ void k_div_m(size_t npad, const double* __restrict__ volc, const double* __restrict__ cc,
                         const double* __restrict__ rho, double* __restrict__ m) {
   for (size_t P = blockIdx.x * (size_t)blockDim.x + threadIdx.x; P < npad; P += (size_t)gridDim.x * blockDim.x)
-    m[P] = volc[P] * cc[P] / (rho[P] + asam::kEps);
+    m[P] = (Num(volc[P]) * cc[P] / (Num(rho[P]) + asam::kEps)).v;
 }
 
 // face terms F = Fa * u * (m_L + m_R) / (V_L + V_R + Eps) of the u, v and w
@@ -1498,21 +1507,21 @@ __global__ void k_div_faces(Dims d, GeomT<double> g, const double* __restrict__ 
       const size_t r = e / (nx + 1);
       const int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
       const size_t L = d.P(i, j, k), R = L + 1;
-      fu[e] = g.fu[d.FU(i, j, k)] * u[e] * (m[L] + m[R]) / (g.volc[L] + g.volc[R] + asam::kEps);
+      fu[e] = (Num(g.fu[d.FU(i, j, k)]) * u[e] * (m[L] + m[R]) / (g.volc[L] + g.volc[R] + asam::kEps)).v;
     } else if (e < nu + nv) {  // j = 0..ny
       const size_t q = e - nu;
       const int i = (int)(q % nx) + 1;
       const size_t r = q / nx;
       const int j = (int)(r % (ny + 1)), k = (int)(r / (ny + 1)) + 1;
       const size_t L = d.P(i, j, k), R = L + sy;
-      fv[q] = g.fv[d.FV(i, j, k)] * v[q] * (m[L] + m[R]) / (g.volc[L] + g.volc[R] + asam::kEps);
+      fv[q] = (Num(g.fv[d.FV(i, j, k)]) * v[q] * (m[L] + m[R]) / (g.volc[L] + g.volc[R] + asam::kEps)).v;
     } else {  // k = 0..nz
       const size_t q = e - nu - nv;
       const int i = (int)(q % nx) + 1;
       const size_t r = q / nx;
       const int j = (int)(r % ny) + 1, k = (int)(r / ny);
       const size_t L = d.P(i, j, k), R = L + sz;
-      fw[q] = g.fw[d.FW(i, j, k)] * w[q] * (m[L] + m[R]) / (g.volc[L] + g.volc[R] + asam::kEps);
+      fw[q] = (Num(g.fw[d.FW(i, j, k)]) * w[q] * (m[L] + m[R]) / (g.volc[L] + g.volc[R] + asam::kEps)).v;
     }
   }
 }
@@ -1529,7 +1538,7 @@ __global__ void k_div_apply(Dims d, GeomT<double> g, const double* __restrict__ 
     const size_t P = d.P(i, j, k);
     const double s = fu[d.UF(i, j, k)] - fu[d.UF(i - 1, j, k)] + fv[d.VF(i, j, k)] - fv[d.VF(i, j - 1, k)] +
                      fw[d.WF(i, j, k)] - fw[d.WF(i, j, k - 1)];
-    cd[P] = cd[P] - dtp * beta0 * s / (g.volc[P] + asam::kEps);
+    cd[P] = cd[P] - (Num(dtp * beta0) * s / (g.volc[P] + asam::kEps)).v;
   }
 }
 
@@ -1765,17 +1774,18 @@ __global__ void k_weights_density(Dims d, GeomT<double> g, Wts wt, const double*
   const size_t nc = (size_t)nx * ny * nz, nu = (size_t)(nx + 1) * ny * nz, nv = (size_t)nx * (ny + 1) * nz,
                nw = (size_t)nx * ny * (nz + 1);
   const size_t tot = nc + nu + nv + nw;
-  auto th = [&](size_t P) { return rth[P] / (rho[P] + asam::kEps); };
+  auto th = [&](size_t P) { return fpi::div_rn(rth[P], rho[P] + asam::kEps); };
   auto face = [&](size_t P, size_t Q) {
     const double* V = g.volc;
-    return (V[P] * rth[P] / (rho[P] + asam::kEps) + V[Q] * rth[Q] / (rho[Q] + asam::kEps)) / (V[P] + V[Q] + asam::kEps);
+    return ((Num(V[P]) * rth[P] / (rho[P] + asam::kEps) + Num(V[Q]) * rth[Q] / (rho[Q] + asam::kEps)) /
+            (V[P] + V[Q] + asam::kEps)).v;
   };
   // a periodic x or y side ('iw'/'ie'/'is'/'in' with equal refinement,
   // MULTI/JacAccGrav_Mod.f90:3313-3321, 3360-3368, 3407-3415, 3454-3462): theta
   // first, then times the volume; the halo cell holds the periodic image
   auto pface = [&](size_t P, size_t Q) {
     const double* V = g.volc;
-    return (th(P) * V[P] + th(Q) * V[Q]) / (V[P] + V[Q] + asam::kEps);
+    return ((Num(th(P)) * V[P] + Num(th(Q)) * V[Q]) / (V[P] + V[Q] + asam::kEps)).v;
   };
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
     if (e < nc) {
@@ -1786,10 +1796,10 @@ __global__ void k_weights_density(Dims d, GeomT<double> g, Wts wt, const double*
       const double rvl = rv ? rv[P] : 0.0;
       const double rll = (rc ? rc[P] : 0.0) + (rr ? rr[P] : 0.0);
       const double rd = rho[P] - rvl - rll + asam::kEps;
-      const double rm = kRd + kRv * rvl / rd;
-      const double cpml = kCpd + kCpv * rvl / rd + kCpl * rll / rd;
-      const double kap = rm / cpml;
-      wt.dut[e] = tabs[P] / (rth[P] + asam::kEps) * (rd * kRd + rvl * kRv) / (1.0 - kap);
+      const Num rm = kRd + Num(kRv) * rvl / rd;
+      const Num cpml = kCpd + Num(kCpv) * rvl / rd + Num(kCpl) * rll / rd;
+      const Num kap = rm / cpml;
+      wt.dut[e] = (Num(tabs[P]) / (rth[P] + asam::kEps) * (Num(rd) * kRd + Num(rvl) * kRv) / (1.0 - kap)).v;
       wt.dtt[e] = 1.0;
     } else if (e < nc + nu) {
       const size_t q = e - nc;
@@ -1801,7 +1811,7 @@ __global__ void k_weights_density(Dims d, GeomT<double> g, Wts wt, const double*
       else
         wt.dtu[q] = i == 0 ? th(d.P(1, j, k)) : (i == nx ? th(d.P(nx, j, k)) : face(d.P(i, j, k), d.P(i + 1, j, k)));
       const double f = g.fu[d.FU(i, j, k)];
-      wt.duu[q] = f / (f + asam::kEps);
+      wt.duu[q] = fpi::div_rn(f, f + asam::kEps);
     } else if (e < nc + nu + nv) {
       const size_t q = e - nc - nu;
       const int i = (int)(q % nx) + 1;
@@ -1812,7 +1822,7 @@ __global__ void k_weights_density(Dims d, GeomT<double> g, Wts wt, const double*
       else
         wt.dtv[q] = j == 0 ? th(d.P(i, 1, k)) : (j == ny ? th(d.P(i, ny, k)) : face(d.P(i, j, k), d.P(i, j + 1, k)));
       const double f = g.fv[d.FV(i, j, k)];
-      wt.duv[q] = f / (f + asam::kEps);
+      wt.duv[q] = fpi::div_rn(f, f + asam::kEps);
     } else {
       const size_t q = e - nc - nu - nv;
       const int i = (int)(q % nx) + 1;
@@ -1823,7 +1833,7 @@ __global__ void k_weights_density(Dims d, GeomT<double> g, Wts wt, const double*
       else
         wt.dtw[q] = k == 0 ? th(d.P(i, j, 1)) : (k == nz ? th(d.P(i, j, nz)) : face(d.P(i, j, k), d.P(i, j, k + 1)));
       const double f = g.fw[d.FW(i, j, k)];
-      wt.duw[q] = f / (f + asam::kEps);
+      wt.duw[q] = fpi::div_rn(f, f + asam::kEps);
     }
   }
 }
