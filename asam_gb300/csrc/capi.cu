@@ -802,6 +802,15 @@ __global__ void k_probe_div(unsigned long long n, unsigned long long seed, int s
     if (!same(fpi::div_rn(a, b), __ddiv_rn(a, b))) ++cnt;
     if (!same(fpi::quot_rn(a, b, fpi::recip(b)), __ddiv_rn(a, b))) ++cnt;
     if (!same(fpi::quot_chain(a, b, fpi::recip(b)), __ddiv_rn(a, b))) ++cnt;
+    // conversions between FP32 and FP64: every FP32 pattern, and FP64 numbers of
+    // FP32's range and beyond, half of them next to a rounding point
+    const float f = __uint_as_float((unsigned)(s >> 13));
+    if (!same(fpi::widen(f), (double)f)) ++cnt;
+    const unsigned long long t = splitmix(s);
+    double w = __longlong_as_double((long long)((t & 0x800fffffffffffffull) | (unsigned long long)(863 + (t >> 52) % 320) << 52));
+    if (s >> 20 & 1) w = __longlong_as_double((__double_as_longlong(w) & ~0x1fffffffll) + 0x10000000ll + (long long)((s >> 21) % 3) - 1);
+    for (double v : {w, a})
+      if (__float_as_uint(fpi::narrow(v)) != __float_as_uint((float)v) && !isnan(v)) ++cnt;
   }
   if (cnt) atomicAdd(bad, cnt);
 }

@@ -194,4 +194,25 @@ struct Num {
   friend __device__ __forceinline__ Num operator-(Num a, Num b) { return __dsub_rn(a.v, b.v); }
 };
 
+// FP32 to FP64 and back, rounded to nearest even.  A conversion is an FP64
+// instruction as well (64 cycles of a sub-partition per warp), so the conversions
+// of normal numbers and their products run on the integer units.
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), a = b & 0x7fffffffu;
+  if (a - 0x00800000u >= 0x7f000000u && a != 0) return (double)x;  // subnormal, infinite, NaN
+  const unsigned hi = a == 0 ? b : ((a >> 3) + (896u << 20)) | (b & 0x80000000u);
+  return __hiloint2double((int)hi, (int)(b << 29));
+}
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned a = hi & 0x7fffffffu;
+  if (a - (897u << 20) >= (254u << 20)) {  // the result is not a normal number
+    if ((a | lo) == 0) return __uint_as_float(hi);
+    return (float)x;
+  }
+  const unsigned m = ((a - (896u << 20)) << 3) | (lo >> 29), rest = lo << 3;
+  const unsigned up = rest > 0x80000000u || (rest == 0x80000000u && (m & 1u));
+  return __uint_as_float((m + up) | (hi & 0x80000000u));  // a carry out of the largest exponent gives infinity
+}
+
 }  // namespace fpi
