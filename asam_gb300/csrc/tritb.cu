@@ -41,6 +41,11 @@ __device__ __forceinline__ V2 mult_2(const M2& b, const V2& c) {
   return V2{__dadd_rn(__dmul_rn(b.a11, c.x1), __dmul_rn(b.a12, c.x2)),
             __dadd_rn(__dmul_rn(b.a21, c.x1), __dmul_rn(b.a22, c.x2))};
 }
+// mult_2 with the products on the integer units
+__device__ __forceinline__ V2 mult_2i(const M2& b, const V2& c) {
+  return V2{__dadd_rn(fpi::mul_rn(b.a11, c.x1), fpi::mul_rn(b.a12, c.x2)),
+            __dadd_rn(fpi::mul_rn(b.a21, c.x1), fpi::mul_rn(b.a22, c.x2))};
+}
 // Mult_22(b,c): temp(r,s)=b(r,1)*c(1,s)+b(r,2)*c(2,s)
 __device__ __forceinline__ M2 mult_22(const M2& b, const M2& c) {
   return M2{__dadd_rn(__dmul_rn(b.a11, c.a11), __dmul_rn(b.a12, c.a21)),
@@ -571,36 +576,33 @@ __global__ void k_tri_tb_compute_3d(int tr, int couple, int n3, int n2, int n1, 
 // that multiply the neighbour's first component; TriDiagTR's are 2x2 blocks
 // (Mult_2).
 __device__ __forceinline__ V2 couple_mul(int tr, const double* c, const V2& x) {
-  if (tr) return mult_2(ld_m(c), x);
+  if (tr) return mult_2i(ld_m(c), x);
   return V2{__dmul_rn(c[0], x.x1), __dmul_rn(c[1], x.x1)};
 }
 
-// entry e of the level product; planes are coupled only when u3 is given
-// (otherwise n3 counts independent planes)
-__device__ __forceinline__ V2 level_entry(int tr, int n3, int n2, int n1, const double* __restrict__ d,
+// entry (i, j, k) of the level product; planes are coupled only when u3 is given
+// (otherwise n3 counts independent planes).  The products run on the integer
+// units beside the sums on the FP64 unit.
+__device__ __forceinline__ V2 level_entry_at(int tr, int n3, int n2, int n1, const double* __restrict__ d,
                                           const double* __restrict__ u1, const double* __restrict__ l1,
                                           const double* __restrict__ u2, const double* __restrict__ l2,
                                           const double* __restrict__ u3, const double* __restrict__ l3,
-                                          const double* __restrict__ x, size_t e) {
-  const size_t npl = (size_t)n2 * n1;
-  const int i = (int)(e % n1);
-  const size_t line = e / n1;
-  const int j = (int)(line % n2);
-  const int k = (int)(line / n2);
+                                          const double* __restrict__ x, int i, int j, int k) {
+  const size_t npl = (size_t)n2 * n1, line = (size_t)k * n2 + j, e = line * n1 + i;
   const double* xl = x + line * n1 * 2;
   const M2 di = ld_m(d + e * 4);
   V2 r;  // MatVecTB_1D of the line, entry i
   if (n1 == 1) {
-    r = mult_2(di, ld_v(xl));
+    r = mult_2i(di, ld_v(xl));
   } else if (i == 0) {
-    r = add_v(mult_2(di, ld_v(xl)), mult_2(ld_m(u1 + line * (n1 - 1) * 4), ld_v(xl + 2)));
+    r = add_v(mult_2i(di, ld_v(xl)), mult_2i(ld_m(u1 + line * (n1 - 1) * 4), ld_v(xl + 2)));
   } else if (i == n1 - 1) {
-    r = add_v(mult_2(ld_m(l1 + (line * (n1 - 1) + i - 1) * 4), ld_v(xl + (size_t)(i - 1) * 2)),
-              mult_2(di, ld_v(xl + (size_t)i * 2)));
+    r = add_v(mult_2i(ld_m(l1 + (line * (n1 - 1) + i - 1) * 4), ld_v(xl + (size_t)(i - 1) * 2)),
+              mult_2i(di, ld_v(xl + (size_t)i * 2)));
   } else {
-    r = add_v(add_v(mult_2(ld_m(l1 + (line * (n1 - 1) + i - 1) * 4), ld_v(xl + (size_t)(i - 1) * 2)),
-                    mult_2(di, ld_v(xl + (size_t)i * 2))),
-              mult_2(ld_m(u1 + (line * (n1 - 1) + i) * 4), ld_v(xl + (size_t)(i + 1) * 2)));
+    r = add_v(add_v(mult_2i(ld_m(l1 + (line * (n1 - 1) + i - 1) * 4), ld_v(xl + (size_t)(i - 1) * 2)),
+                    mult_2i(di, ld_v(xl + (size_t)i * 2))),
+              mult_2i(ld_m(u1 + (line * (n1 - 1) + i) * 4), ld_v(xl + (size_t)(i + 1) * 2)));
   }
   if (n2 > 1) {  // between lines of plane k
     const size_t c0 = (size_t)k * (n2 - 1) * n1;
@@ -613,6 +615,15 @@ __device__ __forceinline__ V2 level_entry(int tr, int n3, int n2, int n1, const 
     if (k < n3 - 1) r = add_v(r, couple_mul(tr, u3 + ((size_t)k * npl + r0) * 4, ld_v(x + (e + npl) * 2)));
   }
   return r;
+}
+__device__ __forceinline__ V2 level_entry(int tr, int n3, int n2, int n1, const double* __restrict__ d,
+                                          const double* __restrict__ u1, const double* __restrict__ l1,
+                                          const double* __restrict__ u2, const double* __restrict__ l2,
+                                          const double* __restrict__ u3, const double* __restrict__ l3,
+                                          const double* __restrict__ x, size_t e) {
+  const size_t line = e / n1;
+  const int k = (int)(line / n2);
+  return level_entry_at(tr, n3, n2, n1, d, u1, l1, u2, l2, u3, l3, x, (int)(e - line * n1), (int)(line - (size_t)k * n2), k);
 }
 
 __global__ void k_tri_tb_matvec_3d(int tr, int n3, int n2, int n1, const double* __restrict__ d,
@@ -847,24 +858,48 @@ struct PlaneHierDev {
 // per component, so a row is seven FP64 instructions, a quotient on the
 // integer units and two exchanges with the partner lane forward, and four
 // instructions backward (one lane per line with its own factors: about 70
-// and 8).  The next row's operands are loaded while this row runs.
+// and 8).  The operands of the next rows (three forward, six backward) are in
+// flight while these run: one row ahead was less than an L2 latency backward.
+// The right-hand sides' products run on the integer units.  V-cycle of 48x96x80
+// cells: 26.8 ms, 29.7 with one row ahead and all of it on the FP64 unit.
 __device__ __forceinline__ void tb_half(int tr, int n2, int n1, const double* __restrict__ l2,
                                         const double* __restrict__ u2, const double* __restrict__ fac,
                                         const double* b, double* x, int c, int bwd) {
-  const int nl = (n2 - c + 1) / 2, w1 = 2 * n1;
+  const int nl = (n2 - c + 1) / 2, w1 = 2 * n1, tot = nl * w1;
   const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < nl * w1; e += nt) {
-    const int q = e / w1, o = e - q * w1, r = o & 1;
-    const int j = 2 * q + c;
-    const size_t pos = (size_t)j * w1 + o;
-    const double bv = b[pos];
-    double ml = 0.0, mu = 0.0;  // a missing neighbour: t - 0 leaves every bit of t
-    auto mult = [&](const double* cp, const double* xn) {
-      return tr ? __dadd_rn(__dmul_rn(cp[r], xn[0]), __dmul_rn(cp[r + 2], xn[1])) : __dmul_rn(cp[r], xn[0]);
-    };
-    if (j > 0) ml = mult(l2 + ((size_t)(j - 1) * w1 + (o - r)) * 2, x + pos - r - w1);
-    if (j < n2 - 1) mu = mult(u2 + ((size_t)j * w1 + (o - r)) * 2, x + pos - r + w1);
-    x[pos] = bwd ? __dsub_rn(__dsub_rn(bv, mu), ml) : __dsub_rn(__dsub_rn(bv, ml), mu);
+  auto pair = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
+  // four entries a thread at a time, so that their loads are in flight together
+  constexpr int kU = 4;
+  for (int e0 = tid; e0 < tot; e0 += kU * nt) {
+    double bv[kU];
+    double2 cl[kU], cu[kU], xl[kU], xu[kU];
+    int pos[kU];
+#pragma unroll
+    for (int v = 0; v < kU; ++v) {
+      const int e = e0 + v * nt;
+      pos[v] = -1;
+      // a missing neighbour: t - 0 leaves every bit of t
+      bv[v] = 0.0;
+      cl[v] = cu[v] = xl[v] = xu[v] = make_double2(0.0, 0.0);
+      if (e < tot) {
+        const int q = e / w1, o = e - q * w1, r = o & 1;
+        const int j = 2 * q + c;
+        pos[v] = j * w1 + o;
+        bv[v] = b[pos[v]];
+        auto coef = [&](const double* cp) { return make_double2(cp[r], tr ? cp[r + 2] : 0.0); };
+        if (j > 0) cl[v] = coef(l2 + ((size_t)(j - 1) * w1 + (o - r)) * 2), xl[v] = pair(x + pos[v] - r - w1);
+        if (j < n2 - 1) cu[v] = coef(u2 + ((size_t)j * w1 + (o - r)) * 2), xu[v] = pair(x + pos[v] - r + w1);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < kU; ++v) {
+      auto mult = [&](double2 cp, double2 xn) {
+        return tr ? __dadd_rn(fpi::mul_rn(cp.x, xn.x), fpi::mul_rn(cp.y, xn.y)) : fpi::mul_rn(cp.x, xn.x);
+      };
+      if (pos[v] < 0) continue;
+      const double ml = mult(cl[v], xl[v]), mu = mult(cu[v], xu[v]);
+      x[pos[v]] = bwd ? __dsub_rn(__dsub_rn(bv[v], mu), ml) : __dsub_rn(__dsub_rn(bv[v], ml), mu);
+    }
   }
   __syncthreads();
   const int r = tid & 1;
@@ -874,45 +909,78 @@ __device__ __forceinline__ void tb_half(int tr, int n2, int n1, const double* __
     const int j = 2 * q + c;
     double* xp = x + (size_t)j * w1 + r;
     const double* fp = fac + (size_t)j * n1 * kTbFac;
-    auto pair = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
     auto other = [](double v) { return __shfl_xor_sync(0xffffffffu, v, 1); };
-    double t = xp[0], c1 = 0.0, c2 = 0.0, y = 0.0;
-    double2 ad = pair(fp + 2 * r), l = pair(fp + 4 + 2 * r), dr = pair(fp + 12);
-    for (int i = 0; i < n1; ++i) {
-      const int in = i + 1 < n1 ? i + 1 : i;
-      const double* fn = fp + (size_t)in * kTbFac;
-      const double2 adn = pair(fn + 2 * r), ln = pair(fn + 4 + 2 * r), drn = pair(fn + 12);
-      const double tn = in > i ? xp[2 * in] : 0.0;
-      const double v = __dsub_rn(t, __dadd_rn(__dmul_rn(l.x, c1), __dmul_rn(l.y, c2)));
-      const double vo = other(v);
-      const double num = __dadd_rn(__dmul_rn(ad.x, r ? vo : v), __dmul_rn(ad.y, r ? v : vo));
-      y = fpi::quot_chain(num, dr.x, (unsigned long long)__double_as_longlong(dr.y));
-      if (live) xp[2 * i] = y;
-      const double yo = other(y);
-      c1 = r ? yo : y;
-      c2 = r ? y : yo;
-      t = tn;
-      ad = adn;
-      l = ln;
-      dr = drn;
+    double c1 = 0.0, c2 = 0.0;
+    constexpr int kB = 3;
+    struct Fwd {
+      double t[kB];
+      double2 ad[kB], l[kB], dr[kB];
+    };
+    auto load = [&](Fwd& F, int i0) {
+#pragma unroll
+      for (int m = 0; m < kB; ++m) {
+        const int i = min(i0 + m, n1 - 1);
+        const double* f = fp + (size_t)i * kTbFac;
+        F.t[m] = xp[2 * i];
+        F.ad[m] = pair(f + 2 * r);
+        F.l[m] = pair(f + 4 + 2 * r);
+        F.dr[m] = pair(f + 12);
+      }
+    };
+    auto solve = [&](const Fwd& F, int i0) {
+#pragma unroll
+      for (int m = 0; m < kB; ++m) {
+        if (i0 + m >= n1) break;
+        const double v = __dsub_rn(F.t[m], __dadd_rn(__dmul_rn(F.l[m].x, c1), __dmul_rn(F.l[m].y, c2)));
+        const double vo = other(v);
+        const double num = __dadd_rn(__dmul_rn(F.ad[m].x, r ? vo : v), __dmul_rn(F.ad[m].y, r ? v : vo));
+        const double y = fpi::quot_chain(num, F.dr[m].x, (unsigned long long)__double_as_longlong(F.dr[m].y));
+        if (live) xp[2 * (i0 + m)] = y;
+        const double yo = other(y);
+        c1 = r ? yo : y;
+        c2 = r ? y : yo;
+      }
+    };
+    {
+      Fwd A, B;
+      load(A, 0);
+      for (int i0 = 0; i0 < n1; i0 += 2 * kB) {
+        load(B, i0 + kB);
+        solve(A, i0);
+        load(A, i0 + 2 * kB);
+        solve(B, i0 + kB);
+      }
     }
     __syncwarp();
-    double2 w = make_double2(0.0, 0.0);
-    if (n1 > 1) {
-      t = xp[2 * (n1 - 2)];
-      w = pair(fp + (size_t)(n1 - 2) * kTbFac + 8 + 2 * r);
-    }
-    for (int i = n1 - 2; i >= 0; --i) {
-      const int in = i > 0 ? i - 1 : 0;
-      const double tn = xp[2 * in];
-      const double2 wn = pair(fp + (size_t)in * kTbFac + 8 + 2 * r);
-      y = __dsub_rn(t, __dadd_rn(__dmul_rn(w.x, c1), __dmul_rn(w.y, c2)));
-      if (live) xp[2 * i] = y;
-      const double yo = other(y);
-      c1 = r ? yo : y;
-      c2 = r ? y : yo;
-      t = tn;
-      w = wn;
+    constexpr int kC = 6;
+    double ta[kC], tb[kC];
+    double2 wa[kC], wb[kC];
+    auto load_back = [&](double* t, double2* w, int m0) {  // rows n1-2-m0 downwards
+#pragma unroll
+      for (int m = 0; m < kC; ++m) {
+        const int i = max(n1 - 2 - (m0 + m), 0);
+        t[m] = xp[2 * i];
+        w[m] = pair(fp + (size_t)i * kTbFac + 8 + 2 * r);
+      }
+    };
+    auto solve_back = [&](const double* t, const double2* w, int m0) {
+#pragma unroll
+      for (int m = 0; m < kC; ++m) {
+        const int i = n1 - 2 - (m0 + m);
+        if (i < 0) break;
+        const double y = __dsub_rn(t[m], __dadd_rn(__dmul_rn(w[m].x, c1), __dmul_rn(w[m].y, c2)));
+        if (live) xp[2 * i] = y;
+        const double yo = other(y);
+        c1 = r ? yo : y;
+        c2 = r ? y : yo;
+      }
+    };
+    load_back(ta, wa, 0);
+    for (int m0 = 0; m0 < n1 - 1; m0 += 2 * kC) {
+      load_back(tb, wb, m0 + kC);
+      solve_back(ta, wa, m0);
+      load_back(ta, wa, m0 + 2 * kC);
+      solve_back(tb, wb, m0 + kC);
     }
   }
   __syncthreads();
@@ -976,7 +1044,7 @@ __global__ void __launch_bounds__(256) k_tb_planes(int tr, int n3, int k0, int k
       for (size_t e = tid; e < npc; e += nt) {
         restrict_2d_entry_of(n2, n1, [&](int i, int j) {
           const size_t q = (size_t)j * n1 + i;
-          return sub_v(ld_v(b + q * 2), level_entry(tr, 1, n2, n1, d, u1, l1, u2, l2, nullptr, nullptr, x, q));
+          return sub_v(ld_v(b + q * 2), level_entry_at(tr, 1, n2, n1, d, u1, l1, u2, l2, nullptr, nullptr, x, i, j, 0));
         }, bc, e);
         st_v(xc + e * 2, V2{0.0, 0.0});
       }
