@@ -665,7 +665,9 @@ __device__ __forceinline__ float pivot_quot(float x, float t, float r) { return 
 // (four operations a row) and then runs the recurrence (seven) pays all eleven
 // one after the other while the block's other warps wait.
 // kU entries a thread at a time: 4 where the operands come from L2, 1 for FP64
-// in shared memory (the FP64 unit is the limit there).
+// in shared memory (the FP64 unit is the limit there).  With 4 the FP64 products
+// run on the integer units (plane solves of 125x61: 413 instead of 426 us); a
+// resident level is too small to hide their latency (32x64: 181 instead of 176).
 template <typename T, bool kWrap, int kU>
 __device__ __forceinline__ void rhs_half(const Lev2T<T>& P, size_t mo, const T* b, T* x, int c, int fwd) {
   const int c1 = P.c1, c2 = P.c2, h = P.h, w = P.w;
@@ -704,7 +706,14 @@ __device__ __forceinline__ void rhs_half(const Lev2T<T>& P, size_t mo, const T* 
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      const T ml = cl[u] * xl[u], mr = cr[u] * xr[u];
+      T ml, mr;
+      if constexpr (sizeof(T) == 8 && kU > 1) {
+        ml = fpi::mul_rn(cl[u], xl[u]);
+        mr = fpi::mul_rn(cr[u], xr[u]);
+      } else {
+        ml = cl[u] * xl[u];
+        mr = cr[u] * xr[u];
+      }
       if (pos[u] >= 0) x[pos[u]] = fwd ? (bv[u] - ml) - mr : (bv[u] - mr) - ml;
     }
   }
@@ -974,7 +983,7 @@ __device__ __noinline__ void gs2d_res(const Lev2T<T>& G, int off, int gi) {
 // MatVecT_2D at a fine entry without branches, for the residual: a missing
 // neighbour's coefficient and value are 0 and add 0*0 (which can turn a -0 into
 // +0 only, lost in the sum of residuals that starts from +0)
-template <typename T, bool kWrap>
+template <typename T, bool kWrap, bool kInt>
 __device__ __forceinline__ T matvec2_flat(const Lev2T<T>& P, size_t mo, const T* x, int s, int i, int j, int k) {
   const int c1 = P.c1, c2 = P.c2, w = P.w, h = P.h, row = i * w;
   const bool up = i > 0, dn = i < c1 - 1, lf = j > 0, rt = j < c2 - 1;
@@ -984,8 +993,14 @@ __device__ __forceinline__ T matvec2_flat(const Lev2T<T>& P, size_t mo, const T*
   const T uzv = dn ? P.uz[mo + s] : (T)0, xd = dn ? x[s + w] : (T)0;
   const T lxv = lf ? P.lx[mo + sl] : (T)0, xl = lf ? x[sl] : (T)0;
   const T uxv = rt ? P.ux[mo + s] : (T)0, xr = rt ? x[sr] : (T)0;
-  T y = lzv * xu + dv * xc + uzv * xd;
-  y = y + lxv * xl + uxv * xr;
+  T y;
+  if constexpr (kInt) {
+    y = mulq(lzv, xu) + mulq(dv, xc) + mulq(uzv, xd);
+    y = y + mulq(lxv, xl) + mulq(uxv, xr);
+  } else {
+    y = lzv * xu + dv * xc + uzv * xd;
+    y = y + lxv * xl + uxv * xr;
+  }
   if (kWrap && P.wxl && (j == 0 || j == c2 - 1)) {  // periodic-Laplacian hierarchy: across the periodic x side
     const size_t kc = (size_t)k * c1;
     if (j == 0) y = y + P.wxl[kc + i] * x[row + slot(0, h, 0, c2 - 1)];
@@ -1013,7 +1028,7 @@ __device__ __forceinline__ void restrict2d(const Lev2T<T>& P, size_t mo, const T
       if (kU == 1 && !in) continue;
       const int i1c = in ? i1 : 2 * a, i2c = in ? i2 : 2 * bb;
       const int e = (int)slot(P.w, P.h, i1c, i2c);
-      const T d = b[e] - matvec2_flat<T, kWrap>(P, mo, x, e, i1c, i2c, k);
+      const T d = b[e] - matvec2_flat<T, kWrap, sizeof(T) == 8 && (kU > 1)>(P, mo, x, e, i1c, i2c, k);
       v = v + (in ? d : (T)0);
     }
     bq[s] = v;
