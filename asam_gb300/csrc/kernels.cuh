@@ -2293,11 +2293,10 @@ __global__ void k_axpy_sc(size_t len, const asam::KrylovScalars* sc, int sel, do
 // fused with the partial sums of (y, y) over the interior cells that the
 // residual norm test reads next.  One warp per padded x-row of one
 // component (every cell updated; the interior rows and cells counted).
-template <typename T>
+template <typename T, int kU>
 __global__ void __launch_bounds__(RED_BLOCK) k_axpy_dot(Dims d, int ncomp, const asam::KrylovScalars* sc, int sel,
                                                         double sign, const T* __restrict__ x, T* __restrict__ y,
                                                         double* __restrict__ partial) {
-  constexpr int kU = 4;  // cells a lane whose loads are in flight together
   const T a = (T)(sign * pick(sc, sel));
   const int NX = d.NX(), NY = d.NY();
   const long long rows_c = (long long)NY * d.NZ();
@@ -2316,9 +2315,10 @@ __global__ void __launch_bounds__(RED_BLOCK) k_axpy_dot(Dims d, int ncomp, const
       T v[kU], xv[kU];
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
-        const int i = min(i0 + 32 * u, NX - 1);
-        v[u] = y[base + i];
-        xv[u] = a != (T)0 ? x[base + i] : (T)0;
+        const int i = i0 + 32 * u;
+        const bool in = i < NX;
+        v[u] = in ? y[base + i] : (T)0;
+        xv[u] = in && a != (T)0 ? x[base + i] : (T)0;
       }
 #pragma unroll
       for (int u = 0; u < kU; ++u) {

@@ -35,6 +35,17 @@ void run_matvec(const asam::Launch& L, const asam::Dims& d, int ncomp, const TM*
   }
   k_matvec<TM, T><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, ncomp, val, x, y, plain);
 }
+// kU: cells a lane whose loads are in flight together.  A padded row is often a
+// few cells longer than a multiple of 128, and those took a pass of their own
+// (192x160x96 FP64 step 58.02 -> 57.77 ms, four refined members 92.1 -> 91.3).
+template <typename T>
+void run_axpy_dot(const asam::Launch& L, const asam::Dims& d, int ncomp, const asam::KrylovScalars* sc, int sel,
+                  double sign, const T* x, T* y, double* partial) {
+  if ((d.NX() + 159) / 160 < (d.NX() + 127) / 128)
+    k_axpy_dot<T, 5><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, sc, sel, sign, x, y, partial);
+  else
+    k_axpy_dot<T, 4><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, sc, sel, sign, x, y, partial);
+}
 // Rows per CTA of k_xline_rows: as many as fill one warp with recurrences (a
 // step of a warp costs the same for 10 threads as for 32; 256x256x128 with 10
 // components: 204 us at 3 rows, 228 at 4, 224 at 2), within the shared memory
@@ -283,7 +294,7 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
   }                                                                                                                \
   void launch_axpy_dot(const Launch& L, const Dims& d, int ncomp, KrylovScalars* sc, int sel, double sign,        \
                        const T* x, T* y, double* partial, int op) {                                                \
-    k_axpy_dot<T><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, sc, sel, sign, x, y, partial);                  \
+    run_axpy_dot(L, d, ncomp, sc, sel, sign, x, y, partial);                                                       \
     k_dot_final<<<1, RED_BLOCK, 0, L.stream>>>(partial, RED_GRID, sc, op, nullptr);                                \
     count_launches(2);                                                                                             \
   }                                                                                                                \
