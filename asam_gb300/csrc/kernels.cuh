@@ -38,22 +38,45 @@ __device__ __forceinline__ float div_rn(float x, float d, float rinv) {
   return __fmaf_rn(e, rinv, q0);
 }
 
-// a < b on the integer units (a comparison is an FP64 instruction of 64 cycles
-// as well): false for a quiet NaN a, as in 0/0 at a slope of -Eps; b a number
+// Comparisons on the integer units (a comparison is an FP64 instruction of 64
+// cycles as well): false for NaN on either side, the zeros alike.
+// |a| as an integer, negative for a negative number: ordered like the numbers,
+// NaN beyond the infinities
+constexpr long long kInfKey = 0x7ff0000000000000ll;
+__device__ __forceinline__ long long order_key(double a) {
+  const long long b = __double_as_longlong(a);
+  return b < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)b) : b;
+}
 __device__ __forceinline__ bool less(double a, double b) {
+  const long long x = order_key(a), y = order_key(b);
+  return x < y && x >= -kInfKey && y <= kInfKey;
+}
+__device__ __forceinline__ bool less(float a, float b) { return a < b; }
+// 1 for a positive a, 2 for a negative one, 0 for the zeros and NaN
+__device__ __forceinline__ unsigned direction(double a) {
+  const unsigned long long mag = (unsigned long long)__double_as_longlong(a) << 1;
+  return mag - 1 < 2 * (unsigned long long)kInfKey ? 1u + ((unsigned)__double2hiint(a) >> 31) : 0u;
+}
+__device__ __forceinline__ unsigned direction(float a) { return a > 0.0f ? 1u : a < 0.0f ? 2u : 0u; }
+// The same in fewer instructions where one kind of operand cannot come up.
+// b a number, a a number or a quiet NaN (0/0 at a slope of -Eps); a -0 counts as
+// below +0
+__device__ __forceinline__ bool less_num(double a, double b) {
   if (((unsigned)__double2hiint(a) & 0x7ff80000u) == 0x7ff80000u) return false;
   long long x = __double_as_longlong(a), y = __double_as_longlong(b);
   x ^= (long long)((unsigned long long)(x >> 63) >> 1);
   y ^= (long long)((unsigned long long)(y >> 63) >> 1);
   return x < y;
 }
-__device__ __forceinline__ bool less(float a, float b) { return a < b; }
-__device__ __forceinline__ bool positive(double a) { return __double_as_longlong(a) > 0; }
-__device__ __forceinline__ bool negative(double a) {
+__device__ __forceinline__ bool less_num(float a, float b) { return a < b; }
+// a a number
+__device__ __forceinline__ bool negative_num(double a) {
   return (unsigned long long)__double_as_longlong(a) > 0x8000000000000000ull;
 }
-__device__ __forceinline__ bool positive(float a) { return a > 0.0f; }
-__device__ __forceinline__ bool negative(float a) { return a < 0.0f; }
+__device__ __forceinline__ bool negative_num(float a) { return a < 0.0f; }
+// a not zero, the sign of a NaN of no matter
+__device__ __forceinline__ bool positive_num(double a) { return __double_as_longlong(a) > 0; }
+__device__ __forceinline__ bool positive_num(float a) { return a > 0.0f; }
 
 // RN(x + Eps): from |x| = 2^-45 on Eps is less than half a unit in the last
 // place (of the next smaller number, too), so the sum is x
@@ -89,9 +112,9 @@ __device__ __forceinline__ T k2f(T hL, T hC, T hR) {
 template <typename T>
 __device__ __forceinline__ T koren(T r, T k1, T k2) {
   T a = k1 * r + k2;
-  T m = less(a, (T)1) ? a : (T)1;
-  m = less(r, m) ? r : m;
-  return negative(m) ? (T)0 : m;
+  T m = less_num(a, (T)1) ? a : (T)1;  // a NaN is not taken: m is a number
+  m = less_num(r, m) ? r : m;
+  return negative_num(m) ? (T)0 : m;
 }
 
 using asam::GeomT;
@@ -149,8 +172,9 @@ __global__ void k_face_coef(Dims d, GeomT<T> g, T* __restrict__ coef, unsigned c
     const int s = AXIS == 0 ? i : (AXIS == 1 ? j : k);
     const int smax = AXIS == 0 ? nx : (AXIS == 1 ? ny : nz);
     int orient = 0;
-    if (positive(vel) && s >= 1) orient = 1;           // upwind = left cell, its right face
-    else if (negative(vel) && s + 1 <= smax) orient = -1;  // upwind = right cell, its left face
+    const unsigned flow = direction(vel);
+    if (flow == 1 && s >= 1) orient = 1;                // upwind = left cell, its right face
+    else if (flow == 2 && s + 1 <= smax) orient = -1;  // upwind = right cell, its left face
     T c0 = (T)0, c1 = (T)0, c2 = (T)0, c3 = (T)0;
     unsigned char m = 0;
     if (orient != 0) {
@@ -220,7 +244,7 @@ __global__ void k_face_flux(Dims d, GeomT<T> g, int ncomp, const T* __restrict__
       for (int ic = 0; ic < ncomp; ++ic) gout[ic * nface + f] = (T)0;
       continue;
     }
-    const bool right = positive(pref_s);
+    const bool right = positive_num(pref_s);
     const T pref = right ? pref_s : -pref_s;
     const T ratio = coef[nface + f], k1 = coef[2 * nface + f], k2 = coef[3 * nface + f];
     const bool unit = ratio == (T)1;
@@ -426,26 +450,25 @@ __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict
       const bool exS = d.per_y && j == 1, exN = d.per_y && j == ny;
       const bool exB = d.per_z && k == 1, exT = d.per_z && k == nz;
       // directions of the six faces' flow, tested once for all components
-      const bool puL = positive(uL), nuL = negative(uL), puR = positive(uR), nuR = negative(uR);
-      const bool pvL = positive(vL), nvL = negative(vL), pvR = positive(vR), nvR = negative(vR);
-      const bool pwL = positive(wL), nwL = negative(wL), pwR = positive(wR), nwR = negative(wR);
+      const unsigned m = direction(uL) | direction(uR) << 2 | direction(vL) << 4 | direction(vR) << 6 |
+                         direction(wL) << 8 | direction(wR) << 10;
       for (int ic = 0; ic < ncomp; ++ic) {
         const T* GX = gx + ic * nfx;
         const T* GY = gy + ic * nfy;
         const T* GZ = gz + ic * nfz;
         T a = (T)0;
-        if (pwL) a = a + GZ[fzL];  // FluxZR of the cell below
-        if (pvL) a = a + GY[fyL];  // FluxYR of the cell south
-        if (puL) a = a + GX[fxL];  // FluxXR of the cell west
-        if (nuL) a = a - GX[fxL];  // own x-left
-        if (puR) a = a - GX[fxR];  // own x-right
-        if (nvL) a = a - GY[fyL];
-        if (pvR) a = a - GY[fyR];
-        if (nwL) a = a - GZ[fzL];
-        if (pwR) a = a - GZ[fzR];
-        if (nuR) a = a + GX[fxR];  // FluxXL of the cell east
-        if (nvR) a = a + GY[fyR];
-        if (nwR) a = a + GZ[fzR];
+        if (m & 256) a = a + GZ[fzL];  // FluxZR of the cell below
+        if (m & 16) a = a + GY[fyL];  // FluxYR of the cell south
+        if (m & 1) a = a + GX[fxL];  // FluxXR of the cell west
+        if (m & 2) a = a - GX[fxL];  // own x-left
+        if (m & 4) a = a - GX[fxR];  // own x-right
+        if (m & 32) a = a - GY[fyL];
+        if (m & 64) a = a - GY[fyR];
+        if (m & 512) a = a - GZ[fzL];
+        if (m & 1024) a = a - GZ[fzR];
+        if (m & 8) a = a + GX[fxR];  // FluxXL of the cell east
+        if (m & 128) a = a + GY[fyR];
+        if (m & 2048) a = a + GZ[fzR];
         if (wl.c) {  // inflow through the outer walls' faces, W, E, S, N, B, T (:975-1044)
           const T* cc = wl.c + ic * n;
           const T half = (T)0.5;
@@ -678,10 +701,8 @@ __global__ void __launch_bounds__(256, kMom || kDiff ? 2 : 4) k_flux_plain(Dims 
     const size_t dz = (size_t)nx * ny;
     const T uL = g.uf[fx], uR = g.uf[fx + 1], vL = g.vf[fy], vR = g.vf[fy + nx], wL = g.wf[fz], wR = g.wf[fz + dz];
     // directions of the six faces' flow, tested once for all components
-    const unsigned m = (unsigned)positive(uL) | (unsigned)negative(uL) << 1 | (unsigned)positive(uR) << 2 |
-                       (unsigned)negative(uR) << 3 | (unsigned)positive(vL) << 4 | (unsigned)negative(vL) << 5 |
-                       (unsigned)positive(vR) << 6 | (unsigned)negative(vR) << 7 | (unsigned)positive(wL) << 8 |
-                       (unsigned)negative(wL) << 9 | (unsigned)positive(wR) << 10 | (unsigned)negative(wR) << 11;
+    const unsigned m = direction(uL) | direction(uR) << 2 | direction(vL) << 4 | direction(vR) << 6 |
+                       direction(wL) << 8 | direction(wR) << 10;
 #pragma unroll 2
     for (int ic = 0; ic < ncomp; ++ic) {
       const T* GX = gx + ic * nfx + fx;

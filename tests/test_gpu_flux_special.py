@@ -1,0 +1,54 @@
+"""NaN and signed zeros in the operands that the flux kernels only compare: the
+direction of the flow over a face, and the volumes on its two sides."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+from asam_gb300 import TransportBlock
+from asam_gb300 import geometry as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(periodic):
+    nx, ny, nz = 7, 6, 5
+    rng = np.random.default_rng(5 + periodic)
+    grid = G.Grid(nx, ny, nz, 100.0, 130.0, G.stretched_levels(nz, 50.0, 90.0), periodic, periodic, False)
+    geo = G.cut_cell_geometry(grid, rng.uniform(0.0, 60.0, (ny, nx)))
+    vel = [np.array(v) for v in G.closed_face_velocity(geo, 3.0, seed=1)]
+    c = oracle.Oracle(geo).exchange_cell(rng.uniform(0.5, 1.5, (3,) + grid.pshape))
+    return rng, geo, vel, c
+
+
+def _fcn(geo, vel, c, precision):
+    with TransportBlock(geo, c.shape[0], precision=precision) as blk:
+        blk.set_velocity(*vel)
+        return blk.Fcn(c)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refined"])
+@pytest.mark.parametrize("nan", [np.nan, -np.nan])
+@pytest.mark.parametrize("periodic", [True, False])
+def test_face_with_a_nan_velocity_has_no_flux(built_lib, periodic, nan, precision):
+    """NaN flows in neither direction, so the faces give what resting ones give."""
+    rng, geo, vel, c = _case(periodic)
+    rest = [v.copy() for v in vel]
+    for v, r in zip(vel, rest):
+        inner = v[1:-1, 1:-1, 1:-1]  # off the walls, whose inflow is not a comparison
+        hit = rng.random(inner.shape) < 0.2
+        inner[hit] = nan
+        r[1:-1, 1:-1, 1:-1][hit] = 0.0
+    np.testing.assert_array_equal(_fcn(geo, vel, c, precision), _fcn(geo, rest, c, precision))
+
+
+@pytest.mark.parametrize("value", [np.nan, -np.nan, -0.0, 0.0])
+@pytest.mark.parametrize("periodic", [True, False])
+def test_volumes_that_compare_false(built_lib, periodic, value):
+    """Neither a NaN volume nor a negative zero next to zero is the smaller one."""
+    rng, geo, vel, c = _case(periodic)
+    inner = geo.volc[1:-1, 1:-1, 1:-1]
+    inner[rng.random(inner.shape) < 0.2] = 0.0
+    inner[rng.random(inner.shape) < 0.2] = value
+    np.testing.assert_array_equal(_fcn(geo, vel, c, "fp64"), oracle.Oracle(geo).fcn(c, vel))
