@@ -846,20 +846,31 @@ __global__ void k_div(Dims d, GeomT<T> g, T* __restrict__ rhs) {
 // accumulation order.
 // ---------------------------------------------------------------------------
 // Half*(ABS(u)+/-u)*F/V/(Rho+Eps).  Half*(ABS(u)+/-u) is |u| for one sign of u
-// and 0 for the other, where the term is 0; the product and both quotients (one
-// by a divisor of the whole column) run on the integer units.  All of it on the FP64
-// unit, twelve terms a cell, was what the kernel took its time for (128x128x64:
-// 327 us, now 149).
-__device__ __forceinline__ bool not_positive(double a) {  // false for NaN
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-  return b == 0 || (b >= 0x8000000000000000ull && b <= 0xfff0000000000000ull);
+// and 0 for the other, where the term is 0 (for finite F, and V and Rho+Eps other
+// than 0, infinity and NaN: operands beyond that take the whole expression); the
+// product and both quotients (one by a divisor of the whole column) run on the
+// integer units.  All of it on the FP64 unit, twelve terms a cell, was what the
+// kernel took its time for (128x128x64: 327 us, now 158, nine of them for the
+// tests of F, V and Rho+Eps).
+static __device__ __noinline__ double jac_term_special(double u, double F, double Vden, double rhoe) {
+  return __ddiv_rn(__ddiv_rn(__dmul_rn(__dmul_rn(0.5, __dadd_rn(fabs(u), u)), F), Vden), rhoe);
 }
-__device__ __forceinline__ bool not_positive(float a) { return a <= 0.0f; }
-template <typename T, typename R>
-__device__ __forceinline__ T jac_term(T vel, bool plus, T F, T Vden, T rhoe, R rrhoe) {
-  const T u = plus ? vel : -vel;
-  if (not_positive(u)) return (T)0;
-  return quot_i(div_i(mul_i(u, F), Vden), rhoe, rrhoe);
+template <typename R>
+__device__ __forceinline__ double jac_term(double vel, bool plus, double F, double Vden, double rhoe, R rrhoe) {
+  const double u = plus ? vel : -vel;
+  // below 2^1023, where |u| + u is finite
+  constexpr unsigned long long kTop = 0x7fe0000000000000ull;
+  if ((unsigned long long)__double_as_longlong(u) - 1 < kTop - 1)
+    return quot_i(div_i(mul_i(u, F), Vden), rhoe, rrhoe);
+  if (((unsigned)__double2hiint(u) & 0x7fffffffu) < (unsigned)(kTop >> 32) && fpi::finite((unsigned)__double2hiint(F)) &&
+      fpi::in_range((unsigned)__double2hiint(Vden)) && fpi::in_range((unsigned)__double2hiint(rhoe)))
+    return 0.0;
+  return jac_term_special(u, F, Vden, rhoe);
+}
+template <typename R>
+__device__ __forceinline__ float jac_term(float vel, bool plus, float F, float Vden, float rhoe, R rrhoe) {
+  const float u = plus ? vel : -vel;
+  return quot_i(div_i(mul_i(0.5f * (fabsf(u) + u), F), Vden), rhoe, rrhoe);
 }
 
 template <typename T>

@@ -1,12 +1,13 @@
-"""NaN and signed zeros in the operands that the flux kernels only compare: the
-direction of the flow over a face, and the volumes on its two sides."""
+"""NaN, infinities, signed zeros and the ends of the range in the operands that
+the flux and matrix kernels compare or shortcut: velocities, volumes, areas and
+densities."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
 import oracle
-from asam_gb300 import TransportBlock
+from asam_gb300 import TransportBlock, ros_coeffs
 from asam_gb300 import geometry as G
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +53,23 @@ def test_volumes_that_compare_false(built_lib, periodic, value):
     inner[rng.random(inner.shape) < 0.2] = 0.0
     inner[rng.random(inner.shape) < 0.2] = value
     np.testing.assert_array_equal(_fcn(geo, vel, c, "fp64"), oracle.Oracle(geo).fcn(c, vel))
+
+
+@pytest.mark.parametrize("where", ["velocity", "density", "area", "volume"])
+@pytest.mark.parametrize("periodic", [True, False])
+def test_matrix_of_special_operands(built_lib, periodic, where):
+    """The terms that the direction of the flow makes 0 are so only for
+    ordinary areas, volumes and densities: 0*inf, 0/0 and NaN elsewhere."""
+    rng, geo, vel, c = _case(periodic)
+    values = [np.nan, np.inf, -np.inf, 0.0, -0.0, 1.5e308, -1.5e308, 5e-324, -1e-30, -1.0]
+    for a in {"velocity": vel, "density": [c[0]], "area": [geo.fu, geo.fv, geo.fw], "volume": [geo.volc]}[where]:
+        hit = rng.random(a.shape) < 0.2
+        a[hit] = rng.choice(values, hit.sum())
+    for v in vel if where != "velocity" else []:  # both signs and rest
+        v[...] = rng.choice([0.0, 1.0, -1.0], v.shape) * rng.uniform(0.5, 2.0, v.shape)
+    with TransportBlock(geo, c.shape[0]) as blk:
+        blk.set_velocity(*vel)
+        blk.Jac(c, 2.0)
+        got = blk.jac_matrix()
+    want = oracle.Oracle(geo).jac(c[0], vel, ros_coeffs("RosRK3")[1], 2.0)
+    np.testing.assert_array_equal(got, want)
