@@ -310,12 +310,17 @@ __global__ void k_face_flux(Dims d, GeomT<T> g, int ncomp, const T* __restrict__
 // interior face between padded cells (i,j,k) and their +1 neighbour along
 // axis, with DUU = F/(F+Eps) of IniJacAccGrav (MULTI/JacAccGrav_Mod.f90:297):
 //   DUU*F/(F+Eps)*(p(+1)-p)/(Metr*(d(+1)+d+Eps)), evaluated left to right.
-// An area from 2^-45 on is unchanged by Eps, both ratios are 1 and the products
-// with them exact.
+// A finite area from 2^-45 on is unchanged by Eps, both ratios are 1 and the
+// products with them exact.
+__device__ __forceinline__ bool plain_area(double F) {
+  constexpr unsigned kMin = (1023u - 45u) << 20;
+  return (unsigned)__double2hiint(F) - kMin < 0x7ff00000u - kMin;
+}
+__device__ __forceinline__ bool plain_area(float F) { return add_eps(F) == F && F > 0.0f && F <= 3.4e38f; }
 template <typename T>
 __device__ __forceinline__ T pgrad_ratio(T F, T dp, T den) {
+  if (plain_area(F)) return div_i(dp, den);
   const T Fe = add_eps(F);
-  if (Fe == F && F > (T)0) return div_i(dp, den);
   const T du = div_i(F, Fe);
   return div_i(div_i(du * F, Fe) * dp, den);
 }
@@ -368,8 +373,8 @@ __device__ __forceinline__ T buoy_rho_face(const Dims& d, const GeomT<T>& g, con
   const T e = eps_t<T>();
   const T F = g.fw[d.FW(i, j, k)];
   const T s = ms.dz[k - 1] * ms.rho[d.P(i, j, k)] + ms.dz[k] * ms.rho[d.P(i, j, k + 1)];
-  const T Fe = add_eps(F), den = ms.dz[k - 1] + ms.dz[k] + e;
-  return Fe == F && F > (T)0 ? div_i(s, den) : div_i(div_i(F, Fe) * s, den);
+  const T den = ms.dz[k - 1] + ms.dz[k] + e;
+  return plain_area(F) ? div_i(s, den) : div_i(div_i(F, add_eps(F)) * s, den);
 }
 
 // Gather of the face fluxes into the cell right-hand side in the exact order

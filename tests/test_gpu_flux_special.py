@@ -73,3 +73,31 @@ def test_matrix_of_special_operands(built_lib, periodic, where):
         got = blk.jac_matrix()
     want = oracle.Oracle(geo).jac(c[0], vel, ros_coeffs("RosRK3")[1], 2.0)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 0.0, 2.0 ** -46, 2.0 ** -45, -1.0, 1e-30, 5e-324])
+def test_momentum_sources_of_special_areas(built_lib, value):
+    """F/(F+Eps) is 1 for finite areas from 2^-45 on only."""
+    geo, vel, st, pos, (dx, dy, dz), bound = G.hill_dyn_case(7, 6, 5, seed=3)
+    rng = np.random.default_rng(3)
+    vel = [np.zeros_like(v) for v in vel]  # the sources alone
+    for a in (geo.fu, geo.fv, geo.fw):
+        a[...] = rng.uniform(0.5, 2.0, a.shape)
+        a[rng.random(a.shape) < 0.2] = value
+    pre = rng.uniform(8e4, 1e5, geo.grid.pshape)
+    with TransportBlock(geo, st.c.shape[0]) as blk:
+        blk.set_velocity(*vel)
+        blk.proj_setup(dx, dy, dz)
+        blk.dyn_setup(pos["th"], pos["mom"], rv_pos=pos.get("qv", -1), bound_cells=bound)
+        got = blk.FcnMet(st.c, pre)
+    if np.isfinite(value):
+        want = oracle.Oracle(geo).fcn_dyn(st.c, vel, pre, pos["mom"], dx, dy, dz)
+        for q in pos["mom"]:
+            np.testing.assert_array_equal(got[q], want[q])
+        return
+    # (the oracle's flux over such a face is 0*inf as well; a resting face has none here)
+    nx, ny, nz = 7, 6, 5
+    for comp, F in ((1, geo.fu[:, :, 2:nx + 1]), (3, geo.fv[:, 2:ny + 1]), (5, geo.fw[2:nz + 1])):
+        g = got[pos["mom"][comp]][1:F.shape[0] + 1, 1:F.shape[1] + 1, 1:F.shape[2] + 1]
+        with np.errstate(invalid="ignore"):
+            np.testing.assert_array_equal(np.isnan(g), np.isnan(F / (F + 1e-30)))
