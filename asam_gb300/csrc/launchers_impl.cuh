@@ -162,11 +162,9 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
     }                                                                                                              \
     const dim3 grid(ntx, ntz, nsweep * gs_ngroups(ncomp, group));                                                  \
     const size_t smem = (staged ? gs_smem_elems(group) : gs_tile_elems(std::min(group, ncomp))) * sizeof(T);       \
-    thread_local size_t smem_set = 0;                                                                              \
-    if (staged && smem > smem_set) {                                                                               \
-      cudaFuncSetAttribute(k_gs_pipe_smem<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
-      smem_set = smem;                                                                                             \
-    }                                                                                                              \
+    if (staged) /* the same value whatever the call, as below */                                                   \
+      cudaFuncSetAttribute(k_gs_pipe_smem<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,                     \
+                           (int)(gs_smem_elems(kMaxComp) * sizeof(T)));                                            \
     if (!staged) /* the same value whatever the call: threads with other component counts launch it too */         \
       for (auto* f : {k_gs_tile<TM, T, false>, k_gs_tile<TM, T, true>})                                            \
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,                                       \
@@ -191,11 +189,13 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
     const int ntz = (d.NZ() + GS_TZ - 1) / GS_TZ;                                                                  \
     const int threads = (GS_TY * GS_TZ * sch.group + 31) / 32 * 32;                                                \
     const size_t smem = gs_smem_elems(sch.group) * sizeof(T);                                                      \
-    /* per host thread: the attribute and the occupancy of the last shared-memory size */                       \
+    /* the attribute belongs to the kernel, which host threads with other group sizes launch too: one value for    \
+       all; per host thread the occupancy of the last shared-memory size */                                        \
+    cudaFuncSetAttribute(k_gs_persist<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,                         \
+                         (int)(gs_smem_elems(kMaxComp) * sizeof(T)));                                              \
     thread_local size_t smem_set = 0;                                                                              \
     thread_local int per_sm = 0;                                                                                   \
-    if (smem != smem_set) { /* smem determines threads */                                                         \
-      cudaFuncSetAttribute(k_gs_persist<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+    if (smem != smem_set) { /* smem determines threads */                                                          \
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gs_persist<TM, T>, threads, smem);                  \
       if (per_sm < 1) per_sm = 1;                                                                                  \
       smem_set = smem;                                                                                             \
