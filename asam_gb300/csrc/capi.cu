@@ -537,7 +537,10 @@ int bicgstab_refined(asam_ctx* h, double* x, const double* b, int* maxiter, doub
     rc = bicgstab_dev<float>(h, h->val32, h->x32, nullptr, &it, &tin, h->w32, true, true);
     // an inner breakdown or iteration limit still leaves a usable correction:
     // the outer FP64 residual decides
-    if (rc != kOk && rc != kNotConverged && rc != kBreakdown) return rc;
+    if (rc != kOk && rc != kNotConverged && rc != kBreakdown) {
+      if (outer == 0 && x_is_zero) cudaMemsetAsync(x, 0, len * sizeof(double), L.stream);  // not written yet
+      return rc;
+    }
     total_inner += it < 0 ? -it : (it > h->cfg.bicgstab_maxiter ? it / 2 : it);
     if (outer == 0 && x_is_zero)
       launch_set_f32_to_f64(L, len, h->x32, rnorm, x);
