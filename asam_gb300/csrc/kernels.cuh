@@ -389,7 +389,7 @@ __device__ __forceinline__ T buoy_rho_face(const Dims& d, const GeomT<T>& g, con
 // The cells one in from every side of the block have none of the side terms:
 // k_flux_plain takes them (half of the registers), and this kernel, whose
 // 170 registers leave an SM eight warps, the halo cells and the outermost
-// interior ones, enumerated without gaps.
+// interior ones, enumerated without gaps; all: it takes every cell.
 //
 // Halo and outermost interior cells of a block with at least two cells along
 // every axis: the planes k = 0, 1, nz, nz+1, then of the other planes the rows
@@ -424,14 +424,13 @@ __device__ __forceinline__ void flux_edge_cell(const Dims& d, size_t q, int& i, 
 template <typename T, bool kMom = false, bool kDiff = false>
 __global__ void k_flux_gather(Dims d, GeomT<T> g, int ncomp, const T* __restrict__ gx, const T* __restrict__ gy,
                               const T* __restrict__ gz, const T* __restrict__ rvol, T* __restrict__ f,
-                              MomSrc<T> ms, DiffSrc<T> df = DiffSrc<T>{}, WallIn<T> wl = WallIn<T>{}) {
+                              MomSrc<T> ms, DiffSrc<T> df, WallIn<T> wl, bool all) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const int NX = d.NX(), NY = d.NY(), NZ = d.NZ();
   const size_t n = d.npad();
   const size_t nfx = (size_t)(nx + 1) * ny * nz, nfy = (size_t)nx * (ny + 1) * nz, nfz = (size_t)nx * ny * (nz + 1);
   const T e = eps_t<T>();
-  const bool all = flux_all_edges(d);
-  const size_t nedge = flux_edges(d);
+  const size_t nedge = all ? n : flux_edges(d);
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nedge; q += (size_t)gridDim.x * blockDim.x) {
     int i, j, k;
     if (all)
