@@ -1327,12 +1327,47 @@ struct asam_tri_tb_hier {
   double* du3[32] = {};
   double* dl3[32] = {};
   double* mem = nullptr;
+  double* zmem = nullptr;  // the zebra order's factors and right-hand sides, from its first use on
   double* t = nullptr;
   Scratch sc{nullptr, nullptr};
   ~asam_tri_tb_hier() {
     if (mem) cudaFree(mem);
+    if (zmem) cudaFree(zmem);
   }
 };
+
+// What the zebra order needs beside the hierarchy: the elimination factors of
+// every plane level (kTbFac doubles an entry, where the hierarchy has some 30)
+// and every plane's right-hand side.  A hierarchy that stays in the sequential
+// order, the default, is not charged for them (12x24x20, 3 levels: created in
+// 744 us, 876 with the factors).
+static int zebra_prepare(asam_tri_tb_hier* h) {
+  if (h->zmem) return ASAM_OK;
+  auto entries = [](const PlaneLevel& P, int n3) { return (size_t)n3 * P.n2 * P.n1; };
+  size_t tot = 2 * entries(h->pl[0][0], h->n3s[0]);
+  for (int L = 0; L < h->nlev3; ++L)
+    for (int m = 0; m < h->nlev2s[L]; ++m) tot += entries(h->pl[L][m], h->n3s[L]) * kTbFac;
+  double* z = nullptr;
+  TCU(cudaMalloc((void**)&z, tot * sizeof(double)));
+  h->zmem = z;
+  h->sc.tall = z;
+  z += 2 * entries(h->pl[0][0], h->n3s[0]);
+  for (int L = 0; L < h->nlev3; ++L)
+    for (int m = 0; m < h->nlev2s[L]; ++m) {
+      PlaneLevel& P = h->pl[L][m];
+      const size_t nline = (size_t)h->n3s[L] * P.n2;
+      P.fac = z;
+      z += entries(P, h->n3s[L]) * kTbFac;
+      k_tb_factor<<<(unsigned)((nline + 63) / 64), 64>>>(nline, P.n1, P.a[0], P.a[1], P.a[2], P.fac);
+      asam::count_launches(1);
+    }
+  const cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) return ASAM_OK;
+  cudaFree(h->zmem);
+  h->zmem = nullptr;
+  asam::set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
+  return ASAM_CUDA_ERROR;
+}
 
 extern "C" {
 
@@ -1660,24 +1695,20 @@ int asam_tri_tb_hier_create(int variant, int ref_level, int n3, int n2, int n1, 
     h->nlev2s[L] = ref_level - L;
     for (int m = 0; m < h->nlev2s[L]; ++m)
       tot += plane_block_len(h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m)) +
-             3 * plane_vec_len(h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m)) +
-             (size_t)h->n3s[L] * cdiv(n2, L + m) * cdiv(n1, L + m) * kTbFac;
+             3 * plane_vec_len(h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m));
     tot += 2 * (size_t)(h->n3s[L] - 1) * h->n2s[L] * h->n1s[L] * 4;
   }
   const size_t npl = (size_t)n2 * n1, nc = (size_t)n3 * npl;
   const size_t nz = (size_t)n3 * n2 * (n1 + 1), nx = (size_t)n3 * (n2 + 1) * n1, ny = (size_t)(n3 + 1) * npl;
   const size_t nt = (size_t)n1 * 2, nw = (size_t)(n1 > 1 ? n1 - 1 : 1) * 4;
   const size_t fields = 4 * (nz + nx + ny) + 3 * nc;  // the finest fields, and room for one coarsening of them
-  TCU(cudaMalloc((void**)&h->mem, (tot + npl * 2 + nt + nw + nc * 2) * sizeof(double)));
+  TCU(cudaMalloc((void**)&h->mem, (tot + npl * 2 + nt + nw) * sizeof(double)));
   DevBufs work;
   TCU(cudaMalloc((void**)&work.p[0], 2 * fields * sizeof(double)));
   double* cur = h->mem;
   for (int L = 0; L < ref_level; ++L) {
-    for (int m = 0; m < h->nlev2s[L]; ++m) {
+    for (int m = 0; m < h->nlev2s[L]; ++m)
       TCU(stage_plane_level(h->pl[L][m], h->n3s[L], cdiv(n2, L + m), cdiv(n1, L + m), nullptr, cur));
-      h->pl[L][m].fac = cur;
-      cur += (size_t)h->n3s[L] * cdiv(n2, L + m) * cdiv(n1, L + m) * kTbFac;
-    }
     const size_t ncp = (size_t)(h->n3s[L] - 1) * h->n2s[L] * h->n1s[L] * 4;
     h->du3[L] = ncp ? cur : nullptr;
     h->dl3[L] = ncp ? cur + ncp : nullptr;
@@ -1685,7 +1716,6 @@ int asam_tri_tb_hier_create(int variant, int ref_level, int n3, int n2, int n1, 
   }
   h->t = cur;
   h->sc = Scratch{cur + npl * 2, cur + npl * 2 + nt};
-  h->sc.tall = cur + npl * 2 + nt + nw;
   // the finest fields on the device
   TbFields g;
   double* fp = work.p[0];
@@ -1734,9 +1764,7 @@ int asam_tri_tb_hier_create(int variant, int ref_level, int n3, int n2, int n1, 
                                                                    const_cast<double*>(P.a[0]),
                                                                    couple ? h->du3[L3] : nullptr,
                                                                    couple ? h->dl3[L3] : nullptr);
-      const size_t nline = (size_t)c3 * c2;
-      k_tb_factor<<<(unsigned)((nline + 63) / 64), 64>>>(nline, c1, P.a[0], P.a[1], P.a[2], P.fac);
-      launches += 4;
+      launches += 3;
       TCU(cudaGetLastError());
     }
   TCU(cudaDeviceSynchronize());
@@ -1787,6 +1815,8 @@ int asam_tri_tb_hier_set_zebra(asam_tri_tb_hier* h, int on) {
     asam::set_last_error("asam_tri_tb_hier_set_zebra: bad argument", __FILE__, __LINE__);
     return ASAM_BAD_ARG;
   }
+  if (on)
+    if (const int rc = zebra_prepare(h)) return rc;
   h->zebra = on != 0;
   return ASAM_OK;
 }

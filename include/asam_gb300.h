@@ -719,7 +719,8 @@ int asam_tri_tb_hier_vcycle(asam_tri_tb_hier *h, const double *b, double *x, int
  * backward, all lines (planes) of one parity at once, then the reference's
  * closing solves; every relaxation is the reference's arithmetic, only the
  * order of the lines and planes differs.  0 (the default): the reference's
- * sequential order. */
+ * sequential order.  The first call with on != 0 allocates and computes the
+ * lines' elimination factors, and fails if the device memory does not suffice. */
 int asam_tri_tb_hier_set_zebra(asam_tri_tb_hier *h, int on);
 void asam_tri_tb_hier_destroy(asam_tri_tb_hier *h);
 
