@@ -2095,8 +2095,8 @@ struct PlanePlan {
   size_t smem;
 };
 template <typename T>
-PlanePlan plane_plan(const Lev3T<T>& A, int np) {
-  const size_t cap = np > 152 ? kPlaneSmem2 : kPlaneSmem1;
+PlanePlan plane_plan(const Lev3T<T>& A, int np, int sm_count) {
+  const size_t cap = np > sm_count ? kPlaneSmem2 : kPlaneSmem1;
   size_t used = 0;
   int mr = A.nl;
   while (mr > 0) {
@@ -2107,7 +2107,7 @@ PlanePlan plane_plan(const Lev3T<T>& A, int np) {
     used += add;
     --mr;
   }
-  return PlanePlan{mr, np > 152 || A.pl[0].ps < 4096 ? kPlaneBlock : 2 * kPlaneBlock, used};
+  return PlanePlan{mr, np > sm_count || A.pl[0].ps < 4096 ? kPlaneBlock : 2 * kPlaneBlock, used};
 }
 
 // Solve_3D from a zero start on level 0 (VCycleCG's MatrixT branch): lv[0].b
@@ -2126,7 +2126,7 @@ void vcycle_run(asam_ctx* h, std::vector<Lev3T<T>>& lv, Lev3T<T>* d_lv, int gi2,
     auto half = [&](int c, int fwd) {
       const int np = (A.m3 - c + 1) / 2;
       if (np <= 0) return;
-      const PlanePlan pp = plane_plan(A, np);
+      const PlanePlan pp = plane_plan(A, np, h->L.sm_count);
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(np);
       cfg.blockDim = dim3(pp.threads);
