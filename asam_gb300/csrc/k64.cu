@@ -20,13 +20,9 @@ __global__ void k_add_f2d(size_t len, const float* __restrict__ x, double s, dou
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x)
     y[q] = y[q] + fpi::mul_rn(s, fpi::widen(x[q]));
 }
-// y = (float)(s * x): the residual handed to the FP32 inner solver, scaled to
-// unit norm so that neither tiny nor huge residuals leave the FP32 range
-__global__ void k_cvt_d2f_scaled(size_t len, const double* __restrict__ x, double s, float* __restrict__ y) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x)
-    y[q] = fpi::narrow(fpi::mul_rn(s, x[q]));
-}
-// the same into the inner solver's residual, shadow residual and search direction
+// (float)(s * x): the residual handed to the FP32 inner solver, scaled to
+// unit norm so that neither tiny nor huge residuals leave the FP32 range; into
+// the inner solver's residual, shadow residual and search direction
 __global__ void k_cvt_d2f_scaled3(size_t len, const double* __restrict__ x, double s, float* __restrict__ y0,
                                   float* __restrict__ y1, float* __restrict__ y2) {
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x) {
@@ -119,10 +115,6 @@ void launch_convert_f64_to_f32(const Launch& L, size_t len, const double* x, flo
 }
 void launch_add_f32_to_f64(const Launch& L, size_t len, const float* x, double s, double* y) {
   k_add_f2d<<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, x, s, y);
-  count_launches(1);
-}
-void launch_convert_f64_to_f32_scaled(const Launch& L, size_t len, const double* x, double s, float* y) {
-  k_cvt_d2f_scaled<<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, x, s, y);
   count_launches(1);
 }
 void launch_convert_f64_to_f32_scaled3(const Launch& L, size_t len, const double* x, double s, float* y0, float* y1,

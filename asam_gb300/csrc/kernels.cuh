@@ -1181,21 +1181,14 @@ constexpr int kGsComp = kGsLines * kGsPitch + 2 * 4 * kGsTx + 16;
 constexpr int kGsCoef = 5 * kGsLines * kGsPitch;  // l0, l1, l2, diagonal, reciprocal
 inline size_t gs_tile_elems(int ncomp) { return (size_t)kGsCoef + (size_t)ncomp * kGsComp; }
 
-__device__ __forceinline__ double gs_mul(double a, double b) { return fpi::mul_rn(a, b); }
-__device__ __forceinline__ float gs_mul(float a, float b) { return a * b; }
-__device__ __forceinline__ double gs_quot(double t, double d, double r) {
-  return fpi::quot_chain(t, d, (unsigned long long)__double_as_longlong(r));
-}
-__device__ __forceinline__ float gs_quot(float t, float d, float r) { return div_rn(t, d, r); }
-
-template <typename TM, typename T, bool kIntL>
-__global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int group, const TM* __restrict__ val,
-                                                      const T* __restrict__ b, T* buf_last, T* buf_other, int tau,
+template <bool kIntL>
+__global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int group, const double* __restrict__ val,
+                                                      const double* __restrict__ b, double* buf_last, double* buf_other, int tau,
                                                       int nsweep, int ntx, int nty, int ntz, int nlev) {
   static_assert(kGsLines == 16 && kGsTx * kGsLines == kGsBlock, "a half-warp holds a component's lines, a thread a cell");
   extern __shared__ __align__(16) unsigned char gs_raw[];
-  T* coef = reinterpret_cast<T*>(gs_raw);
-  T* comp = coef + kGsCoef;
+  double* coef = reinterpret_cast<double*>(gs_raw);
+  double* comp = coef + kGsCoef;
   const int s = blockIdx.z % nsweep;
   const int g0 = blockIdx.z / nsweep * group;  // this block's components: g0 .. g0+ncomp-1
   const int ncomp = min(group, ncomp_all - g0);
@@ -1214,8 +1207,8 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
   const size_t n = d.npad();
   const size_t sy = (size_t)NX, sz = (size_t)NX * NY;
   const bool last_parity = ((nsweep - 1 - s) & 1) == 0;
-  T* xn = (last_parity ? buf_last : buf_other) + (size_t)g0 * n;        // x^s
-  const T* xo = (last_parity ? buf_other : buf_last) + (size_t)g0 * n;  // x^{s-1}
+  double* xn = (last_parity ? buf_last : buf_other) + (size_t)g0 * n;        // x^s
+  const double* xo = (last_parity ? buf_other : buf_last) + (size_t)g0 * n;  // x^{s-1}
   b += (size_t)g0 * n;
   const int i0 = I * kGsTx, j0 = J * GS_TY, k0 = K * GS_TZ;
   {
@@ -1226,16 +1219,16 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
     const int e = lb * kGsPitch + a;
     constexpr int kArr = kGsLines * kGsPitch;
     const bool u4 = in && s > 0 && i < NX - 1, u5 = in && s > 0 && j < NY - 1, u6 = in && s > 0 && k < NZ - 1;
-    const T c4 = u4 ? (T)val[4 * n + P + 1] : (T)0;
-    const T c5 = u5 ? (T)val[5 * n + P + sy] : (T)0;
-    const T c6 = u6 ? (T)val[6 * n + P + sz] : (T)0;
+    const double c4 = u4 ? val[4 * n + P + 1] : 0.0;
+    const double c5 = u5 ? val[5 * n + P + sy] : 0.0;
+    const double c6 = u6 ? val[6 * n + P + sz] : 0.0;
     if (in) {
       // a missing neighbour: coefficient and value 0, t - 0 leaves every bit of t
-      coef[e] = k > 0 ? (T)val[0 * n + P - sz] : (T)0;
-      coef[e + kArr] = j > 0 ? (T)val[1 * n + P - sy] : (T)0;
-      coef[e + 2 * kArr] = i > 0 ? (T)val[2 * n + P - 1] : (T)0;
-      coef[e + 3 * kArr] = (T)val[3 * n + P];
-      coef[e + 4 * kArr] = reinterpret_cast<const T*>(val + (sizeof(TM) == 8 ? 8 : 7) * n)[P];
+      coef[e] = k > 0 ? val[0 * n + P - sz] : 0.0;
+      coef[e + kArr] = j > 0 ? val[1 * n + P - sy] : 0.0;
+      coef[e + 2 * kArr] = i > 0 ? val[2 * n + P - 1] : 0.0;
+      coef[e + 3 * kArr] = val[3 * n + P];
+      coef[e + 4 * kArr] = val[8 * n + P];
       for (int ic = 0; ic < ncomp; ++ic) comp[(size_t)ic * kGsComp + e] = b[(size_t)ic * n + P];
     }
     // up to here only the matrix and b were read, which no sweep writes
@@ -1245,16 +1238,16 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
 #pragma unroll 2
       for (int ic = 0; ic < ncomp; ++ic) {
         const size_t q = (size_t)ic * n + P;
-        T* cs = comp + (size_t)ic * kGsComp;
-        const T x4 = u4 ? xo[q + 1] : (T)0, x5 = u5 ? xo[q + sy] : (T)0, x6 = u6 ? xo[q + sz] : (T)0;
-        T* face = cs + kArr;  // faces: below [y][x], south [z][x], west [z][y]
-        if (lz == 0) face[ly * kGsTx + a] = k > 0 ? xn[q - sz] : (T)0;
-        if (ly == 0) face[4 * kGsTx + lz * kGsTx + a] = j > 0 ? xn[q - sy] : (T)0;
-        if (a == 0) face[8 * kGsTx + lb] = i > 0 ? xn[q - 1] : (T)0;
-        T t = cs[e];
-        if (u4) t = t - gs_mul(c4, x4);
-        if (u5) t = t - gs_mul(c5, x5);
-        if (u6) t = t - gs_mul(c6, x6);
+        double* cs = comp + (size_t)ic * kGsComp;
+        const double x4 = u4 ? xo[q + 1] : 0.0, x5 = u5 ? xo[q + sy] : 0.0, x6 = u6 ? xo[q + sz] : 0.0;
+        double* face = cs + kArr;  // faces: below [y][x], south [z][x], west [z][y]
+        if (lz == 0) face[ly * kGsTx + a] = k > 0 ? xn[q - sz] : 0.0;
+        if (ly == 0) face[4 * kGsTx + lz * kGsTx + a] = j > 0 ? xn[q - sy] : 0.0;
+        if (a == 0) face[8 * kGsTx + lb] = i > 0 ? xn[q - 1] : 0.0;
+        double t = cs[e];
+        if (u4) t = t - fpi::mul_rn(c4, x4);
+        if (u5) t = t - fpi::mul_rn(c5, x5);
+        if (u6) t = t - fpi::mul_rn(c6, x6);
         cs[e] = t;
       }
     }
@@ -1268,28 +1261,28 @@ __global__ void __launch_bounds__(kGsBlock) k_gs_tile(Dims d, int ncomp_all, int
     const int ic = c0 + (threadIdx.x / 16 & 1);
     const int lb = threadIdx.x % 16, tb = lb % GS_TY, tc = lb / GS_TY;
     const bool line_ok = ic < ncomp && j0 + tb < NY && k0 + tc < NZ;
-    T* cs = comp + (size_t)(ic < ncomp ? ic : 0) * kGsComp;
-    const T* face = cs + kGsLines * kGsPitch;
-    const T* zb = face + tb * kGsTx;
-    const T* yb = face + 4 * kGsTx + tc * kGsTx;
+    double* cs = comp + (size_t)(ic < ncomp ? ic : 0) * kGsComp;
+    const double* face = cs + kGsLines * kGsPitch;
+    const double* zb = face + tb * kGsTx;
+    const double* yb = face + 4 * kGsTx + tc * kGsTx;
     const int amax = min(kGsTx, NX - i0);
     constexpr int kArr = kGsLines * kGsPitch;
-    T last = line_ok ? face[8 * kGsTx + lb] : (T)0;  // x^s west of the line, then of the previous cell
+    double last = line_ok ? face[8 * kGsTx + lb] : 0.0;  // x^s west of the line, then of the previous cell
     for (int l = 0; l < kGsTx + GS_TY + GS_TZ - 2; ++l) {
-      T from_y = __shfl_up_sync(0xffffffffu, last, 1);
-      T from_z = __shfl_up_sync(0xffffffffu, last, GS_TY);
+      double from_y = __shfl_up_sync(0xffffffffu, last, 1);
+      double from_z = __shfl_up_sync(0xffffffffu, last, GS_TY);
       const int a = l - tb - tc;
       if (line_ok && a >= 0 && a < amax) {
         const int e = lb * kGsPitch + a;
         if (tc == 0) from_z = zb[a];
         if (tb == 0) from_y = yb[a];
-        T t = cs[e];
-        const T mz = kIntL ? gs_mul(coef[e], from_z) : coef[e] * from_z;
-        const T my = kIntL ? gs_mul(coef[e + kArr], from_y) : coef[e + kArr] * from_y;
+        double t = cs[e];
+        const double mz = kIntL ? fpi::mul_rn(coef[e], from_z) : coef[e] * from_z;
+        const double my = kIntL ? fpi::mul_rn(coef[e + kArr], from_y) : coef[e + kArr] * from_y;
         t = t - mz;
         t = t - my;
         t = t - coef[e + 2 * kArr] * last;
-        t = gs_quot(t, coef[e + 3 * kArr], coef[e + 4 * kArr]);
+        t = fpi::quot_chain(t, coef[e + 3 * kArr], (unsigned long long)__double_as_longlong(coef[e + 4 * kArr]));
         cs[e] = t;
         last = t;
       }
@@ -2436,12 +2429,6 @@ __global__ void k_xupdate_half(size_t len, const asam::KrylovScalars* sc, const 
   }
 }
 
-// y = a*x + y with a host coefficient (skipped when a == 0)
-template <typename T>
-__global__ void k_axpy_host(size_t len, T a, const T* __restrict__ x, T* __restrict__ y) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x)
-    y[q] = a * x[q] + y[q];
-}
 // y = a*y + x
 template <typename T>
 __global__ void k_xpay_host(size_t len, const T* __restrict__ x, T a, T* __restrict__ y) {

@@ -56,7 +56,6 @@ struct Launch {
   void launch_xupdate_half(const Launch&, size_t len, const KrylovScalars* sc, const T* ph, T* x);              \
   void launch_xupdate(const Launch&, size_t len, const KrylovScalars* sc, int with_omega, const T* ph,          \
                       const T* rh, T* x);                                                                        \
-  void launch_axpy_host(const Launch&, size_t len, T a, const T* x, T* y);                                      \
   void launch_xpay_host(const Launch&, size_t len, const T* x, T a, T* y);                                      \
   void launch_scale_host(const Launch&, size_t len, T a, T* y);                                                 \
   void launch_tri_solve(const Launch&, int ncol, int n1, const T* d, const T* u, const T* l, T* b, T* w);        \
@@ -71,7 +70,6 @@ void launch_mass(const Launch&, const Dims&, const double* c, const double* volc
 void launch_convert_f64_to_f32(const Launch&, size_t len, const double* x, float* y);
 void launch_convert_f32_to_f64(const Launch&, size_t len, const float* x, double* y);
 void launch_add_f32_to_f64(const Launch&, size_t len, const float* x, double s, double* y);
-void launch_convert_f64_to_f32_scaled(const Launch&, size_t len, const double* x, double s, float* y);
 void launch_convert_f64_to_f32_scaled3(const Launch&, size_t len, const double* x, double s, float* y0, float* y1,
                                        float* y2);
 void launch_set_f32_to_f64(const Launch&, size_t len, const float* x, double s, double* y);

@@ -101,6 +101,45 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
       d, g, ncomp, gx, gy, gz, rvol, f, ms, df, wl, all);
   asam::count_launches(1);
 }
+// The Gauss-Seidel sweeps, one launch per tile level.  A kernel's limit of
+// dynamic shared memory is set to the same value whatever the call: threads
+// with other component counts launch it too.
+template <typename TM, typename T>
+void run_gs_sweeps(const asam::Launch& L, const asam::Dims& d, int ncomp, const TM* val, const T* b, T* out, T* work,
+                   int nsweep, int group) {
+  const int nty = (d.NY() + GS_TY - 1) / GS_TY, ntz = (d.NZ() + GS_TZ - 1) / GS_TZ;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    const int ntx = (d.NX() + GS_TX - 1) / GS_TX, nlev = ntx + nty + ntz - 2;
+    // whole warps (the sweep shuffles), one component group per CTA
+    const int threads = (GS_TY * GS_TZ * group + 31) / 32 * 32;
+    const dim3 grid(ntx, ntz, nsweep * gs_ngroups(ncomp, group));
+    cudaFuncSetAttribute(k_gs_pipe_smem<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(gs_smem_elems(kMaxComp) * sizeof(T)));
+    for (int tau = 0; tau < nlev + 2 * (nsweep - 1); ++tau) {
+      k_gs_pipe_smem<TM, T><<<grid, threads, gs_smem_elems(group) * sizeof(T), L.stream>>>(
+          d, ncomp, group, val, b, out, work, tau, nsweep, ntx, nty, ntz, nlev);
+      asam::count_launches(1);
+    }
+  } else {
+    const int ntx = (d.NX() + kGsTx - 1) / kGsTx, nlev = ntx + nty + ntz - 2;
+    // all components in one CTA, unless a level has too few tiles for two CTAs on every SM: then groups of an even
+    // number of components (a warp walks two), whose CTAs load the coefficients again
+    const int tiles = std::max(1, ntx * nty * ntz / nlev * nsweep);
+    const int ng = std::min((ncomp + 1) / 2, std::max(1, 2 * L.sm_count / tiles));
+    group = (ncomp + 2 * ng - 1) / (2 * ng) * 2;
+    const dim3 grid(ntx, ntz, nsweep * gs_ngroups(ncomp, group));
+    for (auto* f : {k_gs_tile<false>, k_gs_tile<true>})
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(gs_tile_elems(kMaxComp) * sizeof(T)));
+    // the lower part's y and z products on the integer units once the block's walking warps outnumber the
+    // sub-partitions (192x160x96, 10 components: 6.7 against 7.5 ms; 128x128x64, 3: 1.67 against 1.58)
+    auto* kernel = group > 8 ? k_gs_tile<true> : k_gs_tile<false>;
+    for (int tau = 0; tau < nlev + 2 * (nsweep - 1); ++tau) {
+      launch_chained(L, tau > 0, kernel, grid, kGsBlock, gs_tile_elems(std::min(group, ncomp)) * sizeof(T), d, ncomp,
+                     group, val, b, out, work, tau, nsweep, ntx, nty, ntz, nlev);
+      asam::count_launches(1);
+    }
+  }
+}
 }  // namespace
 
 #define ASAM_DEFINE_LAUNCHERS(T, TM)                                                                               \
@@ -153,42 +192,7 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
   }                                                                                                                \
   void launch_gs_sweeps(const Launch& L, const Dims& d, int ncomp, const TM* val, const T* b, T* out, T* work,     \
                         int nsweep, int group) {                                                                   \
-    const bool staged = sizeof(T) == sizeof(float);                                                                \
-    const int tx = staged ? GS_TX : kGsTx;                                                                         \
-    const int ntx = (d.NX() + tx - 1) / tx;                                                                        \
-    const int nty = (d.NY() + GS_TY - 1) / GS_TY;                                                                  \
-    const int ntz = (d.NZ() + GS_TZ - 1) / GS_TZ;                                                                  \
-    const int nlev = ntx + nty + ntz - 2;                                                                          \
-    /* whole warps (the sweep shuffles); the FP32 variant runs one component group per CTA */                      \
-    const int threads = staged ? (GS_TY * GS_TZ * group + 31) / 32 * 32 : kGsBlock;                                \
-    /* FP64: all components in one CTA, unless a level has too few tiles for two CTAs on every SM: then groups     \
-       of an even number of components (a warp walks two), whose CTAs load the coefficients again */               \
-    if (!staged) {                                                                                                 \
-      const int tiles = std::max(1, ntx * nty * ntz / nlev * nsweep);                                              \
-      const int ng = std::min((ncomp + 1) / 2, std::max(1, 2 * L.sm_count / tiles));                               \
-      group = (ncomp + 2 * ng - 1) / (2 * ng) * 2;                                                                 \
-    }                                                                                                              \
-    const dim3 grid(ntx, ntz, nsweep * gs_ngroups(ncomp, group));                                                  \
-    const size_t smem = (staged ? gs_smem_elems(group) : gs_tile_elems(std::min(group, ncomp))) * sizeof(T);       \
-    if (staged) /* the same value whatever the call, as below */                                                   \
-      cudaFuncSetAttribute(k_gs_pipe_smem<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,                     \
-                           (int)(gs_smem_elems(kMaxComp) * sizeof(T)));                                            \
-    if (!staged) /* the same value whatever the call: threads with other component counts launch it too */         \
-      for (auto* f : {k_gs_tile<TM, T, false>, k_gs_tile<TM, T, true>})                                            \
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,                                       \
-                             (int)(gs_tile_elems(kMaxComp) * sizeof(T)));                                          \
-    /* the lower part's y and z products on the integer units once the block's walking warps outnumber the         \
-       sub-partitions (192x160x96, 10 components: 6.7 against 7.5 ms; 128x128x64, 3: 1.67 against 1.58) */         \
-    auto* gs_kernel = group > 8 ? k_gs_tile<TM, T, true> : k_gs_tile<TM, T, false>;                                \
-    for (int tau = 0; tau < nlev + 2 * (nsweep - 1); ++tau) {                                                      \
-      if (staged)                                                                                                  \
-        k_gs_pipe_smem<TM, T><<<grid, threads, smem, L.stream>>>(d, ncomp, group, val, b, out, work, tau, nsweep,  \
-                                                                 ntx, nty, ntz, nlev);                             \
-      else                                                                                                         \
-        launch_chained(L, tau > 0, gs_kernel, grid, threads, smem, d, ncomp, group, val, b, out, work, tau, nsweep,\
-                       ntx, nty, ntz, nlev);                                                                       \
-      count_launches(1);                                                                                           \
-    }                                                                                                              \
+    run_gs_sweeps<TM, T>(L, d, ncomp, val, b, out, work, nsweep, group);                                           \
   }                                                                                                                \
   void launch_gs_persist(const Launch& L, const Dims& d, int ncomp, const TM* val, const T* b, T* out, T* work,    \
                          int nsweep, const GsTileSched& sch) {                                                     \
@@ -197,8 +201,7 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
     const int ntz = (d.NZ() + GS_TZ - 1) / GS_TZ;                                                                  \
     const int threads = (GS_TY * GS_TZ * sch.group + 31) / 32 * 32;                                                \
     const size_t smem = gs_smem_elems(sch.group) * sizeof(T);                                                      \
-    /* the attribute belongs to the kernel, which host threads with other group sizes launch too: one value for    \
-       all; per host thread the occupancy of the last shared-memory size */                                        \
+    /* the limit: one value for all threads, as in run_gs_sweeps; per host thread the occupancy of the last size */ \
     cudaFuncSetAttribute(k_gs_persist<TM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,                         \
                          (int)(gs_smem_elems(kMaxComp) * sizeof(T)));                                              \
     thread_local size_t smem_set = 0;                                                                              \
@@ -318,10 +321,6 @@ void run_flux_gather(const asam::Launch& L, const asam::Dims& d, const asam::Geo
   void launch_xupdate(const Launch& L, size_t len, const KrylovScalars* sc, int with_omega, const T* ph,           \
                       const T* rh, T* x) {                                                                         \
     k_xupdate<T><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, sc, with_omega, ph, rh, x); count_launches(1);                        \
-  }                                                                                                                \
-  void launch_axpy_host(const Launch& L, size_t len, T a, const T* x, T* y) {                                      \
-    if (a == (T)0) return;                                                                                         \
-    k_axpy_host<T><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, a, x, y); count_launches(1);                                        \
   }                                                                                                                \
   void launch_xpay_host(const Launch& L, size_t len, const T* x, T a, T* y) {                                      \
     k_xpay_host<T><<<gs_grid(L, len), kBlock, 0, L.stream>>>(len, x, a, y); count_launches(1);                                        \
