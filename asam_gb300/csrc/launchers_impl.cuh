@@ -36,13 +36,17 @@ void run_matvec(const asam::Launch& L, const asam::Dims& d, int ncomp, const TM*
   k_matvec<TM, T><<<gs_grid(L, d.npad()), kBlock, 0, L.stream>>>(d, ncomp, val, x, y, plain);
 }
 // kU: cells a lane whose loads are in flight together.  A padded row is often a
-// few cells longer than a multiple of 128, and those took a pass of their own
-// (192x160x96 FP64 step 58.02 -> 57.77 ms, four refined members 92.1 -> 91.3).
+// few cells longer than a multiple of 128, and FP64 takes those in the same pass
+// with five cells a lane (us a call, five against four, 10 components: 128x256x64
+// 248 and 269, 150x200x64 197 and 241, 256x256x64 444 and 464, 300x200x64 384 and
+// 450; 192x160x96, where five save no pass, 335 and 335).  FP32 loses by it
+// (256x256x64: 111 and 89, 192x160x96: 90 and 67, 150x200x64: 53 and 51).
 template <typename T>
 void run_axpy_dot(const asam::Launch& L, const asam::Dims& d, int ncomp, const asam::KrylovScalars* sc, int sel,
                   double sign, const T* x, T* y, double* partial) {
-  if ((d.NX() + 159) / 160 < (d.NX() + 127) / 128)
-    k_axpy_dot<T, 5><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, sc, sel, sign, x, y, partial);
+  constexpr int kU = sizeof(T) == sizeof(double) ? 5 : 4;
+  if ((d.NX() + 32 * kU - 1) / (32 * kU) < (d.NX() + 127) / 128)
+    k_axpy_dot<T, kU><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, sc, sel, sign, x, y, partial);
   else
     k_axpy_dot<T, 4><<<RED_GRID, RED_BLOCK, 0, L.stream>>>(d, ncomp, sc, sel, sign, x, y, partial);
 }
