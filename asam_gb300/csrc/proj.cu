@@ -68,8 +68,8 @@ constexpr int kMaxLev = 8;
 constexpr int kPlaneBlock = 256;
 constexpr int kRedGrid = 1024;
 constexpr int kRedBlock = 256;
-// Dynamic shared memory of k_plane_half: one CTA per SM, or two (227 KB of the
-// SM less the kernel's static part)
+// Dynamic shared memory of k_plane_half: one CTA per SM, or two (224 and 110 KB:
+// the SM's 227 KB less the kernel's static part)
 constexpr size_t kPlaneSmem1 = 229376, kPlaneSmem2 = 112640;
 constexpr double kTiny = 1.0e-40;  // initial diagonal of Allocate_1D (TriDiagT_Mod.f90:99)
 
@@ -820,9 +820,9 @@ __device__ __noinline__ void line_half(const Lev2T<T>& P, size_t mo, const T* b,
 // the back substitution from L2, the restriction's round trips.  A
 // 64x32 block runs 2240 half-sweeps per V-cycle and the coarse plane levels
 // have rows and lines in the tens, so the fixed cost was half of the time.
-// The plane levels that fit (from the coarsest up, all of them for a plane of
-// up to about 2800 FP64 entries) are therefore copied to shared memory once
-// per plane solve, and their smoothing, residuals and transfers touch nothing
+// The plane levels that fit (from the coarsest up; 2867 padded FP64 entries in
+// 224 KB, so all four levels of a plane of up to some 2150) are therefore
+// copied to shared memory once per plane solve, and their smoothing, residuals and transfers touch nothing
 // else; a level that does not fit streams from global memory.
 //
 // One resident level, in units of T from its offset: the arrays d, uz, lz,
@@ -902,8 +902,9 @@ __device__ __forceinline__ void res_copy(const Lev2T<T>& G, int off, int k) {
 
 // line_half on a resident level: the same relaxation with its operands in
 // shared memory.  The next row's operands are loaded while this row's
-// recurrence runs, so an FP64 row costs the recurrence alone (five dependent
-// operations forward and two backward; 370 and 150 cycles measured).
+// recurrence runs, so an FP64 row costs the recurrence alone: a product, a
+// difference and the quotient forward (64 + 64 + 142 cycles), a product and a
+// difference backward.
 template <typename T, bool kWrap>
 __device__ __forceinline__ void line_half_res(const Lev2T<T>& S, int c, int fwd) {
   if constexpr (sizeof(T) == 4) {

@@ -372,9 +372,11 @@ def vcycle_bytes(n1, n2, n3, R, gi2=1, gi3=1):
     (z,x,y) = (n1,n2,n3) hierarchy with R levels, counted from its schedule:
     per line-solve element 96 B (rhs b, the two neighbour-line x, the two x
     couplings, the z sub-diagonal, the pivot and its reciprocal, x written;
-    the back substitution reads x and w and writes x), per plane right-hand
-    side element 48 B, per residual element 64 B (plane) / 88 B (3D), per
-    restriction fine element 8 B and coarse element 16 B, per prolongation fine
+    the back substitution reads x and w and writes x), 2*gi + 1 half-sweeps
+    over half the lines a smoothing of a plane level, per plane right-hand
+    side element 48 B, per plane residual element, summed into the coarse
+    right-hand side as it is formed, 56 B, per 3D residual element 88 B and 8 B
+    in the restriction, per coarse element 16 B there, per prolongation fine
     element 16 B and coarse element 8 B, plus the two layout passes (16 B per
     cell each) of the call."""
     cd = lambda n, L: (n + (1 << L) - 1) >> L  # noqa: E731
@@ -384,10 +386,10 @@ def vcycle_bytes(n1, n2, n3, R, gi2=1, gi3=1):
         nq = len(dims)
         for q, (c1, c2) in enumerate(dims):
             n = c1 * c2
-            t += (2 * (q * gi2 + 1) * 2 * n * 96) if c2 > 1 else 2 * n * 96
+            t += (2 * (q * gi2 + 1) + 1) * n * 96 if c2 > 1 else 2 * n * 96
             if q + 1 < nq:
                 nc = dims[q + 1][0] * dims[q + 1][1]
-                t += n * 64 + n * 8 + nc * 16 + n * 16 + nc * 8
+                t += n * 56 + nc * 16 + n * 16 + nc * 8
         return t
 
     total = 2 * 16 * n1 * n2 * n3
@@ -915,7 +917,9 @@ def transport_bench(a, torch, stream, hbm_peak, fp64_inst_peak):
     # the Gauss-Seidel wavefront of one PSolve call: 8 matrix slots (64 B) and b,
     # x_old, x_new of every component (24 B each) per padded cell and sweep
     gs_bytes = npad * nsweep * (64 + 24 * ncomp)
-    gs_dp = npad * nsweep * ncomp * 15  # FP64 instructions per cell, component and sweep
+    # FP64 instructions per cell and component: the upper part's three differences from the second sweep on, the
+    # lower part's three differences and one product (three up to 8 components); the rest on the integer units
+    gs_dp = npad * ncomp * ((nsweep - 1) * 3 + nsweep * (4 if ncomp > 8 else 6))
     ps_s = r64["kernels"]["psolve_ms"] * 1e-3
     flux_bytes = ncell * BYTES_PER_CELL_FLUX(ncomp)
     ref = r64["final"].reshape(st.c.shape)
@@ -1108,7 +1112,7 @@ def main():
     # `python bench.py --probe vcycle` (dram__bytes_read.sum +
     # dram__bytes_write.sum over its 91 launches; one pass, so taken at full
     # size); ncu cannot run inside the timed program
-    traffic = 101.389e9 if (a.nx, a.ny, a.nz, a.seed) == (512, 512, 128, 3) else None
+    traffic = 85.043e9 if (a.nx, a.ny, a.nz, a.seed) == (512, 512, 128, 3) else None
     vc_s = r64["kernels"]["vcycle_ms"] * 1e-3
     vgbs = vb / vc_s / 1e9
     line = {
